@@ -14,7 +14,7 @@
 namespace clg {
 
 clg_status gauge_generate(clg_gauge_s* U, int init, uint64_t seed, uint32_t fid, double eps);
-clg_status gauge_reorder(clg_gauge_s* U, double* dev_buf, int layout, int to_device);
+clg_status gauge_reorder(clg_gauge_s* U, double* dev_buf, int layout, int to_device, unsigned long long* worst);
 clg_status field_reorder(clg_field_s* f, int rhs, double* dev_buf, int to_device);
 clg_status field_stream(clg_field_s* f, int rhs, double* host_dev, int to_device, cudaStream_t s);
 clg_status field_source(clg_field_s* f, int rhs, int kind, uint64_t seed, uint32_t fid, int64_t site, int comp);
@@ -560,30 +560,60 @@ clg_status clg_gauge_destroy(clg_gauge g) {
   return CLG_SUCCESS;
 }
 
-static clg_status refresh_unitarity(clg_gauge_s* g) {
-  double u = 0;
-  clg_status st = gauge_unitarity(g, &u);
-  if (st) return st;
+static void set_unitarity(clg_gauge_s* g, double u) {
   g->unitarity = u;
   g->su3 = u < 1e-12;
   g->dirty_lowp = true;
-  return CLG_SUCCESS;
+}
+
+static clg_status refresh_unitarity(clg_gauge_s* g) {
+  double u = 0;
+  clg_status st = gauge_unitarity(g, &u);
+  if (!st) set_unitarity(g, u);
+  return st;
+}
+
+// Whether the kernels can take the caller's on_device array of doubles as it
+// is: memory of this device, 8-byte aligned.  Anything else a device-to-device
+// copy accepts (another device's memory, an odd address) is staged.
+static bool direct_doubles(const clg_context_s* ctx, const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == ctx->device && (reinterpret_cast<uintptr_t>(p) & 7) == 0;
 }
 
 clg_status clg_gauge_import(clg_gauge g, const double* data, int layout, int on_device) {
   if (!g || !data || (layout != CLG_LAYOUT_CLGBIN && layout != CLG_LAYOUT_BRIDGEPP)) return CLG_ERR_BAD_ARG;
   clg_context_s* ctx = g->lat->ctx;
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
+  const bool direct = on_device && direct_doubles(ctx, data);
+  // the links' deviation from SU(3), then (staged) the links
+  unsigned long long* worst = nullptr;
   double* buf = nullptr;
-  clg_status st = dalloc(ctx, (void**)&buf, bytes);
+  clg_status st = dalloc(ctx, (void**)&worst, sizeof(*worst));
   if (st) return st;
-  cudaError_t e = cudaMemcpyAsync(buf, data, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                                  ctx->stream);
+  if (!direct && (st = dalloc(ctx, (void**)&buf, bytes))) {
+    dfree(worst);
+    return st;
+  }
+  cudaError_t e = cudaMemsetAsync(worst, 0, sizeof(*worst), ctx->stream);
+  if (e == cudaSuccess && !direct)
+    e = cudaMemcpyAsync(buf, data, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) st = ctx->fail(cuda_status(e), cudaGetErrorString(e));
-  if (!st) st = gauge_reorder(g, buf, layout, 1);
+  if (!st) st = gauge_reorder(g, direct ? const_cast<double*>(data) : buf, layout, 1, worst);
+  double u = 0.0;
+  if (!st) {
+    e = cudaMemcpyAsync(&u, worst, sizeof(u), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e != cudaSuccess) st = ctx->fail(cuda_status(e), cudaGetErrorString(e));
+  }
+  // the caller may reuse or free its array once this returns
   if (!st) st = sync_status(ctx);
   dfree(buf);
-  if (!st) st = refresh_unitarity(g);
+  dfree(worst);
+  if (!st) set_unitarity(g, u);
   return st;
 }
 
@@ -591,11 +621,12 @@ clg_status clg_gauge_export(clg_gauge g, double* data, int on_device) {
   if (!g || !data) return CLG_ERR_BAD_ARG;
   clg_context_s* ctx = g->lat->ctx;
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
+  const bool direct = on_device && direct_doubles(ctx, data);
   double* buf = nullptr;
-  clg_status st = dalloc(ctx, (void**)&buf, bytes);
-  if (st) return st;
-  st = gauge_reorder(g, buf, CLG_LAYOUT_CLGBIN, 0);
-  if (!st) {
+  clg_status st = CLG_SUCCESS;
+  if (!direct && (st = dalloc(ctx, (void**)&buf, bytes))) return st;
+  st = gauge_reorder(g, direct ? data : buf, CLG_LAYOUT_CLGBIN, 0, nullptr);
+  if (!st && !direct) {
     cudaError_t e = cudaMemcpyAsync(data, buf, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                     ctx->stream);
     if (e != cudaSuccess) st = ctx->fail(cuda_status(e), cudaGetErrorString(e));
@@ -608,8 +639,13 @@ clg_status clg_gauge_export(clg_gauge g, double* data, int on_device) {
 clg_status clg_gauge_random(clg_gauge g, int init, uint64_t seed, uint32_t field_id, double eps) {
   if (!g || init < 0 || init > CLG_GAUGE_ZERO) return CLG_ERR_BAD_ARG;
   clg_status st = gauge_generate(g, init, seed, field_id, eps);
-  if (!st) st = refresh_unitarity(g);
-  return st;
+  if (st) return st;
+  // unit links deviate by 0, zero links (a force accumulator) by |0 - 1| = 1
+  if (init == CLG_GAUGE_IDENTITY || init == CLG_GAUGE_ZERO) {
+    set_unitarity(g, init == CLG_GAUGE_ZERO ? 1.0 : 0.0);
+    return launch_status(g->lat->ctx);
+  }
+  return refresh_unitarity(g);
 }
 
 clg_status clg_gauge_plaquette(clg_gauge g, double* out) {
