@@ -198,12 +198,22 @@ clg_status apply_op(clg_context_s* ctx, int op, const clg_gauge_s* U, int kind, 
       // Wilson: out_p = in_p - kappa H in_(1-p); staggered: out_p = 2am in_p +/- H in_(1-p)
       const double2 a = wilson ? cmulh(coeff, c2(-param, 0)) : cmulh(coeff, c2(dag ? -1.0 : 1.0, 0));
       const double2 xa = wilson ? coeff : cmulh(coeff, c2(param, 0));
-      for (int p = 0; p < 2; ++p) {
-        FieldRef x = in;
-        st = hop1(ctx, U, kind, dag && wilson, p, in, out, &x, a, xa, nrhs, scale_dev, scale_stride, skip_dev, skip_stride);
-        if (st) return st;
-      }
-      return CLG_SUCCESS;
+      HopSpec h;
+      h.kind = kind;
+      h.prec = out.prec;
+      h.dagger = dag && wilson;
+      h.out_parity = 0;
+      h.in = in;
+      h.out = out;
+      h.x = &in;
+      h.a = a;
+      h.xa = xa;
+      h.scale_dev = scale_dev;
+      h.scale_stride = scale_stride;
+      h.skip_dev = skip_dev;
+      h.skip_stride = skip_stride;
+      h.nrhs = nrhs;
+      return hop_full(ctx, U, h);
     }
     case CLG_OP_DDDAG:
     case CLG_OP_DD: {

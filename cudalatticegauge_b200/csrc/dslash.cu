@@ -33,6 +33,12 @@ cudaError_t launch_wilson_tileN(clg_context_s* ctx, const HopArgs& a0, bool dagg
 
 std::vector<int> tile_warps(int nrhs);
 
+// Four threads per site are timed where one thread per site gives the chip
+// less than SPLIT_MAX threads (it wins up to about 2^14 sites; the autotuner
+// decides between)
+constexpr int64_t SPLIT_MAX = (int64_t)1 << 18;
+bool split_worth(const Geom& g, int nrhs) { return g.Vh * nrhs <= SPLIT_MAX; }
+
 template <int P, int RECON>
 cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int nrhs, const std::string& key) {
   // config = block size | (variant << 16): 0 plain, 1 capped at 80 registers,
@@ -43,6 +49,11 @@ cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int
     const int variant = cfg >> 16;
     if constexpr (P != P16) {
       if (variant >= 16) return launch_wilson_tileN<P, RECON>(ctx, a, dagger, cfg);
+    }
+    if (variant == HOP_SPLIT) {
+      dim3 sg((unsigned)(((a.g.Vh + SPLIT_SITES - 1) / SPLIT_SITES) * nrhs));
+      return dagger ? launch_pdl(ctx, wilson_split_kernel<P, RECON, true, false>, sg, dim3(4 * SPLIT_SITES), 0, a)
+                    : launch_pdl(ctx, wilson_split_kernel<P, RECON, false, false>, sg, dim3(4 * SPLIT_SITES), 0, a);
     }
     dim3 grid((unsigned)(((a.g.Vh + bs - 1) / bs) * nrhs));
     if constexpr (P == P64) {
@@ -72,6 +83,7 @@ cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int
   if (P != P64) cand.push_back(64 | (2 << 16));
   if (P == P64)
     for (int bs : {64, 128, 256}) cand.push_back(bs | (3 << 16));
+  if (split_worth(a.g, nrhs)) cand.push_back((4 * SPLIT_SITES) | (HOP_SPLIT << 16));
   // several right-hand sides: the tile form (links staged once per tile)
   if (P != P16 && nrhs >= 2)
     for (int w : tile_warps(nrhs))
@@ -141,6 +153,19 @@ int tile_rows(const Geom& g, int nrhs, int ts, int sbytes) {
   int best = 0;
   for (int by = 1; by < g.L[1]; ++by)
     if (g.L[1] % by == 0 && 3 * by * slab_row <= (int64_t)24 << 20) best = by;
+  return best;
+}
+
+// The y-rows per chunk of a full-lattice launch (full_site): 0 where two
+// x-slabs of everything a site touches (bytes: its spinors and four links) fit
+// in 40 MB of L2, else the largest divisor of L_y for which they do (0: none).
+int full_rows(const Geom& g, int64_t bytes) {
+  const int64_t row = (int64_t)g.L[2] * g.L[3] * bytes;
+  constexpr int64_t most = (int64_t)40 << 20;
+  if (2 * row * g.L[1] <= most) return 0;
+  int best = 0;
+  for (int by = 1; by < g.L[1]; ++by)
+    if (g.L[1] % by == 0 && 2 * by * row <= most) best = by;
   return best;
 }
 
@@ -299,6 +324,48 @@ cudaError_t launch_staggered(clg_context_s* ctx, const HopArgs& a, int nrhs, con
       for (int v = 0; v < (tile_rows(a.g, nrhs, TILE16, P == P64 ? 48 : 24) ? 4 : 2); ++v)
         cand.push_back((32 * w) | ((16 + v) << 16));
   return go(tune_block(ctx, key, idempotent(a), go, cand));
+}
+
+// ------------------------------------------------------------------ both checkerboards in one launch
+// Launch configurations of a full-lattice D: block | variant << 16 with variant
+// 0 = two checkerboard hops, FULL_ONE + (1: register cap) + (2: chunks of
+// y-rows), FULL_SPLIT = four threads per site
+constexpr int FULL_ONE = 32, FULL_SPLIT = 36;
+
+std::vector<int> full_candidates(const HopArgs& a, int rows, bool split) {
+  std::vector<int> c = {0};
+  for (int v = 0; v < (rows ? 4 : 2); ++v)
+    for (int bs : {64, 128, 256}) c.push_back(bs | ((FULL_ONE + v) << 16));
+  if (split && split_worth(a.g, 2 * a.nrhs)) c.push_back((4 * SPLIT_SITES) | (FULL_SPLIT << 16));
+  return c;
+}
+
+template <int P, int RECON>
+cudaError_t launch_wilson_full(clg_context_s* ctx, const HopArgs& a0, bool dagger, int rows, int cfg) {
+  constexpr int CAP = P == P64 ? 2 : 3;
+  const int bs = cfg & 0xffff, v = cfg >> 16;
+  HopArgs a = a0;
+  const int sites = v == FULL_SPLIT ? SPLIT_SITES : bs;
+  const dim3 grid((unsigned)(2 * ((a.g.Vh + sites - 1) / sites) * a.nrhs));
+  if (v == FULL_SPLIT)
+    return dagger ? launch_pdl(ctx, wilson_split_kernel<P, RECON, true, true>, grid, dim3(bs), 0, a)
+                  : launch_pdl(ctx, wilson_split_kernel<P, RECON, false, true>, grid, dim3(bs), 0, a);
+  a.tile_rows = (v & 2) ? rows : 0;
+  if (v & 1)
+    return dagger ? launch_pdl(ctx, wilson_full_kernel<P, RECON, true, 256, CAP>, grid, dim3(bs), 0, a)
+                  : launch_pdl(ctx, wilson_full_kernel<P, RECON, false, 256, CAP>, grid, dim3(bs), 0, a);
+  return dagger ? launch_pdl(ctx, wilson_full_kernel<P, RECON, true>, grid, dim3(bs), 0, a)
+                : launch_pdl(ctx, wilson_full_kernel<P, RECON, false>, grid, dim3(bs), 0, a);
+}
+
+template <int P, int RECON>
+cudaError_t launch_staggered_full(clg_context_s* ctx, const HopArgs& a0, int rows, int cfg) {
+  const int bs = cfg & 0xffff, v = cfg >> 16;
+  HopArgs a = a0;
+  const dim3 grid((unsigned)(2 * ((a.g.Vh + bs - 1) / bs) * a.nrhs));
+  a.tile_rows = (v & 2) ? rows : 0;
+  if (v & 1) return launch_pdl(ctx, staggered_full_kernel<P, RECON, 3>, grid, dim3(bs), 0, a);
+  return launch_pdl(ctx, staggered_full_kernel<P, RECON, 1>, grid, dim3(bs), 0, a);
 }
 
 // FP64 [mu][9][h] double2 -> FP32 12-real [mu][3][h] float4 or 18-real [mu][9][h] float2
@@ -466,6 +533,9 @@ clg_status make_hop_args(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec
   a.btile = U->btile;
   a.nbtile = U->nbtile;
   a.btiles = U->btiles;
+  a.in_blk = s.in.blk;
+  a.out_blk = s.out.blk;
+  a.x_blk = s.x ? s.x->blk : 0;
   if (U->seg) {
     if (s.kind != CLG_FERMION_WILSON) return ctx->fail(CLG_ERR_UNSUPPORTED, "a batch of lattices takes Wilson fermions");
     a.U_here = a.U_there = nullptr;
@@ -542,6 +612,49 @@ clg_status hop(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s) {
     e = wilson ? launch_wilson<P16, 12>(ctx, a, s.dagger, s.nrhs, key) : launch_staggered<P16, 12>(ctx, a, s.nrhs, key);
   }
   if (e != cudaSuccess) return ctx->fail(cuda_status(e), std::string("hop launch: ") + cudaGetErrorString(e));
+  return CLG_SUCCESS;
+}
+
+clg_status hop_full(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s) {
+  const bool wilson = s.kind == CLG_FERMION_WILSON;
+  auto two = [&]() -> clg_status {
+    HopSpec q = s;
+    for (q.out_parity = 0; q.out_parity < 2; ++q.out_parity)
+      if (clg_status st = hop(ctx, U, q)) return st;
+    return CLG_SUCCESS;
+  };
+  // a batch of lattices and the pinned forms have checkerboard hops only
+  if (U->seg || ctx->hop_config >= 0 || (s.prec == CLG_PREC_HALF && wilson && s.nrhs >= 2 && ctx->hop_pair_mode != 2))
+    return two();
+  HopSpec q = s;
+  q.out_parity = 0;
+  HopArgs a;
+  if (clg_status st = make_hop_args(ctx, U, q, a)) return st;
+  const int real = s.prec == CLG_PREC_DOUBLE ? 8 : (s.prec == CLG_PREC_SINGLE ? 4 : 2);
+  const int links = 4 * (s.prec == CLG_PREC_DOUBLE ? 18 : (s.prec == CLG_PREC_SINGLE ? U->recon32 : 12)) * real;
+  const int rows = full_rows(a.g, links + (int64_t)2 * s.nrhs * (wilson ? 24 : 6) * real);
+  clg_status hst = CLG_SUCCESS;
+  auto go = [&](int cfg) -> cudaError_t {
+    if (cfg == 0) {
+      hst = two();
+      return hst ? cudaErrorUnknown : cudaSuccess;
+    }
+    if (s.prec == CLG_PREC_DOUBLE)
+      return wilson ? launch_wilson_full<P64, 18>(ctx, a, s.dagger, rows, cfg)
+                    : launch_staggered_full<P64, 18>(ctx, a, rows, cfg);
+    if (s.prec == CLG_PREC_HALF)
+      return wilson ? launch_wilson_full<P16, 12>(ctx, a, s.dagger, rows, cfg)
+                    : launch_staggered_full<P16, 12>(ctx, a, rows, cfg);
+    if (U->recon32 == 12)
+      return wilson ? launch_wilson_full<P32, 12>(ctx, a, s.dagger, rows, cfg)
+                    : launch_staggered_full<P32, 12>(ctx, a, rows, cfg);
+    return wilson ? launch_wilson_full<P32, 18>(ctx, a, s.dagger, rows, cfg)
+                  : launch_staggered_full<P32, 18>(ctx, a, rows, cfg);
+  };
+  const cudaError_t e = go(tune_block(ctx, hop_key(U, s) + "_full", idempotent(a), go, full_candidates(a, rows, wilson),
+                                      128 | ((FULL_ONE + 1) << 16)));
+  if (hst) return hst;
+  if (e != cudaSuccess) return ctx->fail(cuda_status(e), std::string("full hop launch: ") + cudaGetErrorString(e));
   return CLG_SUCCESS;
 }
 

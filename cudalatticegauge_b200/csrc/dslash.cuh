@@ -68,6 +68,9 @@ struct HopArgs {
   const struct BatchTile* btile;
   int nbtile;
   int64_t btiles;  // blocks of the batch (all lattices' tiles)
+  // both checkerboards in one launch (the full-lattice forms; the fields above
+  // are those of out_parity 0): bytes from a field's parity 0 to its parity 1
+  int64_t in_blk, out_blk, x_blk;
 };
 struct BatchTile {
   int64_t tile0;
@@ -100,11 +103,12 @@ __device__ __forceinline__ void su3_mv(const cpx<AT> u[9], const cpx<AT> v[3], c
   }
 }
 
-// acc += s * P^{SGN}_mu (Udag? U^+ : U) psi   with P^{SGN} = (1 + SGN g_mu)
+// The two upper rows g0, g1 of (Udag? U^+ : U) P^{SGN}_mu psi, P^{SGN} = (1 + SGN g_mu)
 template <typename AT, int MU, int SGN, bool UDAG>
-__device__ __forceinline__ void wilson_hop_dir(cpx<AT> acc[12], const cpx<AT> psi[12], const cpx<AT> u[9], AT s) {
+__device__ __forceinline__ void wilson_dir_rows(const cpx<AT> psi[12], const cpx<AT> u[9], cpx<AT> g0[3],
+                                                cpx<AT> g1[3]) {
   constexpr int add = SGN < 0 ? 2 : 0;
-  cpx<AT> h0[3], h1[3], g0[3], g1[3];
+  cpx<AT> h0[3], h1[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     h0[c] = psi[c] + mul_i(psi[3 * gperm(MU, 0) + c], gz4(MU, 0) + add);
@@ -112,6 +116,12 @@ __device__ __forceinline__ void wilson_hop_dir(cpx<AT> acc[12], const cpx<AT> ps
   }
   su3_mv<AT, UDAG>(u, h0, g0);
   su3_mv<AT, UDAG>(u, h1, g1);
+}
+
+// acc += s * (the projected direction whose upper rows are g0, g1)
+template <typename AT, int MU, int SGN>
+__device__ __forceinline__ void wilson_dir_acc(cpx<AT> acc[12], const cpx<AT> g0[3], const cpx<AT> g1[3], AT s) {
+  constexpr int add = SGN < 0 ? 2 : 0;
   // each accumulator row takes s * (phase * g) as one fused multiply-add per
   // real component: the phase is a swap / negation (operand modifiers), and s
   // is never applied to g separately
@@ -123,6 +133,14 @@ __device__ __forceinline__ void wilson_hop_dir(cpx<AT> acc[12], const cpx<AT> ps
     acc[6 + c] = cfma(s, mul_i(gperm(MU, 2) == 0 ? g0[c] : g1[c], gz4(MU, 2) + add), acc[6 + c]);
     acc[9 + c] = cfma(s, mul_i(gperm(MU, 3) == 0 ? g0[c] : g1[c], gz4(MU, 3) + add), acc[9 + c]);
   }
+}
+
+// acc += s * P^{SGN}_mu (Udag? U^+ : U) psi
+template <typename AT, int MU, int SGN, bool UDAG>
+__device__ __forceinline__ void wilson_hop_dir(cpx<AT> acc[12], const cpx<AT> psi[12], const cpx<AT> u[9], AT s) {
+  cpx<AT> g0[3], g1[3];
+  wilson_dir_rows<AT, MU, SGN, UDAG>(psi, u, g0, g1);
+  wilson_dir_acc<AT, MU, SGN>(acc, g0, g1, s);
 }
 
 // ---------------------------------------------------------------- FP16 arithmetic in half2 words
@@ -226,7 +244,8 @@ __device__ __forceinline__ float2 f2_fma_signed(float s, float2 f, float2 acc) {
 // Both projected rows' phases i^z have the same parity for every direction
 // of the chiral basis (gz4), which is what lets one plane select serve both.
 template <int MU, int SGN, bool UDAG>
-__device__ __forceinline__ void wilson_hop_dir16_u(Acc16& A, const Packed16& p, const uint32_t (&u)[9], float s) {
+__device__ __forceinline__ void wilson_dir16_rows(const Packed16& p, const uint32_t (&u)[9], __half2 (&gR)[3],
+                                                  __half2 (&gI)[3]) {
   constexpr int add = SGN < 0 ? 2 : 0;
   constexpr int z0 = (gz4(MU, 0) + add) & 3, z1 = (gz4(MU, 1) + add) & 3;
   static_assert(((z0 ^ z1) & 1) == 0, "projected rows with phases of different parity");
@@ -263,7 +282,8 @@ __device__ __forceinline__ void wilson_hop_dir16_u(Acc16& A, const Packed16& p, 
   }
   // g_j = U h_j (UDAG: U^+ h_j), both rows per instruction
   const __half2 zero = __float2half2_rn(0.f);
-  __half2 gR[3] = {zero, zero, zero}, gI[3] = {zero, zero, zero};
+#pragma unroll
+  for (int r = 0; r < 3; ++r) gR[r] = gI[r] = zero;
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -281,6 +301,12 @@ __device__ __forceinline__ void wilson_hop_dir16_u(Acc16& A, const Packed16& p, 
         gI[r] = __hfma2(ei, hR[k], gI[r]);
       }
     }
+}
+
+// A += s * (the projected direction whose upper rows are the planes gR, gI)
+template <int MU, int SGN>
+__device__ __forceinline__ void wilson_dir16_acc(Acc16& A, const __half2 (&gR)[3], const __half2 (&gI)[3], float s) {
+  constexpr int add = SGN < 0 ? 2 : 0;
   // FP32 accumulation.  Rows 0, 1 take s g_0, s g_1; rows 2, 3 take
   // s i^z_r g_perm(r), perm = (1, 0) for mu < 2 (the lanes swapped) and (0, 1)
   // for mu >= 2, with z_2, z_3 of equal parity as well.
@@ -302,6 +328,13 @@ __device__ __forceinline__ void wilson_hop_dir16_u(Acc16& A, const Packed16& p, 
       A.i[3 + c] = f2_fma_signed<z2 == 1, z3 == 1>(s, gr, A.i[3 + c]);
     }
   }
+}
+
+template <int MU, int SGN, bool UDAG>
+__device__ __forceinline__ void wilson_hop_dir16_u(Acc16& A, const Packed16& p, const uint32_t (&u)[9], float s) {
+  __half2 gR[3], gI[3];
+  wilson_dir16_rows<MU, SGN, UDAG>(p, u, gR, gI);
+  wilson_dir16_acc<MU, SGN>(A, gR, gI, s);
 }
 
 // The same with the link as stored (12-real): the third row is rebuilt first.
@@ -510,6 +543,237 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_kernel(HopArgs a) {
   wilson_hop_store<P>(a, rhs, h, acc);
 }
 
+// ---------------------------------------------------------------- both checkerboards in one launch
+// D on a full field is two checkerboard hops that read the same links: U_mu(x)
+// forward from x and backward from x + mu, of the other parity.  As two
+// launches each link and spinor crosses DRAM twice (FP64 Wilson 1728 B per
+// site); with the blocks of the two parities alternating over the same region,
+// the second reader finds them in L2 and the DRAM traffic falls towards one
+// read of links and spinors and one write (960 B per site).  Two hops -> one
+// launch, us per D: 32^3x16 Wilson FP64 150 -> 107, FP32 67 -> 46, FP16 39 ->
+// 33, staggered FP64 107 -> 63, FP32 40 -> 29; 48^3x24 Wilson FP64 744 -> 540
+// (589 without the chunks of y-rows of full_site), FP32 288 -> 226, staggered
+// FP64 501 -> 323.  HopArgs hold parity 0; flip_parity turns them into parity
+// 1's.
+__device__ __forceinline__ void flip_parity(HopArgs& a) {
+  a.out_parity = 1;
+  a.in = static_cast<const char*>(a.in) - a.in_blk;
+  a.out = static_cast<char*>(a.out) + a.out_blk;
+  if (a.x) a.x = static_cast<const char*>(a.x) + a.x_blk;
+  if (a.in_norm) a.in_norm -= a.g.Vh;
+  if (a.out_norm) a.out_norm += a.g.Vh;
+  if (a.x_norm) a.x_norm += a.g.Vh;
+  const void* t = a.U_here;
+  a.U_here = a.U_there;
+  a.U_there = t;
+}
+// Block b of a full-lattice launch: right-hand side, parity, slot of sites
+__device__ __forceinline__ void full_block(const HopArgs& a, int& rhs, int& p, unsigned& slot) {
+  const unsigned b = blockIdx.x / (unsigned)a.nrhs;
+  rhs = (int)(blockIdx.x - b * (unsigned)a.nrhs);
+  p = (int)(b & 1);
+  slot = b >> 1;
+}
+// The checkerboard index of the i-th site in launch order: i itself, or with
+// tile_rows > 0 (a divisor of L_y) chunk after chunk of tile_rows y-rows with x
+// slowest in a chunk, so that three x-slabs of a chunk fit in L2 (full_rows)
+__device__ __forceinline__ int64_t full_site(const HopArgs& a, int64_t i) {
+  if (a.tile_rows <= 0) return i;
+  const unsigned np = (unsigned)a.g.L[2] * (unsigned)a.g.L[3] / 2u;
+  const unsigned per_x = (unsigned)a.tile_rows * np, per_chunk = (unsigned)a.g.L[0] * per_x;
+  const unsigned yc = (unsigned)i / per_chunk, r = (unsigned)i - yc * per_chunk;
+  const unsigned x = r / per_x, r2 = r - x * per_x;
+  return (int64_t)(x * (unsigned)a.g.L[1] + yc * (unsigned)a.tile_rows) * np + r2;
+}
+
+template <int P, int RECON, bool DAGGER, int MAXT = 256, int MINB = 1>
+__global__ void __launch_bounds__(MAXT, MINB) wilson_full_kernel(HopArgs a) {
+  using AT = typename AccT<P>::T;
+  int rhs, p;
+  unsigned slot;
+  full_block(a, rhs, p, slot);
+  const int64_t i = (int64_t)slot * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  if (p) flip_parity(a);
+  pdl_wait();
+  if (i >= a.g.Vh) return;
+  if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;
+  const int64_t h = full_site(a, i);
+  cpx<AT> acc[12];
+  wilson_hop_site<P, RECON, DAGGER>(a, rhs, h, acc);
+  wilson_hop_store<P>(a, rhs, h, acc);
+}
+
+// ---------------------------------------------------------------- four threads per site
+// On a small lattice one thread per site leaves most of the chip idle and each
+// thread walks the 8 directions one after another (8^4: 2048 sites of a
+// checkerboard on 16 of 148 SMs, 8.8 us a hop).  Here a block is 32 sites x 4
+// warps; warp mu loads the two neighbours and links of direction mu and leaves
+// the projected products (the upper rows) in shared memory, then warp 0 adds
+// the 8 directions of its site in the order of the one-thread form (the
+// boundary signs are exact), so the bits are the same.  A whole D on 8^4, back
+// to back: 4.0 us against 5.8 (one thread per site) and 10.1 (two hops); on
+// 16^3x32 it loses (37.5 against 31.1 us, FP64).
+constexpr int SPLIT_SITES = 32;
+constexpr int HOP_SPLIT = 4;  // this form's launch variant (dslash.cu)
+template <int P>
+struct SplitSmem {
+  cpx<typename AccT<P>::T> g[8][6][SPLIT_SITES];  // s (g0, g1) of direction 2 mu + (0 forward, 1 backward)
+};
+template <>
+struct SplitSmem<P16> {
+  uint32_t g[8][6][SPLIT_SITES];  // the planes gR, gI
+  float s[8][SPLIT_SITES];        // boundary sign times the neighbour's site norm
+};
+
+template <int P, int RECON, bool DAGGER, int MU>
+__device__ __forceinline__ void wilson_split_dir(const HopArgs& a, int rhs, int64_t h, int i, const NbrInfo& nb,
+                                                 SplitSmem<P>& t) {
+  using AT = typename AccT<P>::T;
+  constexpr int SF = DAGGER ? 1 : -1, SB = -SF;
+  const int64_t Vh = a.g.Vh;
+  const char* in = reinterpret_cast<const char*>(a.in) + rhs * a.in_stride;
+  const float* in_norm = a.in_norm ? a.in_norm + rhs * a.in_nstride : nullptr;
+  if constexpr (P == P16) {
+    Packed16 pf, pb;
+    PackedLink16 lf, lb;
+    load_packed16(in, in_norm, Vh, nb.hf[MU], pf);
+    load_packed_link16(a.U_here, MU, Vh, h, lf);
+    load_packed16(in, in_norm, Vh, nb.hb[MU], pb);
+    load_packed_link16(a.U_there, MU, Vh, nb.hb[MU], lb);
+    __half2 gR[3], gI[3];
+    uint32_t u[9] = {lf.a.x, lf.a.y, lf.a.z, lf.a.w, lf.b.x, lf.b.y, 0u, 0u, 0u};
+    link16_third_row(u);
+    wilson_dir16_rows<MU, SF, false>(pf, u, gR, gI);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t.g[2 * MU][c][i] = as_u32(gR[c]);
+      t.g[2 * MU][3 + c][i] = as_u32(gI[c]);
+    }
+    t.s[2 * MU][i] = nb.sf[MU] * pf.n;
+    uint32_t w[9] = {lb.a.x, lb.a.y, lb.a.z, lb.a.w, lb.b.x, lb.b.y, 0u, 0u, 0u};
+    link16_third_row(w);
+    wilson_dir16_rows<MU, SB, true>(pb, w, gR, gI);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t.g[2 * MU + 1][c][i] = as_u32(gR[c]);
+      t.g[2 * MU + 1][3 + c][i] = as_u32(gI[c]);
+    }
+    t.s[2 * MU + 1][i] = nb.sb[MU] * pb.n;
+  } else {
+    cpx<AT> pf[12], pb[12], uf[9], ub[9], g0[3], g1[3];
+    load_site<P, 12, AT>(in, in_norm, Vh, nb.hf[MU], pf);
+    load_link<P, RECON, AT>(a.U_here, MU, Vh, h, uf);
+    load_site<P, 12, AT>(in, in_norm, Vh, nb.hb[MU], pb);
+    load_link<P, RECON, AT>(a.U_there, MU, Vh, nb.hb[MU], ub);
+    wilson_dir_rows<AT, MU, SF, false>(pf, uf, g0, g1);
+    const AT sf = (AT)nb.sf[MU], sb = (AT)nb.sb[MU];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t.g[2 * MU][c][i] = sf * g0[c];
+      t.g[2 * MU][3 + c][i] = sf * g1[c];
+    }
+    wilson_dir_rows<AT, MU, SB, true>(pb, ub, g0, g1);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      t.g[2 * MU + 1][c][i] = sb * g0[c];
+      t.g[2 * MU + 1][3 + c][i] = sb * g1[c];
+    }
+  }
+}
+
+// the 8 directions of site i summed, then the finish; by one thread per site
+template <int P, bool DAGGER, typename AT>
+__device__ __forceinline__ void wilson_split_sum(const HopArgs& a, const SplitSmem<P>& t, int rhs, int64_t h, int i,
+                                                 cpx<AT> acc[12]) {
+  constexpr int SF = DAGGER ? 1 : -1, SB = -SF;
+  if constexpr (P == P16) {
+    Acc16 A;
+    acc16_zero(A);
+    __half2 gR[3], gI[3];
+    auto get = [&](int d) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        gR[c] = as_h2(t.g[d][c][i]);
+        gI[c] = as_h2(t.g[d][3 + c][i]);
+      }
+    };
+#define CLG_SPLIT16(MU)                                  \
+  get(2 * MU);                                           \
+  wilson_dir16_acc<MU, SF>(A, gR, gI, t.s[2 * MU][i]);   \
+  get(2 * MU + 1);                                       \
+  wilson_dir16_acc<MU, SB>(A, gR, gI, t.s[2 * MU + 1][i]);
+    CLG_SPLIT16(0)
+    CLG_SPLIT16(1)
+    CLG_SPLIT16(2)
+    CLG_SPLIT16(3)
+#undef CLG_SPLIT16
+    acc16_out(A, acc);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k] = mk<AT>(0, 0);
+    cpx<AT> g0[3], g1[3];
+    auto get = [&](int d) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        g0[c] = t.g[d][c][i];
+        g1[c] = t.g[d][3 + c][i];
+      }
+    };
+#define CLG_SPLIT(MU)                                  \
+  get(2 * MU);                                         \
+  wilson_dir_acc<AT, MU, SF>(acc, g0, g1, (AT)1);      \
+  get(2 * MU + 1);                                     \
+  wilson_dir_acc<AT, MU, SB>(acc, g0, g1, (AT)1);
+    CLG_SPLIT(0)
+    CLG_SPLIT(1)
+    CLG_SPLIT(2)
+    CLG_SPLIT(3)
+#undef CLG_SPLIT
+  }
+  wilson_hop_finish<P>(a, rhs, h, acc);
+}
+
+template <int P, int RECON, bool DAGGER>
+__device__ __forceinline__ void wilson_split_stage(const HopArgs& a, int rhs, int64_t h, int i, SplitSmem<P>& t) {
+  NbrInfo nb;
+  int c[4];
+  neighbours(a.g, a.out_parity, h, nb, c);
+  switch (threadIdx.x >> 5) {
+    case 0: wilson_split_dir<P, RECON, DAGGER, 0>(a, rhs, h, i, nb, t); break;
+    case 1: wilson_split_dir<P, RECON, DAGGER, 1>(a, rhs, h, i, nb, t); break;
+    case 2: wilson_split_dir<P, RECON, DAGGER, 2>(a, rhs, h, i, nb, t); break;
+    default: wilson_split_dir<P, RECON, DAGGER, 3>(a, rhs, h, i, nb, t); break;
+  }
+}
+
+// FULL: both checkerboards in one launch (full_block), else out_parity alone
+template <int P, int RECON, bool DAGGER, bool FULL>
+__global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_kernel(HopArgs a) {
+  using AT = typename AccT<P>::T;
+  __shared__ SplitSmem<P> t;
+  int rhs, p = 0;
+  unsigned slot;
+  if constexpr (FULL) {
+    full_block(a, rhs, p, slot);
+  } else {
+    slot = blockIdx.x / (unsigned)a.nrhs;
+    rhs = (int)(blockIdx.x - slot * (unsigned)a.nrhs);
+  }
+  const int i = threadIdx.x & 31;
+  const int64_t h = (int64_t)slot * SPLIT_SITES + i;
+  pdl_launch_dependents();
+  if (FULL && p) flip_parity(a);
+  pdl_wait();
+  if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;  // uniform over the block
+  if (h < a.g.Vh) wilson_split_stage<P, RECON, DAGGER>(a, rhs, h, i, t);
+  __syncthreads();
+  if (threadIdx.x >= 32 || h >= a.g.Vh) return;
+  cpx<AT> acc[12];
+  wilson_split_sum<P, DAGGER>(a, t, rhs, h, i, acc);
+  wilson_hop_store<P>(a, rhs, h, acc);
+}
+
 // The hop over a batch of lattices (HopArgs::seg): right-hand side r on its own
 // lattice, the grid spanning the largest checkerboard.
 // (the register caps of the tuned one-lattice kernels: 80 for FP32 / FP16,
@@ -568,6 +832,68 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
   grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
                                     gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter,
                                     BATCH ? a.seg_vh : nullptr);
+}
+
+// The epilogue form of wilson_full_kernel, one right-hand side: E::par is set to
+// the block's parity; one slot per block of either parity.
+template <int P, int RECON, bool DAGGER, int MAXT, int MINB, class E>
+__global__ void __launch_bounds__(MAXT, MINB) wilson_full_epi_kernel(HopArgs a, E e, double* partials, double* gpart,
+                                                                     unsigned* counter, unsigned group) {
+  using AT = typename AccT<P>::T;
+  int rhs, p;
+  unsigned slot;
+  full_block(a, rhs, p, slot);
+  const int64_t i = (int64_t)slot * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  if (p) flip_parity(a);
+  e.par = p;
+  pdl_wait();
+  double red[E::NRED];
+#pragma unroll
+  for (int k = 0; k < E::NRED; ++k) red[k] = 0.0;
+  if (i < a.g.Vh) {
+    const int64_t h = full_site(a, i);
+    cpx<AT> acc[12];
+    wilson_hop_site<P, RECON, DAGGER>(a, rhs, h, acc);
+    if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
+    e.site(rhs, h, acc, red);
+  }
+  const int rr[1] = {0};
+  const bool cc[1] = {true}, hh[1] = {true};
+  grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, 0u, 1u, blockIdx.x, gridDim.x, 1, group, partials, gpart,
+                                    counter);
+}
+
+// The epilogue form with four threads per site (wilson_split_kernel): warp 0
+// holds the block's results and reduces them; one slot per 32 sites.
+template <int P, int RECON, bool DAGGER, class E>
+__global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopArgs a, E e, double* partials,
+                                                                          double* gpart, unsigned* counter,
+                                                                          unsigned group) {
+  using AT = typename AccT<P>::T;
+  __shared__ SplitSmem<P> t;
+  const unsigned slot = blockIdx.x / (unsigned)a.nrhs;
+  const int rhs = (int)(blockIdx.x - slot * (unsigned)a.nrhs);
+  const int i = threadIdx.x & 31;
+  const int64_t h = (int64_t)slot * SPLIT_SITES + i;
+  pdl_launch_dependents();
+  pdl_wait();
+  const bool skipped = a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride];
+  double red[E::NRED];
+#pragma unroll
+  for (int k = 0; k < E::NRED; ++k) red[k] = 0.0;
+  if (!skipped && h < a.g.Vh) wilson_split_stage<P, RECON, DAGGER>(a, rhs, h, i, t);
+  __syncthreads();
+  if (!skipped && threadIdx.x < 32 && h < a.g.Vh) {
+    cpx<AT> acc[12];
+    wilson_split_sum<P, DAGGER>(a, t, rhs, h, i, acc);
+    if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
+    e.site(rhs, h, acc, red);
+  }
+  const int rr[1] = {rhs};
+  const bool cc[1] = {!skipped}, hh[1] = {true};
+  grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
+                                    gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter);
 }
 
 // ---------------------------------------------------------------- FP16, two right-hand sides per thread
@@ -827,6 +1153,8 @@ constexpr int TILE16 = 32;
 // the y-rows per chunk of the blocked tile order for this lattice, rhs count
 // and tile size (dslash.cu)
 int tile_rows(const Geom& g, int nrhs, int ts = TILE16, int sbytes = 52);
+// the same for the full-lattice forms (dslash.cu); bytes a site touches
+int full_rows(const Geom& g, int64_t bytes);
 // bytes of one Wilson spinor per site and rhs (FP16: with its norm)
 template <int P> constexpr int spinor_bytes() { return P == P64 ? 192 : (P == P32 ? 96 : 52); }
 struct Tile16 {
@@ -1719,6 +2047,27 @@ __global__ void __launch_bounds__(256) staggered_hop_kernel(HopArgs a) {
 template <int P, int RECON>
 __global__ void __launch_bounds__(256, 3) staggered_hop_kernel_capped(HopArgs a) {
   staggered_hop_body<P, RECON>(a);
+}
+
+// Both checkerboards in one launch (as wilson_full_kernel): a staggered D reads
+// 1152 B of links per output site against 48 B of its neighbours' vectors, so
+// reading each link from DRAM once (672 instead of 1296 B per site) is most of it.
+template <int P, int RECON, int MINB>
+__global__ void __launch_bounds__(256, MINB) staggered_full_kernel(HopArgs a) {
+  using AT = typename AccT<P>::T;
+  int rhs, p;
+  unsigned slot;
+  full_block(a, rhs, p, slot);
+  const int64_t i = (int64_t)slot * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  if (p) flip_parity(a);
+  pdl_wait();
+  if (i >= a.g.Vh) return;
+  if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;
+  const int64_t h = full_site(a, i);
+  cpx<AT> acc[3];
+  staggered_hop_site<P, RECON>(a, rhs, h, acc);
+  staggered_finish_store<P>(a, rhs, h, acc);
 }
 
 // The tile form of the FP64 / FP32 staggered hop for several right-hand sides

@@ -339,6 +339,9 @@ struct HopSpec {
   int nrhs;
 };
 clg_status hop(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s);
+// both checkerboards of full fields (s.out_parity is ignored; in and out must
+// not overlap): one launch, or two hops where the autotuner found those faster
+clg_status hop_full(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s);
 // the kernel arguments of a hop (checked as hop() checks them), for callers
 // that launch a fused variant themselves
 struct HopArgs;

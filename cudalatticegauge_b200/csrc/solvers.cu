@@ -672,6 +672,9 @@ cudaError_t launch_hop_epi(clg_context_s* ctx, const HopArgs& a, const E& e, int
   if (a.seg)  // a batch of lattices
     return launch_pdl(ctx, wilson_hop_epi_kernel<P, RECON, DAG, 256, MINB, E, true>, grid, dim3(bs), 0, a, e,
                       ctx->red_partials, gpart, ctx->red_counter, group);
+  if (bs == SPLIT_SITES)  // four threads per site (bs: sites per block)
+    return launch_pdl(ctx, wilson_split_epi_kernel<P, RECON, DAG, E>, grid, dim3(4 * SPLIT_SITES), 0, a, e,
+                      ctx->red_partials, gpart, ctx->red_counter, group);
   return launch_pdl(ctx, wilson_hop_epi_kernel<P, RECON, DAG, 256, MINB, E>, grid, dim3(bs), 0, a, e,
                     ctx->red_partials, gpart, ctx->red_counter, group);
 }
@@ -713,7 +716,8 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   // odd checkerboard of each iteration run first and are tuned)
   HopSpec plain = s;
   plain.x = nullptr;
-  const int bs = tuned_hop_block(ctx, w.U, plain, P == P64 ? 64 : 128);
+  const int cfg1 = tuned_hop_config(ctx, w.U, plain, P == P64 ? 64 : 128);
+  const int bs = (cfg1 >> 16) == HOP_SPLIT ? SPLIT_SITES : cfg1 & 0xffff;
   if constexpr (P == P16) {
     const int tcfg = w.nrhs >= 2 && !a.seg ? tuned_hop_tile_config(ctx, w.U, plain, -1) : -1;
     if (tcfg >= 0) {
@@ -775,8 +779,9 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
 // The outer residual of a Wilson D / D^+ solve fused into the FP64 hop that
 // computes D x on parity par: r = b - D x is stored in FP64 and in the inner
 // precision PI (the next inner solve's right-hand side), and |r|^2 goes to
-// out[rhs] (the first parity sets it, the second adds), so neither the
-// separate residual pass nor the copy to the inner precision reads r again.
+// out[rhs] (the first parity sets it, the second adds; one launch of both
+// parities sets it once), so neither the separate residual pass nor the copy
+// to the inner precision reads r again.
 template <int PI>
 struct ResidHop {
   static constexpr int NRED = 1;
@@ -808,6 +813,34 @@ template <int PI>
 clg_status fused_residual_t(Work& w, bool dag, const FieldRef& b, const FieldRef& x, const FieldRef& r,
                             const FieldRef& rp, double* out) {
   clg_context_s* ctx = w.ctx;
+  if (w.nrhs == 1 && !w.U->seg && ctx->hop_config < 0) {
+    // one right-hand side: both parities in one launch (wilson_full_epi_kernel)
+    HopSpec s{};
+    s.kind = CLG_FERMION_WILSON;
+    s.prec = CLG_PREC_DOUBLE;
+    s.dagger = dag;
+    s.in = x;
+    s.out = r;
+    s.x = &x;
+    s.a = make_double2(-w.param, 0.0);
+    s.xa = make_double2(1.0, 0.0);
+    s.nrhs = 1;
+    HopArgs a;
+    if (clg_status st = make_hop_args(ctx, w.U, s, a)) return st;
+    a.tile_rows = full_rows(a.g, 4 * 144 + 4 * 192 + 12 * 8);
+    const ResidHop<PI> e{dfield(b), dfield(r), dfield(rp), 0, true, out};
+    constexpr int bs = 128;
+    const int64_t nslots = 2 * ((w.Vh + bs - 1) / bs);
+    if (clg_status st = ensure_reduction(ctx, red2_doubles(nslots, 1, 1, 1))) return st;
+    const unsigned group = red_group(nslots, 1);
+    double* gpart = ctx->red_partials + nslots;
+    auto kern = dag ? wilson_full_epi_kernel<P64, 18, true, 256, 2, ResidHop<PI>>
+                    : wilson_full_epi_kernel<P64, 18, false, 256, 2, ResidHop<PI>>;
+    const cudaError_t err = launch_pdl(ctx, kern, dim3((unsigned)nslots), dim3(bs), 0, a, e, ctx->red_partials, gpart,
+                                       ctx->red_counter, group);
+    if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("residual hop: ") + cudaGetErrorString(err));
+    return CLG_SUCCESS;
+  }
   for (int par = 0; par < 2; ++par) {
     HopSpec s{};
     s.kind = CLG_FERMION_WILSON;
