@@ -39,11 +39,12 @@ __global__ void __launch_bounds__(256)
 
 // The same over a batch of lattices (clg_solve_lattices): right-hand side r
 // holds rhs_vh[r] sites per checkerboard, the rest of the padded range is
-// skipped (it stays zero).
+// skipped (it stays zero).  A launch index is per_rhs consecutive ones per
+// right-hand side.
 template <int NRED, class F>
 __global__ void __launch_bounds__(256)
     site_reduce_batch_kernel(F f, int64_t nsites, int first_parity, int64_t Vh, double* partials, unsigned* counter,
-                             const int64_t* rhs_vh) {
+                             const int64_t* rhs_vh, int per_rhs) {
   const int rhs = blockIdx.y;
   pdl_launch_dependents();
   pdl_wait();
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int k = 0; k < (NRED > 0 ? NRED : 1); ++k) acc[k] = 0.0;
   if (f.active(rhs)) {
-    const int64_t vr = rhs_vh[rhs];
+    const int64_t vr = rhs_vh[rhs / per_rhs];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nsites; i += (int64_t)gridDim.x * blockDim.x) {
       const int pi = (int)(i / Vh);
       const int64_t h = i - (int64_t)pi * Vh;
@@ -80,9 +81,9 @@ clg_status launch_sites(clg_context_s* ctx, const F& f, int first_parity, int np
   }
   dim3 grid((unsigned)nb, (unsigned)nrhs);
   cudaError_t e;
-  if (ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs == ctx->batch_nrhs)
+  if (ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs % ctx->batch_nrhs == 0)
     e = launch_pdl(ctx, site_reduce_batch_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
-                   ctx->red_partials, ctx->red_counter, (const int64_t*)ctx->batch_vh);
+                   ctx->red_partials, ctx->red_counter, (const int64_t*)ctx->batch_vh, nrhs / ctx->batch_nrhs);
   else
     e = launch_pdl(ctx, site_reduce_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
                    ctx->red_partials, ctx->red_counter);
@@ -106,6 +107,34 @@ clg_status with_pn(int prec, int nc, Fn&& fn) {
   if (prec == 0) return fn(I0{}, N3{});
   if (prec == 1) return fn(I1{}, N3{});
   return fn(I2{}, N3{});
+}
+
+// A vector kernel that treats every component alike need not give a site to one
+// thread: a parity block of nc components (chunk-major) is also `pieces` blocks
+// of nc / pieces components, and a field seen that way has `pieces` times the
+// threads, a piece of the registers, and the same coalescing.  On 8^4 one
+// thread per Wilson site is 8 blocks for 148 SMs.  Wilson: FP64 in 4 pieces of
+// 3 components, FP32 in 3 of 4 (whole float4 chunks); FP16 stays whole (its
+// norm covers the site), and so do the 3 components of a staggered site.
+inline FieldRef pieces_view(const FieldRef& f, int pieces) {
+  FieldRef v = f;
+  v.nc = f.nc / pieces;
+  v.blk = f.blk / pieces;
+  v.nparity = f.nparity * pieces;
+  v.first_parity = f.first_parity * pieces;
+  return v;
+}
+template <class Fn>
+clg_status with_pieces(int prec, int nc, Fn&& fn) {
+  using I0 = std::integral_constant<int, 0>;
+  using I1 = std::integral_constant<int, 1>;
+  using I2 = std::integral_constant<int, 2>;
+  using N12 = std::integral_constant<int, 12>;
+  using N4 = std::integral_constant<int, 4>;
+  using N3 = std::integral_constant<int, 3>;
+  if (prec == 0) return fn(I0{}, N3{});
+  if (prec == 1) return nc == 12 ? fn(I1{}, N4{}) : fn(I1{}, N3{});
+  return nc == 12 ? fn(I2{}, N12{}) : fn(I2{}, N3{});
 }
 
 // Device-side view of a field for the functors.

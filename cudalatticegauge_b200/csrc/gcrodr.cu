@@ -40,7 +40,6 @@ namespace {
 
 using dense::Mat;
 using dense::Z;
-using hk::MD;
 using hk::MAXV;
 
 // the recycled subspace and the per-solve vectors, kept by the solver
@@ -132,7 +131,7 @@ clg_status gcrodr_solve(::clg_solver_s* S, clg_field_s* X, clg_field_s* B, clg_g
     }
     if (!st) {
       void* p = nullptr;
-      st = dalloc(ctx, &p, sizeof(double) * 2 * MD);
+      st = dalloc(ctx, &p, sizeof(double) * 2 * hk::MAXV);
       if (!st) {
         nw->allocs.push_back(p);
         nw->dev_out = static_cast<double*>(p);

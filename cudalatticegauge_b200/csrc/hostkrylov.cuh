@@ -1,7 +1,8 @@
 // hostkrylov.cuh -- FP64 Krylov building blocks driven from the host: one
 // right-hand side, the small dense algebra on the host (dense.h), every
-// orthogonalisation one multi-dot launch (up to MD inner products, read back)
-// and one linear-combination launch.  Used by the recycled solver (GCRO-DR)
+// orthogonalisation one multi-dot launch and one linear-combination launch per
+// pass, with the coefficients read back (HostKrylov::orthogonalise) or kept on
+// the device for a whole Arnoldi cycle (arnoldi_step).  Used by the recycled solver (GCRO-DR)
 // and by the multi-shift solvers that share one Krylov space over all shifts
 // (multi-shift FOM and BiCGStab-M), whose per-cycle work is dominated by the
 // operator applications, not by these launches.
@@ -18,27 +19,53 @@ namespace hk {
 
 using dense::Z;
 
-constexpr int MD = 16;    // inner products per multi-dot launch
-constexpr int MAXV = 34;  // vectors per linear combination (m + 1 <= 33, + 1)
+constexpr int MAXV = 34;  // vectors of one multi-dot or linear combination (m + 1 <= 33, + 1)
+constexpr int MDG = 4;    // inner products per block of a multi-dot
 
-template <int NC>
-struct MultiDotF {  // out[i] = sum_x conj(v_i(x)) w(x), i < n
-  DField w;
-  DField v[MD];
-  int n;
-  double* out;
-  __device__ bool active(int) const { return true; }
-  __device__ void operator()(int, int p, int64_t h, double* acc) const {
-    cpx<double> wv[NC];
-    ldv<P64, NC, double>(w, 0, p, h, wv);
+// The vectors of one launch by their data pointers; all have the shape of the
+// launch (HostVecs::proto), seen as NC / 3 times as many blocks of 3 components
+// (the storage is [parity][component][h], so a block is a run of 3 Vh complex
+// numbers): four times the threads of one per Wilson site, and a third of the
+// registers.
+struct VecTab {
+  const char* v[MAXV];
+};
+__device__ __forceinline__ void ld3(const char* v, int64_t off, int64_t kstride, cpx<double> o[3]) {
 #pragma unroll
-    for (int i = 0; i < MD; ++i) {
-      if (i >= n) break;
-      cpx<double> a[NC];
-      ldv<P64, NC, double>(v[i], 0, p, h, a);
+  for (int k = 0; k < 3; ++k) {
+    const double2 d = *reinterpret_cast<const double2*>(v + off + k * kstride);
+    o[k] = mk<double>(d.x, d.y);
+  }
+}
+
+// out[i] = s_i v_i^+ w for n vectors, MDG of them per block (right-hand side g
+// of the launch = vectors MDG g ..): w is read once per MDG vectors, and the
+// blocks of all vectors run side by side.  One block over all vectors reduced
+// 32 numbers per block on 32 blocks of 8^3x16 (19 us a launch whatever n).
+// With hcol the results are also added to (first: stored in) a Hessenberg
+// column.
+struct MultiDotF {
+  const char* w;
+  VecTab v;
+  int64_t blk, kstride;
+  int n;
+  const double* scale;  // device, nullable: s_i
+  double2* out;
+  double2* hcol;        // nullable
+  int first;
+  __device__ bool active(int) const { return true; }
+  __device__ void operator()(int g, int p, int64_t h, double* acc) const {
+    const int64_t off = p * blk + h * 16;
+    cpx<double> wv[3];
+    ld3(w, off, kstride, wv);
+#pragma unroll
+    for (int i = 0; i < MDG; ++i) {
+      if (MDG * g + i >= n) break;
+      cpx<double> a[3];
+      ld3(v.v[MDG * g + i], off, kstride, a);
       double re = 0.0, im = 0.0;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
+      for (int c = 0; c < 3; ++c) {
         re = fma(a[c].x, wv[c].x, fma(a[c].y, wv[c].y, re));
         im = fma(a[c].x, wv[c].y, fma(-a[c].y, wv[c].x, im));
       }
@@ -46,40 +73,76 @@ struct MultiDotF {  // out[i] = sum_x conj(v_i(x)) w(x), i < n
       acc[2 * i + 1] += im;
     }
   }
-  __device__ void finalize(int, const double* s) const {
-    for (int k = 0; k < 2 * n; ++k) out[k] = s[k];
+  __device__ void finalize(int g, const double* s) const {
+#pragma unroll
+    for (int i = 0; i < MDG; ++i) {
+      const int k = MDG * g + i;
+      if (k >= n) break;
+      const double sc = scale ? scale[k] : 1.0;
+      const double2 d = make_double2(sc * s[2 * i], sc * s[2 * i + 1]);
+      out[k] = d;
+      if (hcol) hcol[k] = first ? d : make_double2(hcol[k].x + d.x, hcol[k].y + d.y);
+    }
   }
 };
 
-template <int NC>
-struct LinCombF {  // out = beta out + sum_i c_i v_i
-  DField out;
-  DField v[MAXV];
+// out_r = beta in_r + sum_i c_(r,i) s_i v_i for the `rhs` outputs r of the
+// launch (ostride bytes apart); the coefficients are kernel arguments (c) or
+// device-resident (dc, times sign).  NRED = 1 also reduces |out|^2: its root
+// goes to hn and its reciprocal (0 for a zero vector) to inv.
+template <int NRED>
+struct LinCombF {
+  char* out;
+  const char* in;
+  int64_t ostride;
+  VecTab v;
   double2 c[MAXV];
+  const double2* dc;
+  const double* scale;
+  double sign;
   double2 beta;
+  int64_t blk, kstride;
   int n;
+  double2* hn;
+  double* inv;
   __device__ bool active(int) const { return true; }
-  __device__ void operator()(int, int p, int64_t h, double*) const {
-    cpx<double> o[NC];
+  __device__ void operator()(int r, int p, int64_t h, double* acc) const {
+    const int64_t off = p * blk + h * 16;
+    cpx<double> o[3];
     if (beta.x != 0.0 || beta.y != 0.0) {
-      ldv<P64, NC, double>(out, 0, p, h, o);
+      ld3(in + r * ostride, off, kstride, o);
       const cpx<double> b = mk<double>(beta.x, beta.y);
 #pragma unroll
-      for (int k = 0; k < NC; ++k) o[k] = b * o[k];
+      for (int k = 0; k < 3; ++k) o[k] = b * o[k];
     } else {
 #pragma unroll
-      for (int k = 0; k < NC; ++k) o[k] = mk<double>(0, 0);
+      for (int k = 0; k < 3; ++k) o[k] = mk<double>(0, 0);
     }
+#pragma unroll 4
     for (int i = 0; i < n; ++i) {
-      cpx<double> a[NC];
-      ldv<P64, NC, double>(v[i], 0, p, h, a);
-      const cpx<double> ci = mk<double>(c[i].x, c[i].y);
+      cpx<double> a[3];
+      ld3(v.v[i], off, kstride, a);
+      double2 ci = dc ? dc[r * n + i] : c[i];
+      const double sc = (scale ? scale[i] : 1.0) * sign;
+      const cpx<double> cc = mk<double>(sc * ci.x, sc * ci.y);
 #pragma unroll
-      for (int k = 0; k < NC; ++k) o[k] = o[k] + ci * a[k];
+      for (int k = 0; k < 3; ++k) o[k] = o[k] + cc * a[k];
     }
-    stv<P64, NC, double>(out, 0, p, h, o);
+    char* q = out + r * ostride + off;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) *reinterpret_cast<double2*>(q + k * kstride) = make_double2(o[k].x, o[k].y);
+    if constexpr (NRED > 0) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) acc[0] = fma(o[k].x, o[k].x, fma(o[k].y, o[k].y, acc[0]));
+    }
   }
-  __device__ void finalize(int, const double*) const {}
+  __device__ void finalize(int, const double* s) const {
+    if constexpr (NRED > 0) {
+      const double d = sqrt(s[0]);
+      if (hn) *hn = make_double2(d, 0.0);
+      if (inv) *inv = d > 0.0 ? 1.0 / d : 0.0;
+    }
+  }
 };
 
 // device vectors of one shape owned by a solver cache
@@ -113,7 +176,7 @@ struct HostVecs : SolveCacheBase {
   }
   clg_status out_buffer() {
     void* p = nullptr;
-    if (clg_status st = dalloc(ctx, &p, sizeof(double) * 2 * MD)) return st;
+    if (clg_status st = dalloc(ctx, &p, sizeof(double) * 2 * MAXV)) return st;
     allocs.push_back(p);
     dev_out = static_cast<double*>(p);
     return CLG_SUCCESS;
@@ -129,33 +192,37 @@ struct HostKrylov {
   int64_t Vh;
   int apps = 0;
 
-  clg_status apply(const FieldRef& out, const FieldRef& in) {
+  clg_status apply(const FieldRef& out, const FieldRef& in, const double* scale = nullptr) {
     ++apps;
-    return apply_op(ctx, op, Ug, kind, param, out, in, &W.tmp, make_double2(1.0, 0.0), 1);
+    return apply_op(ctx, op, Ug, kind, param, out, in, &W.tmp, make_double2(1.0, 0.0), 1, scale);
+  }
+  // blocks of 3 components of a vector (VecTab)
+  int blocks() const { return W.proto.nparity * (nc / 3); }
+  int64_t block_bytes() const { return 3 * Vh * 16; }
+  // device out[i] = s_i v_i^+ w (and the Hessenberg column), no host read
+  clg_status dots_dev(const FieldRef& w, const FieldRef* const* vs, int n, double2* out, const double* scale = nullptr,
+                      double2* hcol = nullptr, bool first = true) {
+    if (n > MAXV) return ctx->fail(CLG_ERR_UNSUPPORTED, "too many vectors in one multi-dot");
+    MultiDotF f;
+    f.w = w.data;
+    for (int i = 0; i < n; ++i) f.v.v[i] = vs[i]->data;
+    for (int i = n; i < MAXV; ++i) f.v.v[i] = nullptr;
+    f.blk = block_bytes();
+    f.kstride = Vh * 16;
+    f.n = n;
+    f.scale = scale;
+    f.out = out;
+    f.hcol = hcol;
+    f.first = first;
+    return launch_sites<2 * MDG>(ctx, f, 0, blocks(), Vh, (n + MDG - 1) / MDG);
   }
   // out[i] = v_i^+ w for the n vectors vs (n arbitrary), read to the host
   clg_status dots(const FieldRef& w, const std::vector<const FieldRef*>& vs, std::vector<Z>& out) {
     out.assign(vs.size(), Z(0.0, 0.0));
-    for (size_t i0 = 0; i0 < vs.size(); i0 += MD) {
-      const int n = (int)std::min<size_t>(MD, vs.size() - i0);
-      clg_status st;
-      if (nc == 12) {
-        MultiDotF<12> f;
-        f.w = dfield(w);
-        for (int i = 0; i < MD; ++i) f.v[i] = dfield(*vs[i0 + std::min(i, n - 1)]);
-        f.n = n;
-        f.out = W.dev_out;
-        st = launch_sites<2 * MD>(ctx, f, W.proto.first_parity, W.proto.nparity, Vh, 1);
-      } else {
-        MultiDotF<3> f;
-        f.w = dfield(w);
-        for (int i = 0; i < MD; ++i) f.v[i] = dfield(*vs[i0 + std::min(i, n - 1)]);
-        f.n = n;
-        f.out = W.dev_out;
-        st = launch_sites<2 * MD>(ctx, f, W.proto.first_parity, W.proto.nparity, Vh, 1);
-      }
-      if (st) return st;
-      double h[2 * MD];
+    for (size_t i0 = 0; i0 < vs.size(); i0 += MAXV) {
+      const int n = (int)std::min<size_t>(MAXV, vs.size() - i0);
+      if (clg_status st = dots_dev(w, vs.data() + i0, n, reinterpret_cast<double2*>(W.dev_out))) return st;
+      double h[2 * MAXV];
       cudaError_t e = cudaMemcpyAsync(h, W.dev_out, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, ctx->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
       if (e != cudaSuccess) return ctx->fail(cuda_status(e), cudaGetErrorString(e));
@@ -168,26 +235,33 @@ struct HostKrylov {
     if (dots(a, {&a}, d)) return -1.0;
     return std::sqrt(std::max(d[0].real(), 0.0));
   }
+  template <int NRED>
+  LinCombF<NRED> combination(const FieldRef& out, const FieldRef& in, Z beta, const FieldRef* const* vs, int n) const {
+    LinCombF<NRED> f;
+    f.out = out.data;
+    f.in = in.data;
+    f.ostride = out.rstride;
+    for (int i = 0; i < MAXV; ++i) {
+      f.v.v[i] = i < n ? vs[i]->data : nullptr;
+      f.c[i] = make_double2(0.0, 0.0);
+    }
+    f.dc = nullptr;
+    f.scale = nullptr;
+    f.sign = 1.0;
+    f.beta = make_double2(beta.real(), beta.imag());
+    f.blk = block_bytes();
+    f.kstride = Vh * 16;
+    f.n = n;
+    f.hn = nullptr;
+    f.inv = nullptr;
+    return f;
+  }
   // out = beta out + sum_i c_i v_i
   clg_status lincomb(const FieldRef& out, Z beta, const std::vector<const FieldRef*>& vs, const std::vector<Z>& c) {
     if (vs.size() > (size_t)MAXV) return ctx->fail(CLG_ERR_UNSUPPORTED, "too many vectors in one linear combination");
-    auto fill = [&](auto& f) {
-      f.out = dfield(out);
-      f.n = (int)vs.size();
-      f.beta = make_double2(beta.real(), beta.imag());
-      for (size_t i = 0; i < vs.size(); ++i) {
-        f.v[i] = dfield(*vs[i]);
-        f.c[i] = make_double2(c[i].real(), c[i].imag());
-      }
-    };
-    if (nc == 12) {
-      LinCombF<12> f;
-      fill(f);
-      return launch_sites<0>(ctx, f, W.proto.first_parity, W.proto.nparity, Vh, 1);
-    }
-    LinCombF<3> f;
-    fill(f);
-    return launch_sites<0>(ctx, f, W.proto.first_parity, W.proto.nparity, Vh, 1);
+    LinCombF<0> f = combination<0>(out, out, beta, vs.data(), (int)vs.size());
+    for (size_t i = 0; i < vs.size(); ++i) f.c[i] = make_double2(c[i].real(), c[i].imag());
+    return launch_sites<0>(ctx, f, 0, blocks(), Vh, 1);
   }
   clg_status copy(const FieldRef& dst, const FieldRef& src) { return lincomb(dst, Z(0.0, 0.0), {&src}, {Z(1.0, 0.0)}); }
   clg_status scale(const FieldRef& a, Z s) { return lincomb(a, s, {}, {}); }
@@ -207,6 +281,52 @@ struct HostKrylov {
     return CLG_SUCCESS;
   }
 };
+
+// Device state of an Arnoldi cycle (arnoldi_step): the basis vectors are
+// V'_i = v_i / s_i, not normalised, so that no pass over a vector only scales
+// it; d holds the inner products of the current pass.
+struct ArnoldiState {
+  double2 d[MAXV];
+  double2 H[(MAXV - 1) * MAXV];  // column j at H + j MAXV, h_(j+1,j) included
+  double2 norm;                  // of the vector arnoldi_start normalised
+  double s[MAXV];
+};
+
+// V'_0 = scale-free copy of src, s_0 = 1 / |src|, norm = |src|
+inline clg_status arnoldi_start(HostKrylov& K, ArnoldiState* st, const FieldRef& v0, const FieldRef& src) {
+  auto f = K.combination<1>(v0, src, Z(1.0, 0.0), nullptr, 0);
+  f.hn = &st->norm;
+  f.inv = &st->s[0];
+  return launch_sites<1>(K.ctx, f, 0, K.blocks(), K.Vh, 1);
+}
+// Column j of the Arnoldi relation: w = A v_j orthogonalised against
+// v_0 .. v_j by classical Gram-Schmidt twice, left in next = V'_(j+1), all of
+// it on the device: 4 launches after the operator, no host read.  The host
+// reads the whole H at the end of a cycle.
+inline clg_status arnoldi_step(HostKrylov& K, ArnoldiState* st, const FieldRef* const* V, int j, const FieldRef& w,
+                               const FieldRef& next) {
+  if (clg_status e = K.apply(w, *V[j], &st->s[j])) return e;
+  double2* hcol = st->H + (size_t)j * MAXV;
+  for (int pass = 0; pass < 2; ++pass) {
+    if (clg_status e = K.dots_dev(w, V, j + 1, st->d, st->s, hcol, pass == 0)) return e;
+    if (pass == 0) {
+      auto f = K.combination<0>(w, w, Z(1.0, 0.0), V, j + 1);
+      f.dc = st->d;
+      f.scale = st->s;
+      f.sign = -1.0;
+      if (clg_status e = launch_sites<0>(K.ctx, f, 0, K.blocks(), K.Vh, 1)) return e;
+    } else {
+      auto f = K.combination<1>(next, w, Z(1.0, 0.0), V, j + 1);
+      f.dc = st->d;
+      f.scale = st->s;
+      f.sign = -1.0;
+      f.hn = hcol + j + 1;
+      f.inv = &st->s[j + 1];
+      if (clg_status e = launch_sites<1>(K.ctx, f, 0, K.blocks(), K.Vh, 1)) return e;
+    }
+  }
+  return CLG_SUCCESS;
+}
 
 }  // namespace hk
 }  // namespace clg

@@ -464,30 +464,41 @@ struct GmStart {
   }
 };
 
-// h_ij = s_i <V'_i, w>, i <= J: J+1 dot products (2(J+1) reductions) in one pass;
-// J is a template argument so the reduction width matches the column
-template <int P, int NC, int J>
-struct GmDotsJ {
+// h_ij = s_i <V'_i, w>, i <= j: the column's j + 1 dot products, GM_DG of them
+// per block (launch index y = rhs * groups + group), so that the groups run
+// side by side and a block reduces 2 GM_DG numbers; one block over all columns
+// took 8-21 us a launch on 8^4, growing with j.
+constexpr int GM_DG = 4;
+template <int P, int NC>
+struct GmDots {
   VList V;
   DField w;
   KState* st;
-  __device__ bool active(int q) const { return !st[q].skip; }
-  __device__ void operator()(int rhs, int par, int64_t h, double* acc) const {
+  int j, groups;
+  __device__ bool active(int y) const { return !st[y / groups].skip; }
+  __device__ void operator()(int y, int par, int64_t h, double* acc) const {
     using AT = typename AccT<P>::T;
+    const int rhs = y / groups, i0 = GM_DG * (y - rhs * groups);
     cpx<AT> vw[NC];
     ldv<P, NC, AT>(w, rhs, par, h, vw);
 #pragma unroll
-    for (int i = 0; i <= J; ++i) {
+    for (int i = 0; i < GM_DG; ++i) {
+      if (i0 + i > j) break;
       cpx<AT> vi[NC];
-      ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
+      ldv<P, NC, AT>(V.v[i0 + i], rhs, par, h, vi);
       acc_dot<NC, AT>(vi, vw, acc + 2 * i);
     }
   }
-  __device__ void finalize(int q, const double* s) const {
-    KState& k = st[q];
+  __device__ void finalize(int y, const double* s) const {
+    const int rhs = y / groups, g = y - rhs * groups;
+    KState& k = st[rhs];
     if (k.skip) return;
-    k.iters += 1;
-    for (int i = 0; i <= J; ++i) k.H[i * GM_MAXK + J] = make_double2(k.s[i] * s[2 * i], k.s[i] * s[2 * i + 1]);
+    if (g == 0) k.iters += 1;
+#pragma unroll
+    for (int i = 0; i < GM_DG; ++i) {
+      const int c = GM_DG * g + i;
+      if (c <= j) k.H[c * GM_MAXK + j] = make_double2(k.s[c] * s[2 * i], k.s[c] * s[2 * i + 1]);
+    }
   }
 };
 
@@ -504,9 +515,8 @@ struct GmOrtho {
     const KState& k = st[rhs];
     cpx<AT> vw[NC];
     ldv<P, NC, AT>(w, rhs, par, h, vw);
-#pragma unroll
-    for (int i = 0; i < GM_MAXK; ++i) {
-      if (i > j) break;
+#pragma unroll 4
+    for (int i = 0; i <= j; ++i) {
       cpx<AT> vi[NC];
       ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
       const double2 c = k.H[i * GM_MAXK + j];
@@ -522,18 +532,34 @@ struct GmOrtho {
     if (k.skip) return;
     const double hn = sqrt(s[0]);
     double2* H = k.H;
-    H[(j + 1) * GM_MAXK + j] = make_double2(hn, 0.0);
     k.s[j + 1] = hn > 0.0 ? 1.0 / hn : 0.0;
-    // apply the previous rotations to column j (RotateH, CSolverGMRES.cpp:262-327, incrementally)
-    for (int i = 0; i < j; ++i) {
-      const double2 hij = H[i * GM_MAXK + j], hi1 = H[(i + 1) * GM_MAXK + j];
-      H[i * GM_MAXK + j] = make_double2(0, 0);
-      const double2 a = cmul(cconj(k.cs[i]), hij), b = cmul(cconj(k.sn[i]), hi1);
-      H[i * GM_MAXK + j] = make_double2(a.x + b.x, a.y + b.y);
-      const double2 c = cmul(k.cs[i], hi1), d = cmul(k.sn[i], hij);
-      H[(i + 1) * GM_MAXK + j] = make_double2(c.x - d.x, c.y - d.y);
+    // apply the previous rotations to column j (RotateH, CSolverGMRES.cpp:262-327,
+    // incrementally); the column and the rotations are loaded before the first
+    // is used (one thread walking them took a global round trip per rotation)
+    double2 hc[GM_MAXK + 1], ci[GM_MAXK], si[GM_MAXK];
+#pragma unroll
+    for (int i = 0; i < GM_MAXK; ++i) {
+      hc[i] = i <= j ? H[i * GM_MAXK + j] : make_double2(i == j + 1 ? hn : 0.0, 0.0);
+      ci[i] = i < j ? k.cs[i] : make_double2(0.0, 0.0);
+      si[i] = i < j ? k.sn[i] : make_double2(0.0, 0.0);
     }
-    const double2 hjj = H[j * GM_MAXK + j], hj1 = H[(j + 1) * GM_MAXK + j];
+    hc[GM_MAXK] = make_double2(j + 1 == GM_MAXK ? hn : 0.0, 0.0);
+    const double2 gj = k.g[j];
+    const double tol2 = k.tol2, rr0 = k.rr0;
+    double2 hjj = hc[0], hj1 = hc[1];
+#pragma unroll
+    for (int i = 0; i < GM_MAXK; ++i) {
+      if (i < j) {
+        const double2 a = cmul(cconj(ci[i]), hc[i]), b = cmul(cconj(si[i]), hc[i + 1]);
+        const double2 c = cmul(ci[i], hc[i + 1]), d = cmul(si[i], hc[i]);
+        H[i * GM_MAXK + j] = make_double2(a.x + b.x, a.y + b.y);
+        hc[i + 1] = make_double2(c.x - d.x, c.y - d.y);
+      }
+      if (i == j) {
+        hjj = hc[i];
+        hj1 = hc[i + 1];
+      }
+    }
     const double den = sqrt(hjj.x * hjj.x + hjj.y * hjj.y + hj1.x * hj1.x + hj1.y * hj1.y);
     if (!(den > 0.0) || bad(den)) {
       k.status = ST_BREAKDOWN;
@@ -545,15 +571,14 @@ struct GmOrtho {
     k.sn[j] = sn;
     H[j * GM_MAXK + j] = make_double2(den, 0.0);
     H[(j + 1) * GM_MAXK + j] = make_double2(0.0, 0.0);
-    const double2 gj = k.g[j];
     const double2 m = cmul(sn, gj);
     k.g[j + 1] = make_double2(-m.x, -m.y);
     k.g[j] = cmul(cconj(cs), gj);
     k.j = j + 1;
-    const double2 gn = k.g[j + 1];
-    k.resid_est = sqrt(gn.x * gn.x + gn.y * gn.y);
+    const double est = sqrt(m.x * m.x + m.y * m.y);
+    k.resid_est = est;
     // happy breakdown or converged: stop extending this cycle
-    if (k.resid_est * k.resid_est <= k.tol2 * k.rr0 || hn == 0.0) k.skip = 1;
+    if (est * est <= tol2 * rr0 || hn == 0.0) k.skip = 1;
   }
 };
 
@@ -573,7 +598,9 @@ struct GmUpdate {
     const KState& k = st[rhs];
     cpx<AT> vx[NC];
     ldv<P, NC, AT>(x, rhs, par, h, vx);
-    for (int i = 0; i < k.j; ++i) {
+    const int kj = k.j;
+#pragma unroll 4
+    for (int i = 0; i < kj; ++i) {
       cpx<AT> vi[NC];
       ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
       const double2 c = k.y[i];

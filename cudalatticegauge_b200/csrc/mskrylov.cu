@@ -16,8 +16,10 @@
 // B200 form: FP64 vectors on the device (the reference's precision for this
 // solver), the Arnoldi orthogonalisation by classical Gram-Schmidt applied
 // twice (one multi-dot and one linear-combination launch per pass; the
-// reference uses modified Gram-Schmidt with one launch per inner product), the
-// m x m shifted systems on the host.  A final batched FP64 defect correction
+// reference uses modified Gram-Schmidt with one launch per inner product) with
+// every coefficient on the device, one host read per cycle; the m x m shifted
+// Hessenberg systems on the host (Givens rotations, O(m^2)) and one launch that
+// adds the cycle's basis to every shift's solution.  A final batched FP64 defect correction
 // (the shifts as right-hand sides, GMRES inside) checks every shift's true
 // residual and refines any shift the recurrence left above tol_true_rel.
 #include <algorithm>
@@ -44,7 +46,78 @@ struct FomWork : hk::HostVecs {
   std::vector<FieldRef> V;  // the cycle's basis v_0 .. v_{m-1}
   FieldRef w, R;            // Arnoldi workspace, the next start vector v_m
   FieldRef X;               // the nshift solutions (FP64, right-hand sides = shifts)
+  hk::ArnoldiState* st = nullptr;  // device
+  double2* coef = nullptr;         // device, [shift][vector]
+  clg_status arnoldi_buffers(int ns) {
+    void* p = nullptr;
+    if (clg_status e = dalloc(ctx, &p, sizeof(hk::ArnoldiState))) return e;
+    allocs.push_back(p);
+    st = static_cast<hk::ArnoldiState*>(p);
+    if (clg_status e = dalloc(ctx, &p, sizeof(double2) * hk::MAXV * ns)) return e;
+    allocs.push_back(p);
+    coef = static_cast<double2*>(p);
+    return CLG_SUCCESS;
+  }
 };
+
+// The cycle's host copy of the Hessenberg matrix and scales
+clg_status read_arnoldi(clg_context_s* ctx, const FomWork& W, hk::ArnoldiState& h) {
+  cudaError_t e = cudaMemcpyAsync(&h, W.st, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  return e == cudaSuccess ? CLG_SUCCESS : ctx->fail(cuda_status(e), cudaGetErrorString(e));
+}
+Z hess(const hk::ArnoldiState& h, int r, int c) {
+  const double2 v = h.H[(size_t)c * hk::MAXV + r];
+  return r > c + 1 ? Z(0.0, 0.0) : Z(v.x, v.y);
+}
+
+// A y = g for an upper Hessenberg A with as many rows as columns, or one row
+// more (then the least-squares solution): Givens rotations and back
+// substitution.  False for a (numerically) singular A.
+bool hess_solve(Mat A, std::vector<Z> g, std::vector<Z>& y) {
+  const int m = A.cols;
+  double fro = 0.0;
+  for (const Z& v : A.a) fro += std::norm(v);
+  const double least = std::max(1e-14 * std::sqrt(fro), 1e-300);
+  for (int j = 0; j < std::min(m, A.rows - 1); ++j) {
+    const Z a = A(j, j), b = A(j + 1, j);
+    const double r = std::sqrt(std::norm(a) + std::norm(b));
+    if (!(r > least)) return false;
+    const Z c = std::conj(a) / r, s = std::conj(b) / r;
+    for (int k = j; k < m; ++k) {
+      const Z x = A(j, k), w = A(j + 1, k);
+      A(j, k) = c * x + s * w;
+      A(j + 1, k) = (a * w - b * x) / r;
+    }
+    const Z x = g[j], w = g[j + 1];
+    g[j] = c * x + s * w;
+    g[j + 1] = (a * w - b * x) / r;
+  }
+  y.assign(m, Z(0.0, 0.0));
+  for (int j = m - 1; j >= 0; --j) {
+    Z s = g[j];
+    for (int l = j + 1; l < m; ++l) s -= A(j, l) * y[l];
+    if (!(std::abs(A(j, j)) > least)) return false;
+    y[j] = s / A(j, j);
+  }
+  return true;
+}
+
+// x_n += sum_i y_(n,i) v_i for every shift n (y: ns rows of dim) in one launch
+clg_status add_basis(hk::HostKrylov& K, FomWork& W, const FieldRef& X, int ns, const std::vector<Z>& y, int dim) {
+  if (cudaMemcpyAsync(W.coef, y.data(), sizeof(Z) * ns * dim, cudaMemcpyHostToDevice, K.ctx->stream) != cudaSuccess)
+    return K.ctx->fail(CLG_ERR_CUDA, "multi-shift: coefficient upload");
+  std::vector<const FieldRef*> vs;
+  for (int i = 0; i < dim; ++i) vs.push_back(&W.V[i]);
+  auto f = K.combination<0>(X, X, Z(1.0, 0.0), vs.data(), dim);
+  f.dc = W.coef;
+  f.scale = W.st->s;
+  return launch_sites<0>(K.ctx, f, 0, K.blocks(), K.Vh, ns);
+}
+// all of X = 0
+clg_status zero_solutions(hk::HostKrylov& K, const FieldRef& X, int ns) {
+  return launch_sites<0>(K.ctx, K.combination<0>(X, X, Z(0.0, 0.0), nullptr, 0), 0, K.blocks(), K.Vh, ns);
+}
 
 template <int NC>
 struct ConjF {  // y = conj(y), elementwise (CField::Dagger)
@@ -95,6 +168,7 @@ clg_status fom_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cache
     if (!st) st = nw->vec(nw->R);
     if (!st) st = nw->full_vec(nw->tmp);
     if (!st) st = nw->out_buffer();
+    if (!st) st = nw->arnoldi_buffers(ns);
     if (!st) {  // the solutions: one allocation, shift k is right-hand side k
       void* p = nullptr;
       st = dalloc(ctx, &p, (size_t)nw->proto.rstride * ns);
@@ -111,69 +185,62 @@ clg_status fom_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cache
     cache = std::move(nw);
   }
   hk::HostKrylov K{ctx, *W, U, kind, op, nc, param, Vh};
-  auto xk = [&](int k) {
-    FieldRef f = W->X;
-    f.data = W->X.data + (int64_t)k * W->X.rstride;
-    f.nrhs = 1;
-    return f;
-  };
   clg_status st;
-  for (int k = 0; k < ns; ++k)
-    if ((st = K.scale(xk(k), Z(0.0, 0.0)))) return st;
+  if ((st = zero_solutions(K, W->X, ns))) return st;
   *X_out = &W->X;
   *apps_out = 0;
   *cycles_out = 0;
-  const double bnorm = K.norm(b);
-  if (bnorm < 0) return ctx->fail(CLG_ERR_CUDA, "multi-shift FOM: reading |b|");
-  if (bnorm == 0.0) return CLG_SUCCESS;
   // v_0 = b / |b|, beta_n = |b| for every shift (CMultiShiftFOM.cpp:141-160)
-  if ((st = K.lincomb(W->R, Z(0.0, 0.0), {&b}, {Z(1.0 / bnorm, 0.0)}))) return st;
-  std::vector<Z> beta(ns, Z(bnorm, 0.0));
+  if ((st = hk::arnoldi_start(K, W->st, W->V[0], b))) return st;
+  hk::ArnoldiState h;
+  double bnorm = 0.0;
+  std::vector<Z> beta(ns);
   std::vector<int> active(ns, 1);
   for (int cyc = 0; cyc < restart; ++cyc) {
     ++*cycles_out;
-    if ((st = K.copy(W->V[0], W->R))) return st;
-    Mat H(m + 1, m);
-    int dim = m;
-    for (int j = 0; j < m; ++j) {
-      if ((st = K.apply(W->w, W->V[j]))) return st;
-      std::vector<const FieldRef*> vs;
-      for (int i = 0; i <= j; ++i) vs.push_back(&W->V[i]);
-      std::vector<Z> h;
-      if ((st = K.orthogonalise(W->w, vs, h))) return st;
-      for (int i = 0; i <= j; ++i) H(i, j) = h[i];
-      const double hn = K.norm(W->w);
-      if (hn < 0) return ctx->fail(CLG_ERR_CUDA, "multi-shift FOM: reading |w|");
-      H(j + 1, j) = Z(hn, 0.0);
-      if (hn <= 1e-300 * bnorm) {  // invariant subspace: the solution lies in V_{j+1}
-        dim = j + 1;
-        break;
+    std::vector<const FieldRef*> V;
+    for (int j = 0; j < m; ++j) V.push_back(&W->V[j]);
+    for (int j = 0; j < m; ++j)
+      if ((st = hk::arnoldi_step(K, W->st, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
+    if ((st = read_arnoldi(ctx, *W, h))) return st;
+    if (cyc == 0) {
+      bnorm = h.norm.x;
+      if (!(bnorm >= 0)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift FOM: NaN in the right-hand side");
+      if (bnorm == 0.0) {
+        *cycles_out = 0;
+        return CLG_SUCCESS;
       }
-      const FieldRef& next = (j + 1 < m) ? W->V[j + 1] : W->R;
-      if ((st = K.lincomb(next, Z(0.0, 0.0), {&W->w}, {Z(1.0 / hn, 0.0)}))) return st;
+      std::fill(beta.begin(), beta.end(), Z(bnorm, 0.0));
     }
+    int dim = m;
+    for (int j = 0; j < m && dim == m; ++j)  // invariant subspace: the solution lies in V_{j+1}
+      if (hess(h, j + 1, j).real() <= 1e-300 * bnorm) dim = j + 1;
     double worst = 0.0;
+    std::vector<Z> Y((size_t)ns * dim, Z(0.0, 0.0));
     for (int n = 0; n < ns; ++n) {
       if (!active[n]) continue;
       Mat Hc(dim, dim);
       for (int r = 0; r < dim; ++r)
-        for (int c = 0; c < dim; ++c) Hc(r, c) = H(r, c) + (r == c ? Z(shifts[n].x, shifts[n].y) : Z(0.0, 0.0));
+        for (int c = 0; c < dim; ++c) Hc(r, c) = hess(h, r, c) + (r == c ? Z(shifts[n].x, shifts[n].y) : Z(0.0, 0.0));
       std::vector<Z> g(dim, Z(0.0, 0.0)), y;
       g[0] = beta[n];
-      if (!dense::lstsq(Hc, g, y)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift FOM: singular shifted Hessenberg");
-      std::vector<const FieldRef*> vs;
-      for (int i = 0; i < dim; ++i) vs.push_back(&W->V[i]);
-      const FieldRef x = xk(n);
-      if ((st = K.lincomb(x, Z(1.0, 0.0), vs, y))) return st;
+      if (!hess_solve(Hc, g, y)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift FOM: singular shifted Hessenberg");
+      std::copy(y.begin(), y.end(), Y.begin() + (size_t)n * dim);
       // the next residual of this shift: beta_n v_m (CMultiShiftFOM.cpp:227-229)
-      beta[n] = (dim == m) ? -H(m, m - 1).real() * y[m - 1] : Z(0.0, 0.0);
+      beta[n] = (dim == m && hess(h, m, m - 1).real() > 1e-300 * bnorm) ? -hess(h, m, m - 1).real() * y[m - 1]
+                                                                       : Z(0.0, 0.0);
       const double bl = std::abs(beta[n]);
       if (!(bl == bl)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift FOM: NaN in the recurrence");
       if (bl <= tol * bnorm) active[n] = 0;
       worst = std::max(worst, bl);
     }
+    if ((st = add_basis(K, *W, W->X, ns, Y, dim))) return st;
     *apps_out += dim;
     if (worst <= tol * bnorm || dim < m) break;
+    // the next cycle starts from v_m: its vector and scale
+    std::swap(W->V[0], W->R);
+    if (cudaMemcpyAsync(&W->st->s[0], &W->st->s[m], sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess)
+      return ctx->fail(CLG_ERR_CUDA, "multi-shift FOM: restart");
   }
   return CLG_SUCCESS;
 }
@@ -212,6 +279,7 @@ clg_status gmres_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cac
     if (!st) st = nw->vec(nw->R);
     if (!st) st = nw->full_vec(nw->tmp);
     if (!st) st = nw->out_buffer();
+    if (!st) st = nw->arnoldi_buffers(ns);
     if (!st) {
       void* p = nullptr;
       st = dalloc(ctx, &p, (size_t)nw->proto.rstride * ns);
@@ -228,76 +296,61 @@ clg_status gmres_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cac
     cache = std::move(nw);
   }
   hk::HostKrylov K{ctx, *W, U, kind, op, nc, param, Vh};
-  auto xk = [&](int k) {
-    FieldRef f = W->X;
-    f.data = W->X.data + (int64_t)k * W->X.rstride;
-    f.nrhs = 1;
-    return f;
-  };
   const Z zero(0.0, 0.0), one(1.0, 0.0);
   FieldRef& xs = W->V[m];
   clg_status st;
-  for (int k = 0; k < ns; ++k)
-    if ((st = K.scale(xk(k), zero))) return st;
-  if ((st = K.scale(xs, zero))) return st;
+  if ((st = zero_solutions(K, W->X, ns)) || (st = K.scale(xs, zero))) return st;
   *X_out = &W->X;
   *apps_out = 0;
   *cycles_out = 0;
-  const double bnorm = K.norm(b);
-  if (bnorm < 0) return ctx->fail(CLG_ERR_CUDA, "multi-shift GMRES: reading |b|");
-  if (bnorm == 0.0) return CLG_SUCCESS;
+  hk::ArnoldiState h;
+  double bnorm = 0.0;
   std::vector<Z> beta0(ns, one);
   for (int cyc = 0; cyc < restart; ++cyc) {
-    ++*cycles_out;
     // the seed residual: b, then b - A x_seed (CMultiShiftGMRES.cpp:158-172)
     if (cyc == 0) {
-      if ((st = K.copy(W->R, b))) return st;
+      if ((st = hk::arnoldi_start(K, W->st, W->V[0], b))) return st;
     } else {
-      if ((st = K.apply(W->w, xs)) || (st = K.lincomb(W->R, zero, {&b, &W->w}, {one, -one}))) return st;
+      if ((st = K.apply(W->w, xs)) || (st = K.lincomb(W->R, zero, {&b, &W->w}, {one, -one})) ||
+          (st = hk::arnoldi_start(K, W->st, W->V[0], W->R)))
+        return st;
     }
-    const double beta = K.norm(W->R);
-    if (beta < 0) return ctx->fail(CLG_ERR_CUDA, "multi-shift GMRES: reading |r|");
+    std::vector<const FieldRef*> V;
+    for (int j = 0; j < m; ++j) V.push_back(&W->V[j]);
+    for (int j = 0; j < m; ++j)
+      if ((st = hk::arnoldi_step(K, W->st, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
+    if ((st = read_arnoldi(ctx, *W, h))) return st;
+    const double beta = h.norm.x;
+    if (!(beta >= 0)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: NaN in the residual");
+    if (cyc == 0) {
+      bnorm = beta;
+      if (bnorm == 0.0) return CLG_SUCCESS;
+    }
+    ++*cycles_out;
     if (beta == 0.0) break;
-    if ((st = K.lincomb(W->V[0], zero, {&W->R}, {Z(1.0 / beta, 0.0)}))) return st;
-    Mat H(m + 1, m);
     int dim = m;
-    for (int j = 0; j < m; ++j) {
-      if ((st = K.apply(W->w, W->V[j]))) return st;
-      std::vector<const FieldRef*> vs;
-      for (int i = 0; i <= j; ++i) vs.push_back(&W->V[i]);
-      std::vector<Z> h;
-      if ((st = K.orthogonalise(W->w, vs, h))) return st;
-      for (int i = 0; i <= j; ++i) H(i, j) = h[i];
-      const double hn = K.norm(W->w);
-      if (hn < 0) return ctx->fail(CLG_ERR_CUDA, "multi-shift GMRES: reading |w|");
-      H(j + 1, j) = Z(hn, 0.0);
-      if (hn <= 1e-300 * bnorm) {
-        dim = j + 1;
-        break;
-      }
-      if (j + 1 < m && (st = K.lincomb(W->V[j + 1], zero, {&W->w}, {Z(1.0 / hn, 0.0)}))) return st;
-    }
+    for (int j = 0; j < m && dim == m; ++j)
+      if (hess(h, j + 1, j).real() <= 1e-300 * bnorm) dim = j + 1;
     *apps_out += dim + (cyc > 0 ? 1 : 0);
     // the seed system: y = argmin |beta e_1 - Hbar y|, z = beta e_1 - Hbar y
     Mat Hb(dim + 1, dim);
     for (int r = 0; r <= dim; ++r)
-      for (int c = 0; c < dim; ++c) Hb(r, c) = H(r, c);
+      for (int c = 0; c < dim; ++c) Hb(r, c) = hess(h, r, c);
     std::vector<Z> g(dim + 1, zero), y;
     g[0] = Z(beta, 0.0);
-    if (!dense::lstsq(Hb, g, y)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: seed least squares");
-    std::vector<const FieldRef*> vs;
-    for (int i = 0; i < dim; ++i) vs.push_back(&W->V[i]);
-    if ((st = K.lincomb(xs, one, vs, y))) return st;
+    if (!hess_solve(Hb, g, y)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: seed least squares");
     std::vector<Z> z(dim + 1);
     for (int r = 0; r <= dim; ++r) {
       Z hy = zero;
       for (int c = 0; c < dim; ++c) hy += Hb(r, c) * y[c];
       z[r] = g[r] - hy;
     }
+    if ((st = add_basis(K, *W, xs, 1, y, dim))) return st;
     double zn = 0.0;
     for (const Z& v : z) zn += std::norm(v);
     zn = std::sqrt(zn);
     double worst = 0.0;
+    std::vector<Z> Y((size_t)ns * dim);
     for (int n = 0; n < ns; ++n) {
       // [Hbar + c_n I~ | z] [y_n; beta_n'] = beta_n beta e_1
       Mat Hh(dim + 1, dim + 1);
@@ -308,14 +361,14 @@ clg_status gmres_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cac
       }
       std::vector<Z> gn(dim + 1, zero), w;
       gn[0] = beta0[n] * beta;
-      if (!dense::lstsq(Hh, gn, w)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: shifted system");
-      std::vector<Z> yn(w.begin(), w.begin() + dim);
-      if ((st = K.lincomb(xk(n), one, vs, yn))) return st;
+      if (!hess_solve(Hh, gn, w)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: shifted system");
+      std::copy(w.begin(), w.begin() + dim, Y.begin() + (size_t)n * dim);
       beta0[n] = w[dim];
       const double e = std::abs(beta0[n]) * zn;
       if (!(e == e)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: NaN in the recurrence");
       worst = std::max(worst, e);
     }
+    if ((st = add_basis(K, *W, W->X, ns, Y, dim))) return st;
     if (worst <= tol * bnorm) break;
   }
   return CLG_SUCCESS;

@@ -28,23 +28,34 @@
 
 namespace clg {
 
-__global__ void gm_solve_y(KState* st, int nrhs) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per right-hand side, lane l = unknown l: its row of the triangle is
+// loaded at once, then column by column (y_i by lane i, the rest updated).
+// One thread per right-hand side took a global round trip per element (17 us).
+__global__ void __launch_bounds__(32) gm_solve_y(KState* st, int nrhs) {
+  const int r = blockIdx.x, l = threadIdx.x;
   if (r >= nrhs) return;
   KState& k = st[r];
-  if (k.done || k.j == 0) return;
   const int m = k.j;
-  for (int i = m - 1; i >= 0; --i) {
-    double2 acc = k.g[i];
-    for (int l = i + 1; l < m; ++l) {
-      const double2 p = cmul(k.H[i * GM_MAXK + l], k.y[l]);
+  if (k.done || m == 0) return;  // uniform over the warp
+  const bool own = l < m;
+  double2 row[GM_MAXK];
+#pragma unroll
+  for (int i = 0; i < GM_MAXK; ++i) row[i] = own && i >= l && i < m ? k.H[l * GM_MAXK + i] : make_double2(0.0, 0.0);
+  double2 acc = own ? k.g[l] : make_double2(0.0, 0.0), y = make_double2(0.0, 0.0);
+  const double s = own ? k.s[l] : 0.0;
+#pragma unroll
+  for (int i = GM_MAXK - 1; i >= 0; --i) {
+    if (i >= m) continue;
+    if (l == i) y = cdiv(acc, row[i]);
+    const double2 yi = make_double2(__shfl_sync(0xffffffffu, y.x, i), __shfl_sync(0xffffffffu, y.y, i));
+    if (l < i) {
+      const double2 p = cmul(row[i], yi);
       acc.x -= p.x;
       acc.y -= p.y;
     }
-    k.y[i] = cdiv(acc, k.H[i * GM_MAXK + i]);
   }
-  for (int i = 0; i < m; ++i) k.y[i] = make_double2(k.y[i].x * k.s[i], k.y[i].y * k.s[i]);
-  if (k.resid_est * k.resid_est <= k.tol2 * k.rr0) k.status = ST_CONVERGED;
+  if (own) k.y[l] = make_double2(y.x * s, y.y * s);
+  if (l == 0 && k.resid_est * k.resid_est <= k.tol2 * k.rr0) k.status = ST_CONVERGED;
 }
 
 namespace {
@@ -540,18 +551,6 @@ clg_status iterate(Work& w, int graph_slot, int chunk, int max_chunks, Body&& bo
   return CLG_SUCCESS;
 }
 
-// GMRES multi-dot of column j with a reduction exactly 2(j+1) wide
-template <int PV, int NV, int J>
-clg_status launch_gm_dots(clg_context_s* ctx, const VList& vl, const FieldRef& wv, KState* st, int j, int fp, int np,
-                          int64_t Vh, int nrhs) {
-  if constexpr (J < GM_MAXK) {
-    if (j == J) return launch_sites<2 * (J + 1)>(ctx, GmDotsJ<PV, NV, J>{vl, dfield(wv), st}, fp, np, Vh, nrhs);
-    return launch_gm_dots<PV, NV, J + 1>(ctx, vl, wv, st, j, fp, np, Vh, nrhs);
-  } else {
-    return ctx->fail(CLG_ERR_BAD_ARG, "GMRES column index out of range");
-  }
-}
-
 // ------------------------------------------------------------------ Krylov methods
 // Solve K x = b (precision P, the subset of b) for every rhs not marked in outer_done.
 // ------------------------------------------------------------------ fused CG on the Wilson normal equations
@@ -1001,13 +1000,16 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       if ((s = vec(V[i]))) return s;
     if ((s = vec(wv))) return s;
     if ((s = blas_zero(ctx, x))) return s;
-    return with_pn(w.P, w.nc, [&](auto PP, auto NN) -> clg_status {
+    return with_pieces(w.P, w.nc, [&](auto PP, auto NN) -> clg_status {
       constexpr int PV = PP.value, NV = NN.value;
+      // the vector kernels see a site as `pieces` threads' work (with_pieces)
+      const int pieces = w.nc / NV, fq = fp * pieces, nq = np * pieces;
+      auto dv = [&](const FieldRef& f) { return dfield(pieces_view(f, pieces)); };
       VList vl;
-      for (int i = 0; i <= GM_MAXK; ++i) vl.v[i] = dfield(V[std::min(i, k)].ref);
+      for (int i = 0; i <= GM_MAXK; ++i) vl.v[i] = dv(V[std::min(i, k)].ref);
       // first cycle start (x = 0)
-      GmStart<PV, NV> st0{dfield(b), dfield(wv.ref), dfield(V[0].ref), w.st, 0, w.tol_d, 1};
-      clg_status e = launch_sites<1>(ctx, st0, fp, np, Vh, nrhs);
+      GmStart<PV, NV> st0{dv(b), dv(wv.ref), dv(V[0].ref), w.st, 0, w.tol_d, 1};
+      clg_status e = launch_sites<1>(ctx, st0, fq, nq, Vh, nrhs);
       if (e) return e;
       bool first_cycle = true;
       auto cycle = [&]() -> clg_status {
@@ -1015,18 +1017,21 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
         if (!first_cycle) {
           // restart: V'_0 = b - K x
           if ((e2 = kapply(w, op, wv.ref, x, nullptr, 0, &w.st[0].done, ks))) return e2;
-          GmStart<PV, NV> sr{dfield(b), dfield(wv.ref), dfield(V[0].ref), w.st, 1, w.tol_d, 0};
-          if ((e2 = launch_sites<1>(ctx, sr, fp, np, Vh, nrhs))) return e2;
+          GmStart<PV, NV> sr{dv(b), dv(wv.ref), dv(V[0].ref), w.st, 1, w.tol_d, 0};
+          if ((e2 = launch_sites<1>(ctx, sr, fq, nq, Vh, nrhs))) return e2;
         }
         for (int j = 0; j < k; ++j) {
           if ((e2 = kapply(w, op, wv.ref, V[j].ref, &w.st[0].s[j], (int)(sizeof(KState) / sizeof(double)), skip, ks)))
             return e2;
-          if ((e2 = launch_gm_dots<PV, NV, 0>(ctx, vl, wv.ref, w.st, j, fp, np, Vh, nrhs))) return e2;
-          if ((e2 = launch_sites<1>(ctx, GmOrtho<PV, NV>{vl, dfield(wv.ref), w.st, j}, fp, np, Vh, nrhs))) return e2;
+          const int groups = j / GM_DG + 1;
+          if ((e2 = launch_sites<2 * GM_DG>(ctx, GmDots<PV, NV>{vl, dv(wv.ref), w.st, j, groups}, fq, nq, Vh,
+                                            nrhs * groups)))
+            return e2;
+          if ((e2 = launch_sites<1>(ctx, GmOrtho<PV, NV>{vl, dv(wv.ref), w.st, j}, fq, nq, Vh, nrhs))) return e2;
         }
-        gm_solve_y<<<(nrhs + 63) / 64, 64, 0, ctx->stream>>>(w.st, nrhs);
+        gm_solve_y<<<nrhs, 32, 0, ctx->stream>>>(w.st, nrhs);
         ctx->kernels++;
-        if ((e2 = launch_sites<0>(ctx, GmUpdate<PV, NV>{vl, dfield(x), w.st, k}, fp, np, Vh, nrhs))) return e2;
+        if ((e2 = launch_sites<0>(ctx, GmUpdate<PV, NV>{vl, dv(x), w.st, k}, fq, nq, Vh, nrhs))) return e2;
         gm_finish<<<(nrhs + 63) / 64, 64, 0, ctx->stream>>>(w.st, nrhs);
         ctx->kernels++;
         return CLG_SUCCESS;

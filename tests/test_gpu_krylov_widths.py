@@ -1,0 +1,50 @@
+"""GMRES and multi-shift FOM / GMRES at Krylov dimensions around the group size
+of the multi-dot launches (4 inner products per block) and at the limits, on a
+lattice whose checkerboard is no multiple of a block: solutions to the oracle's
+true residual 1e-10."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+KAPPA, DIMS, TOL = 0.1355, (4, 6, 4, 10), 1e-10
+
+
+def _setup(clg, ctx, nrhs=1):
+    lat = clg.Lattice(ctx, DIMS)
+    U = clg.CFieldGaugeSU3(lat)
+    U.InitialField(clg.GAUGE_HAAR, 0xC1A60001, 1)
+    b = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=nrhs)
+    for r in range(nrhs):
+        b.InitialField(clg.SOURCE_GAUSS, 50 + r, 2, rhs=r)
+    return lat, U, b
+
+
+@pytest.mark.parametrize("max_dim", [1, 3, 4, 5, 8, 16])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_gmres_widths(ctx, clg, oracle, max_dim, prec):
+    lat, U, b = _setup(clg, ctx, 3)
+    x = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=3)
+    infos = clg.CSLASolverGMRES(ctx, inner_precision=prec, MaxDim=max_dim).Solve(x, b, U, clg.EFO_F_D)
+    op = oracle.Operator("WILSON_D", DIMS, U.CopyDataOut(), KAPPA)
+    for r in range(3):
+        assert infos[r]["status"] == 0
+        assert op.true_residual(b.to_numpy(r), x.to_numpy(r)) <= TOL
+
+
+@pytest.mark.parametrize("solver,max_dim", [("FOM", 2), ("FOM", 4), ("FOM", 5), ("FOM", 32), ("GMRES", 3),
+                                            ("GMRES", 5), ("GMRES", 32)])
+def test_multishift_widths(ctx, clg, oracle, solver, max_dim):
+    lat, U, b = _setup(clg, ctx)
+    shifts = [2.0, 0.5, 1j, 0.5 + 0.5j, 1 - 1j]
+    xs = [clg.CFieldFermionWilsonSquareSU3(lat, KAPPA) for _ in shifts]
+    S = getattr(clg, "CMultiShift" + solver)(ctx, MaxDim=max_dim)
+    op = oracle.Operator("WILSON_D", DIMS, U.CopyDataOut(), KAPPA)
+    for _ in range(2):  # the second call reuses the basis and its device state
+        infos = S.Solve(xs, shifts, b, U, clg.EFO_F_D)
+        for k, s in enumerate(shifts):
+            assert infos[k]["status"] == 0
+            assert op.true_residual(b.to_numpy(), xs[k].to_numpy(), complex(s)) <= TOL
+    # a zero right-hand side has the zero solution
+    b.Zero()
+    S.Solve(xs, shifts, b, U, clg.EFO_F_D)
+    assert max(np.abs(x.to_numpy()).max() for x in xs) == 0.0
