@@ -30,10 +30,29 @@ clg_status cuda_status(cudaError_t e) {
 
 int64_t site_bytes_of(int prec, int nc) { return (int64_t)nc * (prec == 0 ? 16 : (prec == 1 ? 8 : 4)); }
 
+static std::mutex g_contexts_m;
+static std::vector<clg_context_s*> g_contexts;
+void scratch_register(clg_context_s* ctx, bool add) {
+  std::lock_guard<std::mutex> lk(g_contexts_m);
+  if (add)
+    g_contexts.push_back(ctx);
+  else
+    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+}
+
 clg_status dalloc(clg_context_s* ctx, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return CLG_SUCCESS;
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !stream_capturing(ctx->stream)) {
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> lk(g_contexts_m);
+      for (clg_context_s* c : g_contexts)
+        if (c->device == ctx->device) scratch_trim(c);
+    }
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -43,6 +62,62 @@ clg_status dalloc(clg_context_s* ctx, void** p, size_t bytes) {
 }
 void dfree(void* p) {
   if (p) cudaFree(p);
+}
+
+clg_status Scratch::get(clg_context_s* ctx, size_t bytes) {
+  ctx_ = ctx;
+  bytes = std::max<size_t>((bytes + 511) & ~(size_t)511, 512);
+  // a captured call must not leave a pool block in the graph; its cudaMalloc is
+  // refused, as it always was
+  const bool pool = bytes <= ScratchPool::most / 2 && !stream_capturing(ctx->stream);
+  ScratchPool& s = ctx->pool;
+  if (pool) {
+    std::lock_guard<std::mutex> lk(s.m);
+    ScratchPool::Block* best = nullptr;
+    for (auto& b : s.blocks)
+      if (!b.used && b.bytes >= bytes && b.bytes <= 2 * bytes && (!best || b.bytes < best->bytes)) best = &b;
+    if (best) {
+      best->used = true;
+      p_ = best->p;
+      pooled_ = true;
+      return CLG_SUCCESS;
+    }
+  }
+  if (clg_status st = dalloc(ctx, &p_, bytes)) return st;
+  if (!pool) return CLG_SUCCESS;
+  std::lock_guard<std::mutex> lk(s.m);
+  if (s.total + bytes > ScratchPool::most) return CLG_SUCCESS;
+  s.blocks.push_back({p_, bytes, true});
+  s.total += bytes;
+  pooled_ = true;
+  return CLG_SUCCESS;
+}
+
+Scratch::~Scratch() {
+  if (!p_) return;
+  if (!pooled_) {
+    if (!stream_capturing(ctx_->stream)) cudaStreamSynchronize(ctx_->stream);
+    dfree(p_);
+    return;
+  }
+  std::lock_guard<std::mutex> lk(ctx_->pool.m);
+  for (auto& b : ctx_->pool.blocks)
+    if (b.p == p_) b.used = false;
+}
+
+void scratch_trim(clg_context_s* ctx) {
+  ScratchPool& s = ctx->pool;
+  std::lock_guard<std::mutex> lk(s.m);
+  std::vector<ScratchPool::Block> keep;
+  for (auto& b : s.blocks) {
+    if (b.used) {
+      keep.push_back(b);
+      continue;
+    }
+    s.total -= b.bytes;
+    dfree(b.p);  // waits for the kernels that used it
+  }
+  s.blocks.swap(keep);
 }
 
 // bytes of one right-hand side of a host (FP64 lexicographic) field array
@@ -260,30 +335,23 @@ namespace {
 
 bool valid_prec(int p) { return p >= 0 && p <= 2; }
 
-// scratch field with the shape of f (cached per context by shape key)
-struct Scratch {
-  void* data = nullptr;
-  float* norm = nullptr;
+// scratch field with the shape of f, from the context's pool
+struct ScratchField {
+  Scratch data, norm;
   FieldRef ref;
 };
 
-clg_status make_like(clg_context_s* ctx, const clg_field_s* f, int nparity, int first_parity, Scratch& s) {
+clg_status make_like(clg_context_s* ctx, const clg_field_s* f, int nparity, int first_parity, ScratchField& s) {
   const int64_t Vh = f->lat->g.Vh;
   const int64_t blk = Vh * site_bytes_of(f->prec, f->nc());
-  clg_status st = dalloc(ctx, &s.data, (size_t)blk * nparity * f->nrhs);
+  clg_status st = s.data.get(ctx, (size_t)blk * nparity * f->nrhs);
+  if (!st && f->prec == CLG_PREC_HALF) st = s.norm.get(ctx, (size_t)Vh * nparity * f->nrhs * sizeof(float));
   if (st) return st;
-  if (f->prec == CLG_PREC_HALF) {
-    st = dalloc(ctx, (void**)&s.norm, (size_t)Vh * nparity * f->nrhs * sizeof(float));
-    if (st) {
-      dfree(s.data);
-      return st;
-    }
-  }
-  s.ref.data = (char*)s.data;
-  s.ref.norm = s.norm;
+  s.ref.data = s.data.as<char>();
+  s.ref.norm = s.norm.as<float>();
   s.ref.blk = blk;
   s.ref.rstride = blk * nparity;
-  s.ref.nrstride = s.norm ? Vh * nparity : 0;
+  s.ref.nrstride = s.ref.norm ? Vh * nparity : 0;
   s.ref.nparity = nparity;
   s.ref.first_parity = first_parity;
   s.ref.prec = f->prec;
@@ -291,12 +359,6 @@ clg_status make_like(clg_context_s* ctx, const clg_field_s* f, int nparity, int 
   s.ref.nrhs = f->nrhs;
   s.ref.Vh = Vh;
   return CLG_SUCCESS;
-}
-void free_scratch(Scratch& s) {
-  dfree(s.data);
-  dfree(s.norm);
-  s.data = nullptr;
-  s.norm = nullptr;
 }
 
 clg_status sync_status(clg_context_s* ctx) {
@@ -433,12 +495,14 @@ clg_status clg_context_create(int device, void* stream, clg_context* out) {
     delete ctx;
     return st;
   }
+  scratch_register(ctx, true);
   *out = ctx;
   return CLG_SUCCESS;
 }
 
 clg_status clg_context_destroy(clg_context ctx) {
   if (!ctx) return CLG_ERR_BAD_ARG;
+  scratch_register(ctx, false);
   cudaStreamSynchronize(ctx->stream);
   if (!ctx->tune_file.empty()) {
     if (FILE* f = std::fopen(ctx->tune_file.c_str(), "w")) {
@@ -455,6 +519,7 @@ clg_status clg_context_destroy(clg_context ctx) {
     cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, 0);
     cudaGetLastError();
   }
+  scratch_trim(ctx);
   dfree(ctx->red_partials);
   dfree(ctx->red_counter);
   dfree(ctx->staging);
@@ -601,14 +666,12 @@ clg_status clg_gauge_import(clg_gauge g, const double* data, int layout, int on_
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
   const bool direct = on_device && direct_doubles(ctx, data);
   // the links' deviation from SU(3), then (staged) the links
-  unsigned long long* worst = nullptr;
-  double* buf = nullptr;
-  clg_status st = dalloc(ctx, (void**)&worst, sizeof(*worst));
+  Scratch sw, sb;
+  clg_status st = sw.get(ctx, sizeof(unsigned long long));
+  if (!st && !direct) st = sb.get(ctx, bytes);
   if (st) return st;
-  if (!direct && (st = dalloc(ctx, (void**)&buf, bytes))) {
-    dfree(worst);
-    return st;
-  }
+  unsigned long long* worst = sw.as<unsigned long long>();
+  double* buf = sb.as<double>();
   cudaError_t e = cudaMemsetAsync(worst, 0, sizeof(*worst), ctx->stream);
   if (e == cudaSuccess && !direct)
     e = cudaMemcpyAsync(buf, data, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream);
@@ -621,8 +684,6 @@ clg_status clg_gauge_import(clg_gauge g, const double* data, int layout, int on_
   }
   // the caller may reuse or free its array once this returns
   if (!st) st = sync_status(ctx);
-  dfree(buf);
-  dfree(worst);
   if (!st) set_unitarity(g, u);
   return st;
 }
@@ -632,18 +693,17 @@ clg_status clg_gauge_export(clg_gauge g, double* data, int on_device) {
   clg_context_s* ctx = g->lat->ctx;
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
   const bool direct = on_device && direct_doubles(ctx, data);
-  double* buf = nullptr;
+  Scratch sb;
   clg_status st = CLG_SUCCESS;
-  if (!direct && (st = dalloc(ctx, (void**)&buf, bytes))) return st;
+  if (!direct && (st = sb.get(ctx, bytes))) return st;
+  double* buf = sb.as<double>();
   st = gauge_reorder(g, direct ? data : buf, CLG_LAYOUT_CLGBIN, 0, nullptr);
   if (!st && !direct) {
     cudaError_t e = cudaMemcpyAsync(data, buf, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                     ctx->stream);
     if (e != cudaSuccess) st = ctx->fail(cuda_status(e), cudaGetErrorString(e));
   }
-  if (!st) st = sync_status(ctx);
-  dfree(buf);
-  return st;
+  return st ? st : sync_status(ctx);
 }
 
 clg_status clg_gauge_random(clg_gauge g, int init, uint64_t seed, uint32_t field_id, double eps) {
@@ -892,47 +952,33 @@ clg_status clg_apply_to(int op, clg_field out, clg_field in, clg_gauge g, int co
   st = gauge_prepare(g, in->prec);
   if (st) return st;
   const double2 coeff = coeff_of(coeff_type, cre, cim);
-  Scratch t1, t2;
+  ScratchField t1, t2, t3;
   FieldRef o = out->ref(), i = in->ref();
-  const bool alias = out->data == in->data;
-  if (alias) {
-    st = make_like(ctx, in, in->nparity(), 0, t2);
-    if (st) return st;
-    st = blas_copy(ctx, t2.ref, i);
+  // in place: the products go through their temporary anyway (in is read by the
+  // first factor only); the other operators work from a copy
+  const bool product = op == CLG_OP_DDDAG || op == CLG_OP_DD;
+  if (out->data == in->data && !product) {
+    if ((st = make_like(ctx, in, in->nparity(), 0, t2)) || (st = blas_copy(ctx, t2.ref, i))) return st;
     i = t2.ref;
   }
-  if (!st) {
-    if (op == CLG_OP_DDDAG || op == CLG_OP_DD) {
-      st = make_like(ctx, in, 2, 0, t1);
-      if (!st) st = apply_op(ctx, op, g, in->kind, in->param, o, i, &t1.ref, coeff, in->nrhs);
-    } else if (op_on_even(op)) {
-      st = make_like(ctx, in, 1, 1, t1);
-      if (!st) {
-        if (op == CLG_OP_MEE_MEEDAG) {
-          Scratch t3;
-          st = make_like(ctx, in, 1, 0, t3);
-          if (!st) st = apply_op(ctx, CLG_OP_MEE_DAG, g, in->kind, in->param, t3.ref, i, &t1.ref, make_double2(1, 0), in->nrhs);
-          if (!st) st = apply_op(ctx, CLG_OP_MEE, g, in->kind, in->param, o, t3.ref, &t1.ref, coeff, in->nrhs);
-          if (!st) st = sync_status(ctx);
-          free_scratch(t3);
-        } else {
-          st = apply_op(ctx, op, g, in->kind, in->param, o, i, &t1.ref, coeff, in->nrhs);
-        }
-      }
-    } else if (op == CLG_OP_DEO || op == CLG_OP_DOE) {
-      // the other checkerboard of out is left unchanged
-      st = apply_op(ctx, op, g, in->kind, in->param, o, i, nullptr, coeff, in->nrhs);
-    } else {
-      st = apply_op(ctx, op, g, in->kind, in->param, o, i, nullptr, coeff, in->nrhs);
+  if (product) {
+    st = make_like(ctx, in, 2, 0, t1);
+    if (!st) st = apply_op(ctx, op, g, in->kind, in->param, o, i, &t1.ref, coeff, in->nrhs);
+  } else if (op_on_even(op)) {
+    st = make_like(ctx, in, 1, 1, t1);
+    if (!st && op == CLG_OP_MEE_MEEDAG) {
+      st = make_like(ctx, in, 1, 0, t3);
+      if (!st) st = apply_op(ctx, CLG_OP_MEE_DAG, g, in->kind, in->param, t3.ref, i, &t1.ref, make_double2(1, 0), in->nrhs);
+      if (!st) st = apply_op(ctx, CLG_OP_MEE, g, in->kind, in->param, o, t3.ref, &t1.ref, coeff, in->nrhs);
+    } else if (!st) {
+      st = apply_op(ctx, op, g, in->kind, in->param, o, i, &t1.ref, coeff, in->nrhs);
     }
+  } else {
+    // DEO / DOE: the other checkerboard of out is left unchanged
+    st = apply_op(ctx, op, g, in->kind, in->param, o, i, nullptr, coeff, in->nrhs);
   }
-  // Operators that needed scratch fields wait for their kernels before the
-  // scratch is released; the others return once launched, like any stream
-  // operation, and can be captured into a CUDA graph.
-  if (!st) st = (t1.data || t2.data) ? sync_status(ctx) : launch_status(ctx);
-  free_scratch(t1);
-  free_scratch(t2);
-  return st;
+  // returns once launched, like any stream operation
+  return st ? st : launch_status(ctx);
 }
 
 clg_status clg_apply(int op, clg_field inout, clg_gauge g, int coeff_type, double cre, double cim) {
@@ -954,22 +1000,20 @@ clg_status clg_dot(clg_field a, clg_field b, double* re_im) {
   if (clg_status st = settle(a)) return st;
   if (clg_status st = settle(b)) return st;
   clg_context_s* ctx = a->lat->ctx;
-  double* d = nullptr;
-  clg_status st = dalloc(ctx, (void**)&d, sizeof(double) * 2 * a->nrhs);
-  if (!st) st = blas_dot(ctx, a->ref(), b->ref(), d);
-  if (!st) st = read_dev(ctx, re_im, d, 2 * a->nrhs);
-  dfree(d);
+  Scratch d;
+  clg_status st = d.get(ctx, sizeof(double) * 2 * a->nrhs);
+  if (!st) st = blas_dot(ctx, a->ref(), b->ref(), d.as<double>());
+  if (!st) st = read_dev(ctx, re_im, d.as<double>(), 2 * a->nrhs);
   return st;
 }
 
 clg_status clg_norm2(clg_field a, double* out) {
   if (!a || !out) return CLG_ERR_BAD_ARG;
   clg_context_s* ctx = a->lat->ctx;
-  double* d = nullptr;
-  clg_status st = dalloc(ctx, (void**)&d, sizeof(double) * a->nrhs);
-  if (!st) st = blas_norm2(ctx, a->ref(), d);
-  if (!st) st = read_dev(ctx, out, d, a->nrhs);
-  dfree(d);
+  Scratch d;
+  clg_status st = d.get(ctx, sizeof(double) * a->nrhs);
+  if (!st) st = blas_norm2(ctx, a->ref(), d.as<double>());
+  if (!st) st = read_dev(ctx, out, d.as<double>(), a->nrhs);
   return st;
 }
 

@@ -646,9 +646,10 @@ clg_status field_source(clg_field_s* f, int rhs, int kind, uint64_t seed, uint32
 clg_status gauge_plaquette(clg_gauge_s* U, double* host_out) {
   clg_context_s* ctx = U->lat->ctx;
   const Geom& g = U->lat->g;
-  double* d = nullptr;
-  clg_status st = dalloc(ctx, (void**)&d, sizeof(double));
+  Scratch sd;
+  clg_status st = sd.get(ctx, sizeof(double));
   if (st) return st;
+  double* d = sd.as<double>();
   PlaqOut fn{PlaqF{g, LinkPtrs{{(double2*)U->u64[0], (double2*)U->u64[1]}}}, d};
   st = launch_sites<1>(ctx, fn, 0, 2, g.Vh, 1);
   if (!st) {
@@ -657,16 +658,16 @@ clg_status gauge_plaquette(clg_gauge_s* U, double* host_out) {
     if (e != cudaSuccess) st = ctx->fail(cuda_status(e), cudaGetErrorString(e));
     *host_out /= (6.0 * (double)g.V);
   }
-  dfree(d);
   return st;
 }
 
 clg_status gauge_unitarity(clg_gauge_s* U, double* host_out) {
   clg_context_s* ctx = U->lat->ctx;
   const Geom& g = U->lat->g;
-  unsigned long long* d = nullptr;
-  clg_status st = dalloc(ctx, (void**)&d, sizeof(unsigned long long));
+  Scratch sd;
+  clg_status st = sd.get(ctx, sizeof(unsigned long long));
   if (st) return st;
+  unsigned long long* d = sd.as<unsigned long long>();
   cudaError_t e = cudaMemsetAsync(d, 0, sizeof(unsigned long long), ctx->stream);
   if (e == cudaSuccess) {
     unitarity_kernel<<<dim3((unsigned)((g.Vh + 255) / 256), 8), 256, 0, ctx->stream>>>(
@@ -677,7 +678,6 @@ clg_status gauge_unitarity(clg_gauge_s* U, double* host_out) {
   double w = 0.0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&w, d, sizeof(w), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  dfree(d);
   if (e != cudaSuccess) return ctx->fail(cuda_status(e), cudaGetErrorString(e));
   *host_out = w;
   return CLG_SUCCESS;

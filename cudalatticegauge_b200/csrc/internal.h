@@ -58,6 +58,27 @@ int64_t site_bytes_of(int prec, int nc);
 
 }  // namespace clg
 
+namespace clg {
+// Device memory that operators and reductions need for the length of a call,
+// kept between calls: cudaMalloc and cudaFree of a temporary field cost 0.3 to
+// 1 ms and a device-wide wait, more than the operator itself on every lattice
+// up to 32^3x16.  A block belongs to one call from get to put; its next user
+// comes later on the same stream, so nothing waits.  At most `most` bytes are
+// kept, and an allocation of any context of the device that fails gives the
+// idle ones back and is tried once more (dalloc).  Locked: several threads may use one context.
+struct ScratchPool {
+  struct Block {
+    void* p;
+    size_t bytes;
+    bool used;
+  };
+  static constexpr size_t most = (size_t)1 << 30;
+  std::mutex m;
+  std::vector<Block> blocks;
+  size_t total = 0;
+};
+}  // namespace clg
+
 struct clg_context_s {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -77,6 +98,7 @@ struct clg_context_s {
   // two copies and a reorder, not a cudaMalloc/cudaFree pair.
   void* staging = nullptr;
   size_t staging_bytes = 0;
+  clg::ScratchPool pool;  // see Scratch below
   // stream of the asynchronous host transfers (created on first use)
   cudaStream_t copy_stream = nullptr;
   // CLG_ZERO_COPY=1: asynchronous transfers of FP64 fields from/to pinned
@@ -232,6 +254,28 @@ clg_status noalloc_prepare(clg_context_s* ctx);
 clg_status dalloc(clg_context_s* ctx, void** p, size_t bytes);
 void dfree(void* p);
 clg_status ensure_reduction(clg_context_s* ctx, int64_t doubles);
+// A block of the context's pool, or (stream capture, or a block the pool would
+// not keep) memory of its own that is freed, after a wait, when this ends
+class Scratch {
+ public:
+  Scratch() = default;
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch();
+  clg_status get(clg_context_s* ctx, size_t bytes);
+  template <class T>
+  T* as() const {
+    return static_cast<T*>(p_);
+  }
+
+ private:
+  clg_context_s* ctx_ = nullptr;
+  void* p_ = nullptr;
+  bool pooled_ = false;
+};
+void scratch_trim(clg_context_s* ctx);  // frees the idle blocks
+// the contexts whose pools dalloc may trim
+void scratch_register(clg_context_s* ctx, bool add);
 // Group tickets of the two-level reductions, and the group size for nunits x
 // nslots blocks (at least 64 slots, doubled until the tickets fit)
 constexpr int64_t kRedGroups = 65536;

@@ -1,0 +1,78 @@
+"""The context's scratch pool: operators in place and products reuse its blocks,
+results do not depend on what a block held before, the pool stays bounded and
+gives its memory back when an allocation needs it and when the context ends."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+KAPPA = 0.1355
+
+
+def test_products_reuse_scratch(clg, oracle):
+    import torch
+
+    c = clg.Context(0)
+    lat = clg.Lattice(c, (6, 8, 4, 10), (1, 1, 1, -1))
+    U = clg.CFieldGaugeSU3(lat)
+    U.InitialField(clg.GAUGE_HAAR, 5, 1)
+    Uh = U.CopyDataOut()
+    for prec, tol in ((clg.DOUBLE, 1e-13), (clg.SINGLE, 2e-6), (clg.HALF, 5e-3)):
+        for nrhs in (1, 2):
+            a = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, precision=prec, nrhs=nrhs)
+            b = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, precision=prec, nrhs=nrhs)
+            for r in range(nrhs):
+                a.InitialField(clg.SOURCE_GAUSS, 9 + r, 2, rhs=r)
+            src = [a.to_numpy(r) for r in range(nrhs)]
+            a.apply_to(clg.EFO_F_DDdagger, b, U)
+            out = [b.to_numpy(r) for r in range(nrhs)]
+            a.DDdagger(U)  # in place
+            for r in range(nrhs):
+                np.testing.assert_array_equal(a.to_numpy(r), out[r])
+                want = oracle.wilson_D(lat.dims, Uh, oracle.wilson_D(lat.dims, Uh, src[r], KAPPA, dagger=True), KAPPA)
+                assert np.linalg.norm(out[r] - want) <= tol * np.linalg.norm(want)
+            a.close()
+            b.close()
+    # the same calls again allocate nothing
+    f = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA)
+    f.InitialField(clg.SOURCE_GAUSS, 3, 2)
+    f.DDdagger(U)
+    f.Dot(f)
+    U.plaquette()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(0)[0]
+    for _ in range(3):
+        f.DDdagger(U)
+        f.D(U)
+        f.Dot(f)
+        f.norm2()
+        U.plaquette()
+    assert torch.cuda.mem_get_info(0)[0] == free
+    for o in (f, U, lat):
+        o.close()
+    c.close()
+
+
+def test_pool_is_bounded_and_given_back(clg):
+    import torch
+
+    lib = clg.load_library()
+    base = clg.Context(0)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info(0)[0]
+    c = clg.Context(0)
+    lat = clg.Lattice(c, (32, 32, 32, 16))
+    U = clg.CFieldGaugeSU3(lat)
+    for nrhs in (1, 2, 4, 8, 14):  # temporaries of 0.1 to 1.4 GB
+        f = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=nrhs)
+        f.DDdagger(U)
+        f.close()
+    U.close()
+    lat.close()
+    c.synchronize()
+    held = free0 - torch.cuda.mem_get_info(0)[0]
+    assert held <= (1 << 30) + (256 << 20), held  # 1 GB and the context's own scratch
+    c.close()
+    torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info(0)[0] <= 64 << 20
+    assert lib.clg_context_synchronize(base.h) == clg.SUCCESS
+    base.close()
