@@ -67,9 +67,11 @@ void dfree(void* p) {
 clg_status Scratch::get(clg_context_s* ctx, size_t bytes) {
   ctx_ = ctx;
   bytes = std::max<size_t>((bytes + 511) & ~(size_t)511, 512);
-  // a captured call must not leave a pool block in the graph; its cudaMalloc is
-  // refused, as it always was
-  const bool pool = bytes <= ScratchPool::most / 2 && !stream_capturing(ctx->stream);
+  // a graph must not keep a temporary of one call: refused, as the cudaMalloc
+  // and the wait of such a call were
+  if (stream_capturing(ctx->stream))
+    return ctx->fail(CLG_ERR_CUDA, "scratch memory inside a stream capture");
+  const bool pool = bytes <= ScratchPool::most / 2;
   ScratchPool& s = ctx->pool;
   if (pool) {
     std::lock_guard<std::mutex> lk(s.m);
@@ -96,7 +98,7 @@ clg_status Scratch::get(clg_context_s* ctx, size_t bytes) {
 Scratch::~Scratch() {
   if (!p_) return;
   if (!pooled_) {
-    if (!stream_capturing(ctx_->stream)) cudaStreamSynchronize(ctx_->stream);
+    cudaStreamSynchronize(ctx_->stream);
     dfree(p_);
     return;
   }

@@ -26,15 +26,24 @@ __global__ void __launch_bounds__(256)
   double acc[NRED > 0 ? NRED : 1];
 #pragma unroll
   for (int k = 0; k < (NRED > 0 ? NRED : 1); ++k) acc[k] = 0.0;
-  if (f.active(rhs)) {
+  bool work;
+  if constexpr (has_prologue<F>::value)
+    work = f.prologue(rhs, blockIdx.x == 0);
+  else
+    work = f.active(rhs);
+  if (work) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nsites; i += (int64_t)gridDim.x * blockDim.x) {
       const int pi = (int)(i / Vh);
       const int64_t h = i - (int64_t)pi * Vh;
       f(rhs, first_parity + pi, h, acc);
     }
   }
-  if constexpr (NRED > 0)
-    grid_reduce_finalize<NRED>(acc, f, rhs, blockIdx.x, gridDim.x, (int)gridDim.y, partials, counter);
+  if constexpr (NRED > 0) {
+    if constexpr (partials_only<F>::value)
+      block_partials<NRED>(acc, partials, blockIdx.x + rhs * gridDim.x);
+    else
+      grid_reduce_finalize<NRED>(acc, f, rhs, blockIdx.x, gridDim.x, (int)gridDim.y, partials, counter);
+  }
 }
 
 // The same over a batch of lattices (clg_solve_lattices): right-hand side r
@@ -63,9 +72,9 @@ __global__ void __launch_bounds__(256)
     grid_reduce_finalize<NRED>(acc, f, rhs, blockIdx.x, gridDim.x, (int)gridDim.y, partials, counter);
 }
 
-// Launch F over the checkerboards [first_parity, first_parity + nparity) of all nrhs.
-template <int NRED, class F>
-clg_status launch_sites(clg_context_s* ctx, const F& f, int first_parity, int nparity, int64_t Vh, int nrhs) {
+// The blocks per right-hand side of launch_sites
+template <int NRED>
+int64_t site_blocks(const clg_context_s* ctx, int nparity, int64_t Vh, int nrhs) {
   const int bs = 256;
   const int64_t nsites = (int64_t)nparity * Vh;
   int64_t nb = (nsites + bs - 1) / bs;
@@ -75,18 +84,35 @@ clg_status launch_sites(clg_context_s* ctx, const F& f, int first_parity, int np
   const int64_t cap = (int64_t)ctx->num_sms * per_sm / (nrhs > 0 ? nrhs : 1) + 1;
   if (NRED > 0 && nb > cap) nb = cap;
   if (nb > 65535 * 64) nb = 65535 * 64;
+  return nb;
+}
+
+// Launch F over the checkerboards [first_parity, first_parity + nparity) of all nrhs.
+// (part: where a functor with PARTIALS leaves its block sums)
+template <int NRED, class F>
+clg_status launch_sites(clg_context_s* ctx, const F& f, int first_parity, int nparity, int64_t Vh, int nrhs,
+                        double* part = nullptr) {
+  const int bs = 256;
+  const int64_t nsites = (int64_t)nparity * Vh;
+  const int64_t nb = site_blocks<NRED>(ctx, nparity, Vh, nrhs);
   if (NRED > 0) {
     clg_status st = ensure_reduction(ctx, nb * nrhs * (NRED > 0 ? NRED : 1));
     if (st) return st;
   }
   dim3 grid((unsigned)nb, (unsigned)nrhs);
   cudaError_t e;
-  if (ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs % ctx->batch_nrhs == 0)
+  auto plain = [&]() {
+    return launch_pdl(ctx, site_reduce_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
+                      part ? part : ctx->red_partials, ctx->red_counter);
+  };
+  if constexpr (partials_only<F>::value || has_prologue<F>::value) {
+    e = plain();  // solvers of one lattice only
+  } else if (ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs % ctx->batch_nrhs == 0) {
     e = launch_pdl(ctx, site_reduce_batch_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
                    ctx->red_partials, ctx->red_counter, (const int64_t*)ctx->batch_vh, nrhs / ctx->batch_nrhs);
-  else
-    e = launch_pdl(ctx, site_reduce_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
-                   ctx->red_partials, ctx->red_counter);
+  } else {
+    e = plain();
+  }
   if (e != cudaSuccess) return ctx->fail(cuda_status(e), std::string("site kernel: ") + cudaGetErrorString(e));
   return CLG_SUCCESS;
 }

@@ -34,10 +34,18 @@ cudaError_t launch_wilson_tileN(clg_context_s* ctx, const HopArgs& a0, bool dagg
 std::vector<int> tile_warps(int nrhs);
 
 // Four threads per site are timed where one thread per site gives the chip
-// less than SPLIT_MAX threads (it wins up to about 2^14 sites; the autotuner
-// decides between)
+// less than SPLIT_MAX threads, and taken untimed where it gives each of the
+// 592 schedulers less than a warp: there a launch is a few dependent round
+// trips to memory, which a loop of independent launches (the autotuner's, bound
+// by the launches themselves) cannot see.  GMRES on 8^4: SPLIT_US
 constexpr int64_t SPLIT_MAX = (int64_t)1 << 18;
 bool split_worth(const Geom& g, int nrhs) { return g.Vh * nrhs <= SPLIT_MAX; }
+// the untimed choice, recorded like a timed one (the fused epilogues follow it)
+bool take_split(clg_context_s* ctx, const std::string& key, const Geom& g, int nrhs, int variant) {
+  if (g.Vh * nrhs > SPLIT_ALWAYS || !ctx->tuning_enabled || ctx->tuned.count(key)) return false;
+  ctx->tuned[key] = (4 * SPLIT_SITES) | (variant << 16);
+  return true;
+}
 
 template <int P, int RECON>
 cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int nrhs, const std::string& key) {
@@ -48,14 +56,15 @@ cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int
     const int bs = cfg & 0xffff;
     const int variant = cfg >> 16;
     if constexpr (P != P16) {
-      if (variant >= 16) return launch_wilson_tileN<P, RECON>(ctx, a, dagger, cfg);
+      if (variant >= 16)
+        return a.fin.n ? cudaErrorInvalidConfiguration : launch_wilson_tileN<P, RECON>(ctx, a, dagger, cfg);
     }
     if (variant == HOP_SPLIT) {
-      dim3 sg((unsigned)(((a.g.Vh + SPLIT_SITES - 1) / SPLIT_SITES) * nrhs));
+      dim3 sg((unsigned)(((a.g.Vh + SPLIT_SITES - 1) / SPLIT_SITES) * nrhs) + (a.fin.n ? 1u : 0u));
       return dagger ? launch_pdl(ctx, wilson_split_kernel<P, RECON, true, false>, sg, dim3(4 * SPLIT_SITES), 0, a)
                     : launch_pdl(ctx, wilson_split_kernel<P, RECON, false, false>, sg, dim3(4 * SPLIT_SITES), 0, a);
     }
-    dim3 grid((unsigned)(((a.g.Vh + bs - 1) / bs) * nrhs));
+    dim3 grid((unsigned)(((a.g.Vh + bs - 1) / bs) * nrhs) + (a.fin.n ? 1u : 0u));
     if constexpr (P == P64) {
       if (variant == 3)
         return dagger ? launch_pdl(ctx, wilson_hop_kernel<P, RECON, true, 256, 2>, grid, dim3(bs), 0, a)
@@ -76,6 +85,7 @@ cudaError_t launch_wilson(clg_context_s* ctx, const HopArgs& a, bool dagger, int
     ctx->tuned[key] = ctx->hop_config;  // the fused epilogue launches follow the pinned form
     return go(ctx->hop_config);
   }
+  if (nrhs == 1 || P != P16) take_split(ctx, key, a.g, nrhs, HOP_SPLIT);
   // __launch_bounds__(256, ...) caps the block at 256 threads
   std::vector<int> cand = {64, 128, 256};
   if (P != P64)
@@ -533,6 +543,7 @@ clg_status make_hop_args(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec
   a.btile = U->btile;
   a.nbtile = U->nbtile;
   a.btiles = U->btiles;
+  a.fin = s.fin ? *s.fin : AlphaFin{};
   a.in_blk = s.in.blk;
   a.out_blk = s.out.blk;
   a.x_blk = s.x ? s.x->blk : 0;
@@ -651,6 +662,7 @@ clg_status hop_full(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s) 
     return wilson ? launch_wilson_full<P32, 18>(ctx, a, s.dagger, rows, cfg)
                   : launch_staggered_full<P32, 18>(ctx, a, rows, cfg);
   };
+  if (wilson) take_split(ctx, hop_key(U, s) + "_full", a.g, 2 * s.nrhs, FULL_SPLIT);
   const cudaError_t e = go(tune_block(ctx, hop_key(U, s) + "_full", idempotent(a), go, full_candidates(a, rows, wilson),
                                       128 | ((FULL_ONE + 1) << 16)));
   if (hst) return hst;

@@ -29,6 +29,19 @@ struct HopSeg {
   const void* u[3][2];
 };
 
+// alpha = |r|^2 / (p, A p) of a CG iteration from n partials (n = 0: nothing to
+// do), idempotent; the pointers are fields of the solver's state
+struct AlphaFin {
+  const double* partials;
+  int n;
+  const double* rr;
+  double2* alpha;
+  int* status;
+  int* done;
+  int* skip;
+  int breakdown;  // the status value
+};
+
 struct HopArgs {
   Geom g;
   int out_parity;
@@ -71,6 +84,9 @@ struct HopArgs {
   // both checkerboards in one launch (the full-lattice forms; the fields above
   // are those of out_parity 0): bytes from a field's parity 0 to its parity 1
   int64_t in_blk, out_blk, x_blk;
+  // one right-hand side of a fused CG: block 0 of the plain hop, besides the
+  // blocks of the hop, adds up the preceding hop's partials of (p, A p)
+  AlphaFin fin;
 };
 struct BatchTile {
   int64_t tile0;
@@ -345,6 +361,20 @@ __device__ __forceinline__ void wilson_hop_dir16(Acc16& A, const Packed16& p, co
   wilson_hop_dir16_u<MU, SGN, UDAG>(A, p, u, s);
 }
 
+// By one block (AlphaFin)
+__device__ __forceinline__ void alpha_block(const AlphaFin& f) {
+  const int skip = *f.skip;
+  const double rr = *f.rr;
+  const double pAp = block_total(f.partials, f.n);
+  if (threadIdx.x != 0 || skip) return;
+  if (!(pAp > 0.0) || isinf(pAp)) {
+    *f.status = f.breakdown;
+    *f.done = *f.skip = 1;
+  } else {
+    *f.alpha = make_double2(rr / pAp, 0.0);
+  }
+}
+
 struct NbrInfo {
   int hf[4], hb[4];   // checkerboard index of x+mu, x-mu (V < 2^31)
   float sf[4], sb[4]; // boundary signs
@@ -532,10 +562,15 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_kernel(HopArgs a) {
   using AT = typename AccT<P>::T;
   // right-hand sides are interleaved in blockIdx.x so that the CTAs of all rhs
   // for the same sites run back to back and share the links through L2
-  const int rhs = (int)(blockIdx.x % (unsigned)a.nrhs);
-  const int64_t h = (int64_t)(blockIdx.x / (unsigned)a.nrhs) * blockDim.x + threadIdx.x;
+  const unsigned bx = blockIdx.x - (a.fin.n ? 1u : 0u);
+  const int rhs = (int)(bx % (unsigned)a.nrhs);
+  const int64_t h = (int64_t)(bx / (unsigned)a.nrhs) * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();
+  if (a.fin.n && blockIdx.x == 0) {
+    alpha_block(a.fin);
+    return;
+  }
   if (h >= a.g.Vh) return;
   if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;
   cpx<AT> acc[12];
@@ -616,6 +651,9 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_full_kernel(HopArgs a) {
 // 16^3x32 it loses (37.5 against 31.1 us, FP64).
 constexpr int SPLIT_SITES = 32;
 constexpr int HOP_SPLIT = 4;  // this form's launch variant (dslash.cu)
+// up to this many sites a launch gives each of the 592 schedulers less than a
+// warp: the form is taken untimed
+constexpr int64_t SPLIT_ALWAYS = 592 * 32;
 template <int P>
 struct SplitSmem {
   cpx<typename AccT<P>::T> g[8][6][SPLIT_SITES];  // s (g0, g1) of direction 2 mu + (0 forward, 1 backward)
@@ -757,14 +795,19 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_kernel(HopArgs a
   if constexpr (FULL) {
     full_block(a, rhs, p, slot);
   } else {
-    slot = blockIdx.x / (unsigned)a.nrhs;
-    rhs = (int)(blockIdx.x - slot * (unsigned)a.nrhs);
+    const unsigned bx = blockIdx.x - (a.fin.n ? 1u : 0u);
+    slot = bx / (unsigned)a.nrhs;
+    rhs = (int)(bx - slot * (unsigned)a.nrhs);
   }
   const int i = threadIdx.x & 31;
   const int64_t h = (int64_t)slot * SPLIT_SITES + i;
   pdl_launch_dependents();
   if (FULL && p) flip_parity(a);
   pdl_wait();
+  if (!FULL && a.fin.n && blockIdx.x == 0) {
+    alpha_block(a.fin);
+    return;
+  }
   if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;  // uniform over the block
   if (h < a.g.Vh) wilson_split_stage<P, RECON, DAGGER>(a, rhs, h, i, t);
   __syncthreads();
@@ -815,6 +858,8 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
   double red[E::NRED];
 #pragma unroll
   for (int k = 0; k < E::NRED; ++k) red[k] = 0.0;
+  if constexpr (has_prefetch<E>::value)
+    if (!skipped && h < a.g.Vh) e.prefetch(rhs, h);
   if (!skipped && h < a.g.Vh) {
     cpx<AT> acc[12];
     bool valid = true;
@@ -827,11 +872,15 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
       e.site(rhs, h, acc, red);
     }
   }
-  const int rr[1] = {rhs};
-  const bool cc[1] = {!skipped}, hh[1] = {true};
-  grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
-                                    gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter,
-                                    BATCH ? a.seg_vh : nullptr);
+  if constexpr (partials_only<E>::value) {
+    block_partials<E::NRED>(red, partials, slot);  // one right-hand side
+  } else {
+    const int rr[1] = {rhs};
+    const bool cc[1] = {!skipped}, hh[1] = {true};
+    grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
+                                      gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter,
+                                      BATCH ? a.seg_vh : nullptr);
+  }
 }
 
 // The epilogue form of wilson_full_kernel, one right-hand side: E::par is set to
@@ -866,7 +915,9 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_full_epi_kernel(HopArgs a, 
 
 // The epilogue form with four threads per site (wilson_split_kernel): warp 0
 // holds the block's results and reduces them; one slot per 32 sites.
-template <int P, int RECON, bool DAGGER, class E>
+// FULL: both checkerboards of one right-hand side in one launch (E::par as in
+// wilson_full_epi_kernel), two slots per 32 checkerboard sites.
+template <int P, int RECON, bool DAGGER, class E, bool FULL = false>
 __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopArgs a, E e, double* partials,
                                                                           double* gpart, unsigned* counter,
                                                                           unsigned group) {
@@ -875,8 +926,12 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopAr
   const unsigned slot = blockIdx.x / (unsigned)a.nrhs;
   const int rhs = (int)(blockIdx.x - slot * (unsigned)a.nrhs);
   const int i = threadIdx.x & 31;
-  const int64_t h = (int64_t)slot * SPLIT_SITES + i;
+  const int64_t h = (int64_t)(FULL ? slot >> 1 : slot) * SPLIT_SITES + i;
   pdl_launch_dependents();
+  if constexpr (FULL) {
+    if (slot & 1) flip_parity(a);
+    e.par = (int)(slot & 1);
+  }
   pdl_wait();
   const bool skipped = a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride];
   double red[E::NRED];
@@ -890,10 +945,14 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopAr
     if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
     e.site(rhs, h, acc, red);
   }
-  const int rr[1] = {rhs};
-  const bool cc[1] = {!skipped}, hh[1] = {true};
-  grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
-                                    gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter);
+  if constexpr (partials_only<E>::value) {
+    block_partials<E::NRED>(red, partials, slot);  // one right-hand side
+  } else {
+    const int rr[1] = {rhs};
+    const bool cc[1] = {!skipped}, hh[1] = {true};
+    grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
+                                      gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter);
+  }
 }
 
 // ---------------------------------------------------------------- FP16, two right-hand sides per thread
@@ -2004,16 +2063,14 @@ __device__ __forceinline__ void staggered_hop_body(const HopArgs& a) {
 }
 
 // The staggered hop of one right-hand side with its xpay source x and a fused
-// reduction: out = a H in + xa x is stored, and the last block hands
-// Re sum_h <x(h), out(h)> (FP64 over the grid, out as stored: FP64 / FP32) to
-// E::finalize(0, tot) / E::finalize_warp on the device.  The second hop of the
+// reduction: out = a H in + xa x is stored, and every block leaves its part of
+// Re sum_h <x(h), out(h)> (FP64 over the block, out as stored: FP64 / FP32) in
+// partials, for the next kernel to add up (block_total).  The second hop of the
 // Schur operator (2am)^2 p - H_eo H_oe p then yields (p, A p) of a CG
-// iteration without a separate pass over p and A p.  Every thread reaches the
-// reduction; a skipped right-hand side (skip_dev) contributes zero, and E's
-// finalize still runs.
-template <int P, int RECON, int MINB, class E>
-__global__ void __launch_bounds__(256, MINB) staggered_hop_xdot_kernel(HopArgs a, E e, double* partials,
-                                                                      unsigned* counter) {
+// iteration without a separate pass over p and A p.  A skipped right-hand side
+// (skip_dev) contributes zero.
+template <int P, int RECON, int MINB>
+__global__ void __launch_bounds__(256, MINB) staggered_hop_xdot_kernel(HopArgs a, double* partials) {
   static_assert(P != P16, "the FP16 result is rounded when stored: reduce it from memory");
   using AT = typename AccT<P>::T;
   const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2034,7 +2091,7 @@ __global__ void __launch_bounds__(256, MINB) staggered_hop_xdot_kernel(HopArgs a
     store_site<P, 3, AT>(reinterpret_cast<char*>(a.out), nullptr, a.g.Vh, h, acc);
     red[0] = (double)re;
   }
-  grid_reduce_finalize<1>(red, e, 0, blockIdx.x, gridDim.x, 1, partials, counter);
+  block_partials<1>(red, partials, blockIdx.x);
 }
 
 // __launch_bounds__(256): the FP64 kernel takes 90 registers (22 warps per

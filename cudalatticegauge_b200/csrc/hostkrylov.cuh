@@ -118,7 +118,7 @@ struct LinCombF {
 #pragma unroll
       for (int k = 0; k < 3; ++k) o[k] = mk<double>(0, 0);
     }
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < n; ++i) {
       cpx<double> a[3];
       ld3(v.v[i], off, kstride, a);

@@ -254,8 +254,8 @@ clg_status noalloc_prepare(clg_context_s* ctx);
 clg_status dalloc(clg_context_s* ctx, void** p, size_t bytes);
 void dfree(void* p);
 clg_status ensure_reduction(clg_context_s* ctx, int64_t doubles);
-// A block of the context's pool, or (stream capture, or a block the pool would
-// not keep) memory of its own that is freed, after a wait, when this ends
+// A block of the context's pool, or (a block the pool would not keep) memory of
+// its own that is freed, after a wait, when this ends.  Refused in a capture.
 class Scratch {
  public:
   Scratch() = default;
@@ -367,6 +367,7 @@ int tune_block(clg_context_s* ctx, const std::string& key, bool can_repeat, Go&&
 
 // ------------------------------------------------------------ operators (dslash.cu)
 // A single checkerboard hop:  out_p = xa * x_p + a * H in_(1-p)  [ * scale_dev[rhs] ]
+struct AlphaFin;
 struct HopSpec {
   int kind;        // CLG_FERMION_WILSON / STAGGERED
   int prec;
@@ -381,6 +382,7 @@ struct HopSpec {
   const int* skip_dev;
   int skip_stride;
   int nrhs;
+  const AlphaFin* fin = nullptr;  // one right-hand side, plain Wilson hop (dslash.cuh)
 };
 clg_status hop(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s);
 // both checkerboards of full fields (s.out_parity is ignored; in and out must

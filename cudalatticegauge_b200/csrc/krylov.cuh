@@ -17,6 +17,7 @@ struct KState {
   // BiCGStab / CG scalars
   double2 rho, alpha, omega, beta;
   double rr, rr0, tol2;
+  double rr1;    // CG on one right-hand side: |r|^2 alternates between rr and rr1 (Cg1P)
   int done;      // this rhs needs no more work in the current inner solve
   int skip;      // kernels skip this rhs (done, or converged mid-iteration)
   int conv_s;    // BiCGStab: |s| small, finish with x += alpha p
@@ -389,6 +390,84 @@ struct CgHopUpdate {
   }
   __device__ void finalize(int w, const double* s) const { cg_update_finalize(st[w], s[0]); }
 };
+// CG on one right-hand side: the same iteration with the scalars made by the
+// kernels that need them (block_total) instead of at the end of the reducing
+// launch.  (p, A p) is left as partials by the alpha hop; the next hop, which
+// does not need alpha, adds them up in a block of its own (AlphaFin); |r|^2 is
+// left by the update hop and added up by every block of Cg1P, whose first block
+// writes the state.
+template <int P>
+struct Cg1HopAlpha : CgHopAlpha<P> {
+  static constexpr bool PARTIALS = true;
+};
+template <int P>
+struct Cg1HopUpdate : CgHopUpdate<P> {
+  static constexpr bool PARTIALS = true;
+  // x, r and p come from DRAM where the vectors and links exceed L2: requested
+  // before the stencil
+  __device__ void prefetch(int rhs, int64_t h) const {
+    constexpr int W = P == P64 ? 12 : (P == P32 ? 6 : 3);  // 16-byte words per site
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const int64_t off = (k * this->x.Vh + h) * 16;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->x.base(rhs, 0) + off));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->r.base(rhs, 0) + off));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->p.base(rhs, 0) + off));
+    }
+  }
+};
+// beta = |r_new|^2 / |r|^2; p = r + beta p.  `odd`: the iteration's parity, even
+// ones hold the old |r|^2 in rr and leave the new one in rr1, so that no block
+// reads what the first one writes (a finished solve leaves both in rr).
+template <int P, int NC>
+struct Cg1P {
+  DField p, r;
+  KState* st;
+  const double* rrp;  // nrr partials of |r_new|^2
+  int nrr, odd, weight;
+  __device__ static double* beta_of() {
+    __shared__ double b;
+    return &b;
+  }
+  __device__ bool active(int) const { return true; }
+  __device__ bool prologue(int, bool first) const {
+    KState& k = *st;
+    const int skip = k.skip;
+    const double old = odd ? k.rr1 : k.rr, lim = k.tol2 * k.rr0;
+    const double rr_new = block_total(rrp, nrr);
+    if (skip) return false;
+    const bool wrong = bad(rr_new), conv = !wrong && rr_new <= lim;
+    if (threadIdx.x == 0) *beta_of() = rr_new / old;
+    if (first && threadIdx.x == 0) {
+      k.iters += weight;
+      if (wrong) {
+        k.status = ST_BREAKDOWN;
+        k.done = k.skip = 1;
+      } else {
+        k.beta = make_double2(rr_new / old, 0.0);
+        if (odd || conv) k.rr = rr_new;
+        if (!odd || conv) k.rr1 = rr_new;
+        if (conv) {
+          k.status = ST_CONVERGED;
+          k.done = k.skip = 1;
+        }
+      }
+    }
+    __syncthreads();
+    return !wrong && !conv;
+  }
+  __device__ void operator()(int rhs, int par, int64_t h, double*) const {
+    using AT = typename AccT<P>::T;
+    const AT be = (AT)*beta_of();
+    cpx<AT> vp[NC], vr[NC];
+    ldv<P, NC, AT>(p, rhs, par, h, vp);
+    ldv<P, NC, AT>(r, rhs, par, h, vr);
+#pragma unroll
+    for (int i = 0; i < NC; ++i) vp[i] = vr[i] + be * vp[i];
+    stv<P, NC, AT>(p, rhs, par, h, vp);
+  }
+  __device__ void finalize(int, const double*) const {}
+};
 // p = r + beta p
 template <int P, int NC>
 struct CgP {
@@ -464,13 +543,15 @@ struct GmStart {
   }
 };
 
-// h_ij = s_i <V'_i, w>, i <= j: the column's j + 1 dot products, GM_DG of them
-// per block (launch index y = rhs * groups + group), so that the groups run
-// side by side and a block reduces 2 GM_DG numbers; one block over all columns
-// took 8-21 us a launch on 8^4, growing with j.
+// <V'_i, w>, i <= j: the column's j + 1 dot products, GM_DG of them per block
+// (launch index y = rhs * groups + group), so that the groups run side by side
+// and a block reduces 2 GM_DG numbers (one block over all columns took 8-21 us
+// a launch on 8^4, growing with j).  Left as block partials: GmOrtho's blocks
+// make the Hessenberg column of them.
 constexpr int GM_DG = 4;
 template <int P, int NC>
 struct GmDots {
+  static constexpr bool PARTIALS = true;
   VList V;
   DField w;
   KState* st;
@@ -489,38 +570,59 @@ struct GmDots {
       acc_dot<NC, AT>(vi, vw, acc + 2 * i);
     }
   }
-  __device__ void finalize(int y, const double* s) const {
-    const int rhs = y / groups, g = y - rhs * groups;
-    KState& k = st[rhs];
-    if (k.skip) return;
-    if (g == 0) k.iters += 1;
-#pragma unroll
-    for (int i = 0; i < GM_DG; ++i) {
-      const int c = GM_DG * g + i;
-      if (c <= j) k.H[c * GM_MAXK + j] = make_double2(k.s[c] * s[2 * i], k.s[c] * s[2 * i + 1]);
-    }
-  }
+  __device__ void finalize(int, const double*) const {}
 };
 
 // V'_{j+1} = w - sum_i h_ij v_i ; h_{j+1,j} = |V'_{j+1}| ; Givens rotation of column j
+// (h_ij = s_i <V'_i, w> from GmDots's partials, summed by every block; block 0
+// of the right-hand side stores the column for the last block's rotation)
 template <int P, int NC>
 struct GmOrtho {
   VList V;
   DField w;
   KState* st;
   int j;
-  __device__ bool active(int q) const { return !st[q].skip; }
+  const double* dots;  // [rhs * groups + group][nslots][2 GM_DG]
+  int nslots;
+  __device__ static double2* coef() {  // h_ij s_i
+    __shared__ double2 c[GM_MAXK];
+    return c;
+  }
+  __device__ bool active(int) const { return true; }
+  __device__ bool prologue(int q, bool first) const {
+    KState& k = st[q];
+    const bool run = !k.skip;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int groups = j / GM_DG + 1;
+    double* c = reinterpret_cast<double*>(coef());
+    for (int v = warp; v < 2 * (j + 1); v += nw) {
+      const int i = v >> 1;
+      const double* p = dots + (int64_t)(q * groups + i / GM_DG) * nslots * (2 * GM_DG) + 2 * (i % GM_DG) + (v & 1);
+      const double si = k.s[i];
+      double s = 0.0;
+      for (int b = lane; b < nslots; b += 32) s += __ldcg(p + (int64_t)b * (2 * GM_DG));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const double h = si * s;
+      if (lane == 0) {
+        c[v] = h * si;
+        if (first && run) reinterpret_cast<double*>(&k.H[i * GM_MAXK + j])[v & 1] = h;
+      }
+    }
+    if (first && run && threadIdx.x == 0) k.iters += 1;
+    __syncthreads();
+    return run;
+  }
   __device__ void operator()(int rhs, int par, int64_t h, double* acc) const {
     using AT = typename AccT<P>::T;
-    const KState& k = st[rhs];
+    const double2* c = coef();
     cpx<AT> vw[NC];
     ldv<P, NC, AT>(w, rhs, par, h, vw);
 #pragma unroll 4
     for (int i = 0; i <= j; ++i) {
       cpx<AT> vi[NC];
       ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
-      const double2 c = k.H[i * GM_MAXK + j];
-      const cpx<AT> cc = mk<AT>((AT)(c.x * k.s[i]), (AT)(c.y * k.s[i]));
+      const cpx<AT> cc = mk<AT>((AT)c[i].x, (AT)c[i].y);
 #pragma unroll
       for (int m = 0; m < NC; ++m) vw[m] = vw[m] - cc * vi[m];
     }

@@ -54,8 +54,16 @@ constexpr int cgm_ring(int nc) { return nc == 3 ? 8 : 2; }
 //   p_k^j = cg_k p_k^s + sum_u cc_k[u] r_{s+u},
 //   x_k^j = x_k^s + ch_k p_k^s + sum_u ce_k[u] r_{s+u},
 // and one flush per block writes x_k^{s+M}, p_k^{s+M}.
+//
+// The scalars of an iteration are computed by their consumers (block_total):
+// CgmR's blocks add up (p, A p) to alpha, CgmP's blocks |r|^2 to beta, and the
+// first block of each writes the state, the shifts' recurrences included, while
+// the others work.  |r|^2 alternates between rr and rr1 (iteration parity), so
+// that block 0 of CgmP replaces neither value the other blocks read.  Only the
+// last iteration of a block, whose flush needs every shift's coefficients, has
+// them finalised by CgmR's last block.
 struct CgmState {
-  double rr, bb, tol2, alpha, alpha_old, beta, pq;
+  double rr, rr1, bb, tol2, alpha, alpha_old, beta;
   int iters, done, nshift, nvalid;  // nvalid: residuals of the current block in the ring
   double shift[CGM_MAXSHIFT];
   double zeta[CGM_MAXSHIFT], zeta_old[CGM_MAXSHIFT], zeta_new[CGM_MAXSHIFT];
@@ -69,15 +77,12 @@ struct CgmState {
 
 namespace {
 
-// (p, q) -> alpha and the shifted alpha_k (Jegerlehner eq. for zeta_{n+1});
-// x_k^{j+1} = x_k^j + alpha_k p_k^j goes into the block coefficients.  t is
-// the iteration's position in its block (t = 0 opens a block: the previous
-// one was flushed).
+// (p, q), left as block partials (CgmR's blocks make alpha of them)
 template <int P, int NC>
 struct CgmAlpha {
+  static constexpr bool PARTIALS = true;
   DField p, q;
   CgmState* st;
-  int t;
   __device__ bool active(int) const { return !st->done; }
   __device__ void operator()(int, int par, int64_t h, double* acc) const {
     using AT = typename AccT<P>::T;
@@ -89,152 +94,186 @@ struct CgmAlpha {
     for (int k = 0; k < NC; ++k) re += a[k].x * b[k].x + a[k].y * b[k].y;
     acc[0] += (double)re;
   }
-  // shift k's part of the finalize; every load comes before the first store,
-  // so one round of memory latency covers them
-  __device__ void shift_alpha(CgmState& c, int k, bool go, double alpha, double beta, double aold) const {
-    constexpr int R = CGM_RING_MAX;
-    const int act = c.active[k];
-    const double zn = c.zeta[k], zo = c.zeta_old[k], sh = c.shift[k];
-    double cg = 1.0, ch = 0.0, cc[R + 1], ce[R + 1];
-#pragma unroll
-    for (int u = 1; u <= R; ++u) cc[u] = ce[u] = 0.0;
-    if (t > 0) {
-      cg = c.cg[k];
-      ch = c.ch[k];
-#pragma unroll
-      for (int u = 1; u <= R; ++u)
-        if (u <= t) {
-          cc[u] = c.cc[k][u];
-          ce[u] = c.ce[k][u];
-        }
-    } else {
-      // a block opens: the previous one was flushed
-      c.pend_x[k] = c.pend_p[k] = 0;
-      c.cg[k] = 1.0;
-      c.ch[k] = 0.0;
-#pragma unroll
-      for (int u = 0; u <= R; ++u) c.cc[k][u] = c.ce[k][u] = 0.0;
-    }
-    if (!go || !act) return;
-    const double den = alpha * beta * (zo - zn) + zo * aold * (1.0 + sh * alpha);
-    const double znew = zn * zo * aold / den;
-    const double ak = alpha * znew / zn;
-    c.zeta_new[k] = znew;
-    c.alpha_k[k] = ak;
-    c.ch[k] = ch + ak * cg;
-#pragma unroll
-    for (int u = 1; u <= R; ++u)
-      if (u <= t) c.ce[k][u] = ce[u] + ak * cc[u];
-    c.pend_x[k] = 1;
-  }
-  // warp 0 of the last block: lane l owns the shifts k = l, l + 32.  Runs on
-  // every replayed iteration, also once all shifts are done, so a flushed
-  // block is never applied twice.
-  __device__ void finalize_warp(int, const double* s, int lane) const {
-    CgmState& c = *st;
-    const int ns = c.nshift, done = c.done;
-    const double rr = c.rr, beta = c.beta, aold = c.alpha_old;
-    const bool ok = s[0] > 0.0 && !bad(s[0]);
-    const bool go = !done && ok;
-    const double alpha = rr / s[0];
-    if (lane < ns) shift_alpha(c, lane, go, alpha, beta, aold);
-    if (lane + 32 < ns) shift_alpha(c, lane + 32, go, alpha, beta, aold);
-    __syncwarp();
-    if (lane == 0) {
-      if (t == 0) c.nvalid = 0;
-      if (!done) {
-        c.iters += 1;
-        if (ok) c.alpha = alpha;
-        else c.done = 2;
-      }
-    }
-  }
 };
 
-// r_{j+1} = r_j - alpha q (ring slots t -> t + 1 mod M); |r|^2 -> beta,
-// beta_k, p_k^{j+1} = zeta_k r_{j+1} + beta_k p_k^j into the coefficients,
-// convergence per shift
-template <int P, int NC>
+// Shift k's part of the alpha step: alpha_k (Jegerlehner eq. for zeta_{n+1});
+// x_k^{j+1} = x_k^j + alpha_k p_k^j goes into the block coefficients.  t is the
+// iteration's position in its block (t = 0 opens a block: the previous one was
+// flushed).  Every load comes before the first store, so one round of memory
+// latency covers them.
+__device__ __forceinline__ void cgm_shift_alpha(CgmState& c, int k, int t, bool go, double alpha, double beta,
+                                                double aold) {
+  constexpr int R = CGM_RING_MAX;
+  const int act = c.active[k];
+  const double zn = c.zeta[k], zo = c.zeta_old[k], sh = c.shift[k];
+  double cg = 1.0, ch = 0.0, cc[R + 1], ce[R + 1];
+#pragma unroll
+  for (int u = 1; u <= R; ++u) cc[u] = ce[u] = 0.0;
+  if (t > 0) {
+    cg = c.cg[k];
+    ch = c.ch[k];
+#pragma unroll
+    for (int u = 1; u <= R; ++u)
+      if (u <= t) {
+        cc[u] = c.cc[k][u];
+        ce[u] = c.ce[k][u];
+      }
+  } else {
+    // a block opens: the previous one was flushed
+    c.pend_x[k] = c.pend_p[k] = 0;
+    c.cg[k] = 1.0;
+    c.ch[k] = 0.0;
+#pragma unroll
+    for (int u = 0; u <= R; ++u) c.cc[k][u] = c.ce[k][u] = 0.0;
+  }
+  if (!go || !act) return;
+  const double den = alpha * beta * (zo - zn) + zo * aold * (1.0 + sh * alpha);
+  const double znew = zn * zo * aold / den;
+  const double ak = alpha * znew / zn;
+  c.zeta_new[k] = znew;
+  c.alpha_k[k] = ak;
+  c.ch[k] = ch + ak * cg;
+#pragma unroll
+  for (int u = 1; u <= R; ++u)
+    if (u <= t) c.ce[k][u] = ce[u] + ak * cc[u];
+  c.pend_x[k] = 1;
+}
+
+// Shift k's part of the beta step: beta_k and p_k^{j+1} = zeta_k r_{j+1} +
+// beta_k p_k^j into the coefficients, convergence.  Returns whether shift k
+// still iterates.
+__device__ __forceinline__ int cgm_shift_r(CgmState& c, int k, int t, double beta, double s0, double lim) {
+  constexpr int R = CGM_RING_MAX;
+  const int act = c.active[k];
+  const double znew = c.zeta_new[k], z = c.zeta[k], cg = c.cg[k];
+  double cc[R + 1];
+#pragma unroll
+  for (int u = 1; u <= R; ++u) cc[u] = u <= t ? c.cc[k][u] : 0.0;
+  if (!act) return 0;
+  const double ratio = znew / z;
+  const double bk = beta * ratio * ratio;
+  c.zeta_old[k] = z;
+  c.zeta[k] = znew;
+  c.cg[k] = cg * bk;
+#pragma unroll
+  for (int u = 1; u <= R; ++u)
+    if (u <= t) c.cc[k][u] = cc[u] * bk;
+  c.cc[k][t + 1] = znew;
+  const bool conv = znew * znew * s0 <= lim;
+  if (conv) c.active[k] = 0;
+  c.pend_p[k] = conv ? 0 : 1;
+  return conv ? 0 : 1;
+}
+
+// The whole beta step by one warp (lane l owns the shifts l, l + 32)
+__device__ __forceinline__ void cgm_beta_step(CgmState& c, int t, double s0, int lane) {
+  const int ns = c.nshift;
+  const double rr = (t & 1) ? c.rr1 : c.rr, lim = c.tol2 * c.bb;
+  if (bad(s0)) {
+    if (lane == 0) c.done = 2;
+    return;
+  }
+  const double beta = s0 / rr;
+  int nact = 0;
+  if (lane < ns) nact += cgm_shift_r(c, lane, t, beta, s0, lim);
+  if (lane + 32 < ns) nact += cgm_shift_r(c, lane + 32, t, beta, s0, lim);
+  nact = __reduce_add_sync(0xffffffffu, nact);
+  if (lane == 0) {
+    c.nvalid = t + 1;
+    c.alpha_old = c.alpha;
+    c.beta = beta;
+    if ((t & 1) || nact == 0) c.rr = s0;
+    if (!(t & 1) || nact == 0) c.rr1 = s0;
+    if (nact == 0) c.done = 1;
+  }
+}
+
+// a scalar the prologue of a block leaves to its sites
+__device__ __forceinline__ double* cgm_scalar() {
+  __shared__ double v;
+  return &v;
+}
+
+// alpha = |r|^2 / (p, q); r_{j+1} = r_j - alpha q (ring slots t -> t + 1 mod M);
+// |r|^2.  LAST: finalised here (the flush follows), else left to CgmP.
+template <int P, int NC, bool LAST>
 struct CgmR {
+  static constexpr bool PARTIALS = !LAST;
   DField ring, q;
   CgmState* st;
   int t, M;
-  __device__ bool active(int) const { return !st->done; }
+  const double* pq;  // npq partials of (p, q)
+  int npq;
+  __device__ bool active(int) const { return true; }
+  // block 0 runs the shifts' alpha step on every replayed iteration, also once
+  // all shifts are done, so a flushed block is never applied twice
+  __device__ bool prologue(int, bool first) const {
+    CgmState& c = *st;
+    const int done = c.done;
+    const double rr = (t & 1) ? c.rr1 : c.rr;
+    const double s = block_total(pq, npq);
+    const bool ok = s > 0.0 && !bad(s);
+    const double alpha = rr / s;
+    const bool go = !done && ok;
+    if (threadIdx.x == 0) *cgm_scalar() = alpha;
+    __syncthreads();
+    if (first && threadIdx.x < 32) {
+      const int lane = (int)threadIdx.x, ns = c.nshift;
+      const double beta = c.beta, aold = c.alpha_old;
+      if (lane < ns) cgm_shift_alpha(c, lane, t, go, alpha, beta, aold);
+      if (lane + 32 < ns) cgm_shift_alpha(c, lane + 32, t, go, alpha, beta, aold);
+      if (lane == 0) {
+        if (t == 0) c.nvalid = 0;
+        if (!done) {
+          c.iters += 1;
+          if (ok) c.alpha = alpha;
+          else c.done = 2;
+        }
+      }
+    }
+    return go;
+  }
   __device__ void operator()(int, int par, int64_t h, double* acc) const {
     using AT = typename AccT<P>::T;
     cpx<AT> vr[NC], vq[NC];
     ldv<P, NC, AT>(ring, t, par, h, vr);
     ldv<P, NC, AT>(q, 0, par, h, vq);
-    const AT a = (AT)st->alpha;
+    const AT a = (AT)*cgm_scalar();
 #pragma unroll
     for (int i = 0; i < NC; ++i) vr[i] = vr[i] - a * vq[i];
     stv<P, NC, AT>(ring, (t + 1) % M, par, h, vr);
     acc[0] += site_norm2<NC, AT>(vr);
   }
-  // shift k's part; loads before stores (one round of memory latency).
-  // Returns whether shift k still iterates.
-  __device__ int shift_r(CgmState& c, int k, double beta, double s0, double lim) const {
-    constexpr int R = CGM_RING_MAX;
-    const int act = c.active[k];
-    const double znew = c.zeta_new[k], z = c.zeta[k], cg = c.cg[k];
-    double cc[R + 1];
-#pragma unroll
-    for (int u = 1; u <= R; ++u) cc[u] = u <= t ? c.cc[k][u] : 0.0;
-    if (!act) return 0;
-    const double ratio = znew / z;
-    const double bk = beta * ratio * ratio;
-    c.zeta_old[k] = z;
-    c.zeta[k] = znew;
-    c.cg[k] = cg * bk;
-#pragma unroll
-    for (int u = 1; u <= R; ++u)
-      if (u <= t) c.cc[k][u] = cc[u] * bk;
-    c.cc[k][t + 1] = znew;
-    const bool conv = znew * znew * s0 <= lim;
-    if (conv) c.active[k] = 0;
-    c.pend_p[k] = conv ? 0 : 1;
-    return conv ? 0 : 1;
-  }
-  // warp 0 of the last block: lane l owns the shifts k = l, l + 32
   __device__ void finalize_warp(int, const double* s, int lane) const {
-    CgmState& c = *st;
-    const int ns = c.nshift, done = c.done;
-    const double rr = c.rr, lim = c.tol2 * c.bb;
-    if (done) return;
-    if (bad(s[0])) {
-      __syncwarp();
-      if (lane == 0) c.done = 2;
-      return;
-    }
-    const double beta = s[0] / rr;
-    int nact = 0;
-    if (lane < ns) nact += shift_r(c, lane, beta, s[0], lim);
-    if (lane + 32 < ns) nact += shift_r(c, lane + 32, beta, s[0], lim);
-    nact = __reduce_add_sync(0xffffffffu, nact);
-    __syncwarp();  // every lane has read rr before lane 0 replaces it
-    if (lane == 0) {
-      c.nvalid = t + 1;
-      c.alpha_old = c.alpha;
-      c.beta = beta;
-      c.rr = s[0];
-      if (nact == 0) c.done = 1;
-    }
+    if (!st->done) cgm_beta_step(*st, t, s[0], lane);
   }
 };
 
-// p = r_{j+1} + beta p (ring slot `slot`), inside a block
+// beta = |r_{j+1}|^2 / |r_j|^2; p = r_{j+1} + beta p (ring slot t + 1), inside a block
 template <int P, int NC>
 struct CgmP {
   DField ring, p;
   CgmState* st;
-  int slot;
-  __device__ bool active(int) const { return !st->done; }
+  int t;
+  const double* rrp;  // nrr partials of |r_{j+1}|^2
+  int nrr;
+  __device__ bool active(int) const { return true; }
+  __device__ bool prologue(int, bool first) const {
+    CgmState& c = *st;
+    const int done = c.done;
+    const double rr = (t & 1) ? c.rr1 : c.rr;
+    const double s = block_total(rrp, nrr);
+    if (threadIdx.x == 0) *cgm_scalar() = s / rr;
+    __syncthreads();
+    if (first && threadIdx.x < 32 && !done) cgm_beta_step(c, t, s, (int)threadIdx.x);
+    return !done && !bad(s);
+  }
   __device__ void operator()(int, int par, int64_t h, double*) const {
     using AT = typename AccT<P>::T;
     cpx<AT> vr[NC], vp[NC];
-    ldv<P, NC, AT>(ring, slot, par, h, vr);
+    ldv<P, NC, AT>(ring, t + 1, par, h, vr);
     ldv<P, NC, AT>(p, 0, par, h, vp);
-    const AT b = (AT)st->beta;
+    const AT b = (AT)*cgm_scalar();
 #pragma unroll
     for (int i = 0; i < NC; ++i) vp[i] = vr[i] + b * vp[i];
     stv<P, NC, AT>(p, 0, par, h, vp);
@@ -334,7 +373,7 @@ struct CgmInit {
   }
   __device__ void finalize(int, const double* s) const {
     CgmState& c = *st;
-    c.rr = c.bb = s[0];
+    c.rr = c.rr1 = c.bb = s[0];
     c.alpha_old = 1.0;
     c.beta = 0.0;
     c.iters = 0;
@@ -426,7 +465,10 @@ struct CgmWork : SolveCacheBase {
   int M = 1;  // ring length (residuals per flush block)
   CgmState* st = nullptr;
   CgmState* hs = nullptr;  // pinned copy read per chunk
+  double* part = nullptr;  // block partials of (p, A p), then of |r|^2
+  int64_t npart = 0;       // room for each
   ~CgmWork() {
+    dfree(part);
     dfree(st);
     if (hs) cudaFreeHost(hs);
   }
@@ -440,6 +482,8 @@ struct CgmWork : SolveCacheBase {
       return s;
     if (P != CLG_PREC_DOUBLE && (s = it[1].alloc(ctx, P, nc, np, fp, M, Vh, op))) return s;
     if ((s = dalloc(ctx, (void**)&st, sizeof(CgmState)))) return s;
+    npart = std::max<int64_t>(site_blocks<1>(ctx, np, Vh, 1), (Vh + 255) / 256);
+    if ((s = dalloc(ctx, (void**)&part, sizeof(double) * 2 * npart))) return s;
     if (cudaMallocHost((void**)&hs, sizeof(CgmState)) != cudaSuccess) {
       hs = nullptr;
       return ctx->fail(CLG_ERR_OOM, "multi-shift: pinned state");
@@ -453,7 +497,7 @@ struct CgmWork : SolveCacheBase {
 // epilogue: the iteration needs no separate pass over p and q.
 template <int PR, int NC>
 clg_status cgm_schur_alpha(clg_context_s* ctx, CgmIter& I, clg_gauge_s* U, int kind, double param, CgmState* st,
-                           int t) {
+                           double* part, int* npart) {
   HopSpec s1;
   s1.kind = kind;
   s1.prec = PR;
@@ -481,18 +525,14 @@ clg_status cgm_schur_alpha(clg_context_s* ctx, CgmIter& I, clg_gauge_s* U, int k
   if (clg_status e = make_hop_args(ctx, U, s2, a)) return e;
   const int bs = 256;
   const int64_t nb = (a.g.Vh + bs - 1) / bs;
-  if (clg_status e = ensure_reduction(ctx, nb)) return e;
-  const CgmAlpha<PR, NC> f{dfield(I.p.ref), dfield(I.q.ref), st, t};
+  *npart = (int)nb;
   cudaError_t err;
   if constexpr (PR == P64)
-    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P64, 18, 3, CgmAlpha<PR, NC>>, dim3((unsigned)nb), dim3(bs), 0, a,
-                     f, ctx->red_partials, ctx->red_counter);
+    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P64, 18, 3>, dim3((unsigned)nb), dim3(bs), 0, a, part);
   else if (U->recon32 == 12)
-    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P32, 12, 4, CgmAlpha<PR, NC>>, dim3((unsigned)nb), dim3(bs), 0, a,
-                     f, ctx->red_partials, ctx->red_counter);
+    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P32, 12, 4>, dim3((unsigned)nb), dim3(bs), 0, a, part);
   else
-    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P32, 18, 4, CgmAlpha<PR, NC>>, dim3((unsigned)nb), dim3(bs), 0, a,
-                     f, ctx->red_partials, ctx->red_counter);
+    err = launch_pdl(ctx, staggered_hop_xdot_kernel<P32, 18, 4>, dim3((unsigned)nb), dim3(bs), 0, a, part);
   if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("multi-shift hop: ") + cudaGetErrorString(err));
   return CLG_SUCCESS;
 }
@@ -513,22 +553,26 @@ clg_status cgm_chunk(clg_context_s* ctx, CgmWork& W, CgmIter& I, clg_gauge_s* U,
     clg_status e;
     bool fused = false;
     if constexpr (PR != P16 && NC == 3) fused = op == CLG_OP_DDDAG_EE && ctx->fused_cg;
+    double *pq = W.part, *rrp = W.part + W.npart;
+    int npq = (int)site_blocks<1>(ctx, np, Vh, 1);
+    const int nrr = npq;
     if (fused) {
       if constexpr (PR != P16 && NC == 3)
-        if ((e = cgm_schur_alpha<PR, NC>(ctx, I, U, kind, param, st, t))) return e;
+        if ((e = cgm_schur_alpha<PR, NC>(ctx, I, U, kind, param, st, pq, &npq))) return e;
     } else {
       if ((e = apply_op(ctx, op, U, kind, param, I.q.ref, I.p.ref, tmp, one, 1, nullptr, 0, skip, 0))) return e;
-      if ((e = launch_sites<1>(ctx, CgmAlpha<PR, NC>{dfield(I.p.ref), dfield(I.q.ref), st, t}, fp, np, Vh, 1)))
+      if ((e = launch_sites<1>(ctx, CgmAlpha<PR, NC>{dfield(I.p.ref), dfield(I.q.ref), st}, fp, np, Vh, 1, pq)))
         return e;
     }
-    if ((e = launch_sites<1>(ctx, CgmR<PR, NC>{dfield(I.ring.ref), dfield(I.q.ref), st, t, MV}, fp, np, Vh, 1)))
-      return e;
-    if (t + 1 < MV)
-      e = launch_sites<0>(ctx, CgmP<PR, NC>{dfield(I.ring.ref), dfield(I.p.ref), st, t + 1}, fp, np, Vh, 1);
-    else
+    const DField ring = dfield(I.ring.ref), q = dfield(I.q.ref);
+    if (t + 1 < MV) {
+      if ((e = launch_sites<1>(ctx, CgmR<PR, NC, false>{ring, q, st, t, MV, pq, npq}, fp, np, Vh, 1, rrp))) return e;
+      e = launch_sites<0>(ctx, CgmP<PR, NC>{ring, dfield(I.p.ref), st, t, rrp, nrr}, fp, np, Vh, 1);
+    } else {
+      if ((e = launch_sites<1>(ctx, CgmR<PR, NC, true>{ring, q, st, t, MV, pq, npq}, fp, np, Vh, 1))) return e;
       e = launch_sites<0>(
-          ctx, CgmFlush<PR, NC, MV>{dfield(I.ring.ref), dfield(W.X.ref), dfield(W.pk.ref), dfield(I.p.ref), st, ns},
-          fp, np, Vh, 1);
+          ctx, CgmFlush<PR, NC, MV>{ring, dfield(W.X.ref), dfield(W.pk.ref), dfield(I.p.ref), st, ns}, fp, np, Vh, 1);
+    }
     if (e) return e;
   }
   return CLG_SUCCESS;

@@ -24,6 +24,71 @@ struct has_warp_finalize : std::false_type {};
 template <class F>
 struct has_warp_finalize<F, std::void_t<decltype(&F::finalize_warp)>> : std::true_type {};
 
+// A reduction whose result the next kernel needs can leave the last step to it:
+// the producer's blocks only write their partials (block_partials) and end, and
+// every block of the consumer adds them up itself (block_total, the same order
+// in every block) while its own loads are in flight.  The fence, the ticket,
+// the last block's second pass and its scalar update, 4 to 6 us at the end of a
+// launch during which nothing else runs, become about 1 us beside other work.
+// For few partials (a launch of one right-hand side).
+template <int NRED>
+__device__ __forceinline__ void block_partials(const double (&acc)[NRED], double* partials, unsigned slot) {
+  __shared__ double sm[NRED][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < NRED; ++k) {
+    double v = acc[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) sm[k][warp] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < NRED) {
+    double v = 0.0;
+    for (int w = 0; w < nw; ++w) v += sm[threadIdx.x][w];
+    partials[(int64_t)slot * NRED + threadIdx.x] = v;
+  }
+}
+// sum of n partials, the same in every thread of the block (at most 8 warps)
+__device__ __forceinline__ double block_total(const double* partials, int n) {
+  __shared__ double sm[8];
+  constexpr int U = 4;
+  double s = 0.0;
+  for (int i0 = threadIdx.x; i0 < n; i0 += U * (int)blockDim.x) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * (int)blockDim.x;
+      v[u] = i < n ? __ldcg(partials + i) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  double t = 0.0;
+  for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) t += sm[w];
+  return t;
+}
+// A site functor with PARTIALS = true leaves its partials to the next kernel; one
+// with a member prologue(rhs, first block) has it run by every thread before the
+// sites (it may hold barriers) and returns whether there is work.
+template <class F, class = void>
+struct partials_only : std::false_type {};
+template <class F>
+struct partials_only<F, std::void_t<decltype(F::PARTIALS)>> : std::bool_constant<F::PARTIALS> {};
+template <class F, class = void>
+struct has_prefetch : std::false_type {};
+template <class F>
+struct has_prefetch<F, std::void_t<decltype(&F::prefetch)>> : std::true_type {};
+template <class F, class = void>
+struct has_prologue : std::false_type {};
+template <class F>
+struct has_prologue<F, std::void_t<decltype(&F::prologue)>> : std::true_type {};
+
 // The last block's part: totals per right-hand side -> f.finalize.  Called by
 // every thread of that block (at most 256 threads, 8 warps).
 template <int NRED, class F>

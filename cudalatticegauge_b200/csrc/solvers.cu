@@ -304,6 +304,20 @@ struct Work : public SolveCacheBase {
   double2* shift_dev = nullptr;  // per-rhs shift sigma_r: the system is (op + sigma_r) x_r = b_r
   // Krylov operator temporaries (precision P)
   Owned kt_odd, kt_even, kt_full;
+  // block partials left to the next kernel: CG on one right-hand side ((p, A p),
+  // then |r|^2), GMRES (a column's inner products)
+  double* part = nullptr;
+  int64_t npart = 0;
+  clg_status partials(int64_t doubles) {
+    if (doubles <= npart) return CLG_SUCCESS;
+    if (part) cudaStreamSynchronize(ctx->stream);
+    dfree(part);
+    part = nullptr;
+    npart = 0;
+    if (clg_status s = dalloc(ctx, (void**)&part, sizeof(double) * doubles)) return s;
+    npart = doubles;
+    return CLG_SUCCESS;
+  }
   // Krylov vectors per graph slot: they persist for the whole solve so a
   // captured graph stays valid across defect-correction cycles
   std::map<int, std::vector<std::unique_ptr<Owned>>> kv;
@@ -339,6 +353,7 @@ struct Work : public SolveCacheBase {
       if (g) cudaGraphExecDestroy(g);
     dfree(ctl_d);
     if (ctl_h) cudaFreeHost(ctl_h);
+    dfree(part);
     dfree(st);
     dfree(sum_d);
     dfree(outer_done_d);
@@ -772,6 +787,54 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   return CLG_SUCCESS;
 }
 
+// The same for one right-hand side with the block sums of e left in part
+// (*npart of them) for the next kernel
+template <int P, int RECON, class E>
+cudaError_t launch_hop_epi1(clg_context_s* ctx, const HopArgs& a, const E& e, bool dag, int bs, double* part) {
+  constexpr int MINB = P == P64 ? 1 : 3;
+  const dim3 grid((unsigned)((a.g.Vh + bs - 1) / bs));
+  if (bs == SPLIT_SITES) {
+    auto k = dag ? wilson_split_epi_kernel<P, RECON, true, E> : wilson_split_epi_kernel<P, RECON, false, E>;
+    return launch_pdl(ctx, k, grid, dim3(4 * SPLIT_SITES), 0, a, e, part, (double*)nullptr, (unsigned*)nullptr, 1u);
+  }
+  auto k = dag ? wilson_hop_epi_kernel<P, RECON, true, 256, MINB, E> : wilson_hop_epi_kernel<P, RECON, false, 256, MINB, E>;
+  return launch_pdl(ctx, k, grid, dim3(bs), 0, a, e, part, (double*)nullptr, (unsigned*)nullptr, 1u);
+}
+template <int P, class E>
+clg_status schur_hop_epi1(Work& w, bool dag, const FieldRef& t_odd, const FieldRef& in_even, const FieldRef& out_even,
+                          const E& e, const int* skip, int ks, double* part, int* npart) {
+  clg_context_s* ctx = w.ctx;
+  HopSpec s{};
+  s.kind = CLG_FERMION_WILSON;
+  s.prec = P;
+  s.dagger = dag;
+  s.out_parity = 0;
+  s.in = t_odd;
+  s.out = out_even;
+  s.x = &in_even;
+  s.a = make_double2(-w.param * w.param, 0.0);
+  s.xa = make_double2(1.0, 0.0);
+  s.skip_dev = skip;
+  s.skip_stride = ks;
+  s.nrhs = 1;
+  HopArgs a;
+  if (clg_status st = make_hop_args(ctx, w.U, s, a)) return st;
+  HopSpec plain = s;
+  plain.x = nullptr;
+  const int cfg = tuned_hop_config(ctx, w.U, plain, P == P64 ? 64 : 128);
+  const int bs = (cfg >> 16) == HOP_SPLIT ? SPLIT_SITES : cfg & 0xffff;
+  *npart = (int)((w.Vh + bs - 1) / bs);
+  cudaError_t err;
+  if constexpr (P == P64)
+    err = launch_hop_epi1<P, 18>(ctx, a, e, dag, bs, part);
+  else if (P == P16 || w.U->recon32 == 12)
+    err = launch_hop_epi1<P, 12>(ctx, a, e, dag, bs, part);
+  else
+    err = launch_hop_epi1<P, P == P16 ? 12 : 18>(ctx, a, e, dag, bs, part);
+  if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("fused hop: ") + cudaGetErrorString(err));
+  return CLG_SUCCESS;
+}
+
 // t_o = H_oe^(dag) in_e
 }  // namespace (a kernel's template argument must not have internal linkage)
 
@@ -829,12 +892,16 @@ clg_status fused_residual_t(Work& w, bool dag, const FieldRef& b, const FieldRef
     a.tile_rows = full_rows(a.g, 4 * 144 + 4 * 192 + 12 * 8);
     const ResidHop<PI> e{dfield(b), dfield(r), dfield(rp), 0, true, out};
     constexpr int bs = 128;
-    const int64_t nslots = 2 * ((w.Vh + bs - 1) / bs);
+    const bool split = 2 * w.Vh <= SPLIT_ALWAYS;
+    const int sites = split ? SPLIT_SITES : bs;
+    const int64_t nslots = 2 * ((w.Vh + sites - 1) / sites);
     if (clg_status st = ensure_reduction(ctx, red2_doubles(nslots, 1, 1, 1))) return st;
     const unsigned group = red_group(nslots, 1);
     double* gpart = ctx->red_partials + nslots;
-    auto kern = dag ? wilson_full_epi_kernel<P64, 18, true, 256, 2, ResidHop<PI>>
-                    : wilson_full_epi_kernel<P64, 18, false, 256, 2, ResidHop<PI>>;
+    auto kern = dag ? (split ? wilson_split_epi_kernel<P64, 18, true, ResidHop<PI>, true>
+                             : wilson_full_epi_kernel<P64, 18, true, 256, 2, ResidHop<PI>>)
+                    : (split ? wilson_split_epi_kernel<P64, 18, false, ResidHop<PI>, true>
+                             : wilson_full_epi_kernel<P64, 18, false, 256, 2, ResidHop<PI>>);
     const cudaError_t err = launch_pdl(ctx, kern, dim3((unsigned)nslots), dim3(bs), 0, a, e, ctx->red_partials, gpart,
                                        ctx->red_counter, group);
     if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("residual hop: ") + cudaGetErrorString(err));
@@ -880,7 +947,8 @@ clg_status fused_residual(Work& w, bool dag, const FieldRef& b, const FieldRef& 
                                   : fused_residual_t<P64>(w, dag, b, x, r, rp, out);
 }
 
-clg_status schur_hop_odd(Work& w, bool dag, const FieldRef& in_even, const FieldRef& t_odd, const int* skip, int ks) {
+clg_status schur_hop_odd(Work& w, bool dag, const FieldRef& in_even, const FieldRef& t_odd, const int* skip, int ks,
+                         const AlphaFin* fin = nullptr) {
   HopSpec s;
   s.kind = CLG_FERMION_WILSON;
   s.prec = t_odd.prec;
@@ -896,6 +964,7 @@ clg_status schur_hop_odd(Work& w, bool dag, const FieldRef& in_even, const Field
   s.skip_dev = skip;
   s.skip_stride = ks;
   s.nrhs = w.nrhs;
+  s.fin = fin;
   return hop(w.ctx, w.U, s);
 }
 
@@ -915,6 +984,30 @@ clg_status cg_fused_iteration(Work& w, int op, const FieldRef& x, const FieldRef
   if ((s = schur_hop_epi<P>(w, d1, to, p, te, CgHopAlpha<P>{w.st, op_weight(op)}, skip, ks))) return s;
   if ((s = schur_hop_odd(w, !d1, te, to, skip, ks))) return s;
   return schur_hop_epi<P>(w, !d1, to, te, te, CgHopUpdate<P>{dfield(x), dfield(r), dfield(p), w.st}, skip, ks);
+}
+
+// The same for one right-hand side, with p = r + beta p: the reductions'
+// results are made by the kernels that need them (Cg1HopAlpha .. Cg1P).  On the
+// 32^3x16 FP16-inner solve (ncu, warm): alpha hop 27.1 -> 22.8 us, update hop
+// 34.5 -> 30.7, p 9.8 -> 12.4; the solve 13.07 -> 12.39 ms.
+template <int P>
+clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, const FieldRef& p, const int* skip,
+                         int ks, int odd) {
+  const bool d1 = op == CLG_OP_MEE_MEEDAG;
+  const FieldRef& to = w.kt_odd.ref;
+  const FieldRef& te = w.kt_even.ref;
+  const int64_t most = (w.Vh + SPLIT_SITES - 1) / SPLIT_SITES;
+  double *pap = w.part, *rrp = w.part + most;
+  int npap = 0, nrr = 0;
+  KState* st = w.st;
+  clg_status s;
+  if ((s = schur_hop_odd(w, d1, p, to, skip, ks))) return s;
+  if ((s = schur_hop_epi1<P>(w, d1, to, p, te, Cg1HopAlpha<P>{{st, 0}}, skip, ks, pap, &npap))) return s;
+  const AlphaFin fin{pap, npap, odd ? &st->rr1 : &st->rr, &st->alpha, &st->status, &st->done, &st->skip, ST_BREAKDOWN};
+  if ((s = schur_hop_odd(w, !d1, te, to, skip, ks, &fin))) return s;
+  const Cg1HopUpdate<P> up{{dfield(x), dfield(r), dfield(p), st}};
+  if ((s = schur_hop_epi1<P>(w, !d1, to, te, te, up, skip, ks, rrp, &nrr))) return s;
+  return launch_sites<0>(w.ctx, Cg1P<P, 12>{dfield(p), dfield(r), st, rrp, nrr, odd, op_weight(op)}, 0, 1, w.Vh, 1);
 }
 
 clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slot_base) {
@@ -970,8 +1063,14 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       clg_status e = launch_sites<1>(ctx, init, fp, np, Vh, nrhs);
       if (e) return e;
       const bool fused = NV == 12 && fused_cg(w, op);
+      // (a pinned tile form has no block for AlphaFin)
+      const bool one = fused && nrhs == 1 && !w.U->seg && (ctx->hop_config < 0 || (ctx->hop_config >> 16) < 16);
+      if (one && (e = w.partials(2 * ((Vh + SPLIT_SITES - 1) / SPLIT_SITES)))) return e;
+      int it = 0;  // a chunk is an even number of iterations: replays keep the parity
       auto body = [&]() -> clg_status {
         clg_status e2;
+        if constexpr (NV == 12)
+          if (one) return cg1_iteration<PV>(w, op, x, r.ref, p.ref, skip, ks, it++ & 1);
         if (fused) {
           if constexpr (NV == 12)
             if ((e2 = cg_fused_iteration<PV>(w, op, x, r.ref, p.ref, skip, ks))) return e2;
@@ -1007,6 +1106,12 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       auto dv = [&](const FieldRef& f) { return dfield(pieces_view(f, pieces)); };
       VList vl;
       for (int i = 0; i <= GM_MAXK; ++i) vl.v[i] = dv(V[std::min(i, k)].ref);
+      int64_t most = 0;
+      for (int j = 0; j < k; ++j) {
+        const int n = nrhs * (j / GM_DG + 1);
+        most = std::max(most, site_blocks<2 * GM_DG>(ctx, nq, Vh, n) * n * 2 * GM_DG);
+      }
+      if (clg_status e = w.partials(most)) return e;
       // first cycle start (x = 0)
       GmStart<PV, NV> st0{dv(b), dv(wv.ref), dv(V[0].ref), w.st, 0, w.tol_d, 1};
       clg_status e = launch_sites<1>(ctx, st0, fq, nq, Vh, nrhs);
@@ -1025,9 +1130,11 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
             return e2;
           const int groups = j / GM_DG + 1;
           if ((e2 = launch_sites<2 * GM_DG>(ctx, GmDots<PV, NV>{vl, dv(wv.ref), w.st, j, groups}, fq, nq, Vh,
-                                            nrhs * groups)))
+                                            nrhs * groups, w.part)))
             return e2;
-          if ((e2 = launch_sites<1>(ctx, GmOrtho<PV, NV>{vl, dv(wv.ref), w.st, j}, fq, nq, Vh, nrhs))) return e2;
+          const int nslots = (int)site_blocks<2 * GM_DG>(ctx, nq, Vh, nrhs * groups);
+          if ((e2 = launch_sites<1>(ctx, GmOrtho<PV, NV>{vl, dv(wv.ref), w.st, j, w.part, nslots}, fq, nq, Vh, nrhs)))
+            return e2;
         }
         gm_solve_y<<<nrhs, 32, 0, ctx->stream>>>(w.st, nrhs);
         ctx->kernels++;
