@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
     }
   }
   if constexpr (partials_only<E>::value) {
-    block_partials<E::NRED>(red, partials, slot);  // one right-hand side
+    if (!skipped) block_partials<E::NRED>(red, partials, (int64_t)rhs * (gridDim.x / (unsigned)a.nrhs) + slot);
   } else {
     const int rr[1] = {rhs};
     const bool cc[1] = {!skipped}, hh[1] = {true};
@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopAr
     e.site(rhs, h, acc, red);
   }
   if constexpr (partials_only<E>::value) {
-    block_partials<E::NRED>(red, partials, slot);  // one right-hand side
+    if (!skipped) block_partials<E::NRED>(red, partials, (int64_t)rhs * (gridDim.x / (unsigned)a.nrhs) + slot);
   } else {
     const int rr[1] = {rhs};
     const bool cc[1] = {!skipped}, hh[1] = {true};
@@ -1189,10 +1189,23 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_pair_epi_kernel(HopArgs
       e.site(rhs1, h, acc1, red + E::NRED);
     }
   }
-  const int rr[2] = {rhs0, rhs1};
-  const bool cc[2] = {run0, run1}, hh[2] = {true, has1};
-  grid_reduce_finalize2<E::NRED, 2>(red, e, rr, cc, hh, (unsigned)(rhs0 / 2), npairs, slot, gridDim.x / npairs,
-                                    a.nrhs, group, partials, gpart, counter);
+  if constexpr (partials_only<E>::value) {
+    double r0[E::NRED], r1[E::NRED];
+#pragma unroll
+    for (int k = 0; k < E::NRED; ++k) {
+      r0[k] = red[k];
+      r1[k] = red[E::NRED + k];
+    }
+    const int64_t nslots = gridDim.x / npairs;
+    if (run0) block_partials<E::NRED>(r0, partials, rhs0 * nslots + slot);
+    __syncthreads();
+    if (run1) block_partials<E::NRED>(r1, partials, rhs1 * nslots + slot);
+  } else {
+    const int rr[2] = {rhs0, rhs1};
+    const bool cc[2] = {run0, run1}, hh[2] = {true, has1};
+    grid_reduce_finalize2<E::NRED, 2>(red, e, rr, cc, hh, (unsigned)(rhs0 / 2), npairs, slot, gridDim.x / npairs,
+                                      a.nrhs, group, partials, gpart, counter);
+  }
 }
 
 // ---------------------------------------------------------------- FP16, a tile of sites for every right-hand side
@@ -1421,8 +1434,10 @@ __device__ __forceinline__ void tile16_epi_body(const HopArgs& a, const E& e, Ti
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + k] = v;
     }
-    if (lane == 0) __threadfence();
+    if constexpr (!partials_only<E>::value)
+      if (lane == 0) __threadfence();
   }
+  if constexpr (partials_only<E>::value) return;  // left to the next kernel (a batch: this lattice's slots only)
   if (r0 > 0 || r1 < a.nrhs) {
     for (int q = threadIdx.x; q < a.nrhs * E::NRED; q += blockDim.x) {
       const int rhs = q / E::NRED;
@@ -1583,8 +1598,10 @@ __device__ __forceinline__ void tileN_epi_body(const HopArgs& a, const E& e, Til
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + k] = v;
     }
-    if (lane == 0) __threadfence();
+    if constexpr (!partials_only<E>::value)
+      if (lane == 0) __threadfence();
   }
+  if constexpr (partials_only<E>::value) return;  // left to the next kernel (a batch: this lattice's slots only)
   if (r0 > 0 || r1 < a.nrhs) {
     for (int q = threadIdx.x; q < a.nrhs * E::NRED; q += blockDim.x) {
       const int rhs = q / E::NRED;
@@ -1924,11 +1941,13 @@ __global__ void __launch_bounds__(256, MINB) wilson_hop_mma16_epi_kernel(HopArgs
         for (int o = MMA_TS / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, MMA_TS);
         if (live && i == 0) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + k] = v;
       }
-      if (live && i == 0) __threadfence();
+      if constexpr (!partials_only<E>::value)
+        if (live && i == 0) __threadfence();
     }
     __syncthreads();
   }
-  tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
+  if constexpr (!partials_only<E>::value)
+    tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
 }
 
 // The FP16 staggered direction on half2 words: o = U chi (UDAG: U^+ chi) with

@@ -6,6 +6,7 @@
 // copy: Core/CudaHelper.cu:697-710).
 #pragma once
 #include "blas.cuh"
+#include "dslash.cuh"
 
 namespace clg {
 
@@ -353,9 +354,12 @@ struct CgUpdate {
 // second hop of the second factor produces A p in registers only and applies
 //   x += alpha p,  r -= alpha A p,  |r|^2 -> beta
 // at its own site, so A p is never written and the separate (p, A p) and
-// update passes disappear.  Both act on the even checkerboard (parity 0).
+// update passes disappear.  Both act on the even checkerboard (parity 0); their
+// sums are left as partials for epi_final_kernel, or for the next kernel (one
+// right-hand side, Cg1P).
 template <int P>
 struct CgHopAlpha {
+  static constexpr bool PARTIALS = true;
   static constexpr int NRED = 1;
   static constexpr bool STORE = true;
   KState* st;
@@ -368,6 +372,7 @@ struct CgHopAlpha {
 };
 template <int P>
 struct CgHopUpdate {
+  static constexpr bool PARTIALS = true;
   static constexpr int NRED = 1;
   static constexpr bool STORE = false;
   DField x, r, p;
@@ -390,6 +395,48 @@ struct CgHopUpdate {
   }
   __device__ void finalize(int w, const double* s) const { cg_update_finalize(st[w], s[0]); }
 };
+// E::finalize of right-hand side blockIdx.x from the partials [rhs][nslots] its
+// hop left: all slots, or in a batch of lattices those of its lattice's tiles.
+// The 28-right-hand-side update hop of 32^3x32 used to fence each partial and
+// take a ticket per block, and a batch of lattices wrote zero partials for the
+// other lattices' right-hand sides; without: the 28-right-hand-side solve 664 ->
+// 639 ms, the uneven lattices 51.8 -> 44.0 ms.
+template <class E>
+__global__ void __launch_bounds__(512) epi_final_kernel(E e, const double* partials, int64_t nslots,
+                                                        const int* skip, int skip_stride, const BatchTile* bt, int nbt,
+                                                        int64_t btiles) {
+  const int rhs = blockIdx.x;
+  pdl_launch_dependents();
+  int64_t lo = 0, hi = nslots;
+  for (int l = 0; l < nbt; ++l)
+    if (rhs >= bt[l].rhs0 && rhs < bt[l].rhs0 + bt[l].nrhs) {
+      lo = bt[l].tile0;
+      hi = l + 1 < nbt ? bt[l + 1].tile0 : btiles;
+    }
+  pdl_wait();
+  if (skip[(int64_t)rhs * skip_stride]) return;  // finished before this hop: stale partials
+  constexpr int U = 8;
+  const double* p = partials + rhs * nslots;
+  double s = 0.0;
+  for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += U * 512) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = i0 + u * 512 < hi ? __ldcg(p + i0 + u * 512) : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u];
+  }
+  __shared__ double sm[16];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t[1] = {0.0};
+    for (int k = 0; k < 16; ++k) t[0] += sm[k];
+    e.finalize(rhs, t);
+  }
+}
+
 // CG on one right-hand side: the same iteration with the scalars made by the
 // kernels that need them (block_total) instead of at the end of the reducing
 // launch.  (p, A p) is left as partials by the alpha hop; the next hop, which
@@ -397,12 +444,7 @@ struct CgHopUpdate {
 // left by the update hop and added up by every block of Cg1P, whose first block
 // writes the state.
 template <int P>
-struct Cg1HopAlpha : CgHopAlpha<P> {
-  static constexpr bool PARTIALS = true;
-};
-template <int P>
 struct Cg1HopUpdate : CgHopUpdate<P> {
-  static constexpr bool PARTIALS = true;
   // x, r and p come from DRAM where the vectors and links exceed L2: requested
   // before the stencil
   __device__ void prefetch(int rhs, int64_t h) const {

@@ -30,9 +30,11 @@ struct has_warp_finalize<F, std::void_t<decltype(&F::finalize_warp)>> : std::tru
 // in every block) while its own loads are in flight.  The fence, the ticket,
 // the last block's second pass and its scalar update, 4 to 6 us at the end of a
 // launch during which nothing else runs, become about 1 us beside other work.
-// For few partials (a launch of one right-hand side).
+// For few partials (a launch of one right-hand side); with many right-hand
+// sides a kernel of one block each does it (epi_final_kernel), which still
+// spares every block of the producer its fence and ticket.
 template <int NRED>
-__device__ __forceinline__ void block_partials(const double (&acc)[NRED], double* partials, unsigned slot) {
+__device__ __forceinline__ void block_partials(const double (&acc)[NRED], double* partials, int64_t slot) {
   __shared__ double sm[NRED][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nw = (blockDim.x + 31) >> 5;
@@ -47,7 +49,7 @@ __device__ __forceinline__ void block_partials(const double (&acc)[NRED], double
   if (threadIdx.x < NRED) {
     double v = 0.0;
     for (int w = 0; w < nw; ++w) v += sm[threadIdx.x][w];
-    partials[(int64_t)slot * NRED + threadIdx.x] = v;
+    partials[slot * NRED + threadIdx.x] = v;
   }
 }
 // sum of n partials, the same in every thread of the block (at most 8 warps)

@@ -716,6 +716,14 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   s.nrhs = w.nrhs;
   HopArgs a;
   if (clg_status st = make_hop_args(ctx, w.U, s, a)) return st;
+  // after the hop: its partials to E::finalize, one block per right-hand side
+  auto finish = [&](cudaError_t err, int64_t nslots) -> clg_status {
+    if (err == cudaSuccess)
+      err = launch_pdl(ctx, epi_final_kernel<E>, dim3((unsigned)w.nrhs), dim3(512), 0, e,
+                       (const double*)ctx->red_partials, nslots, skip, ks, a.btile, a.btile ? a.nbtile : 0, a.btiles);
+    if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("fused hop: ") + cudaGetErrorString(err));
+    return CLG_SUCCESS;
+  };
   if (a.seg && a.btile) {  // a batch of lattices: the tile form
     if (clg_status st = ensure_reduction(ctx, red2_doubles(a.btiles, w.nrhs, 1, E::NRED))) return st;
     cudaError_t berr;
@@ -723,8 +731,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
       berr = dag ? launch_hop_batch_tile_epi<P, 18, true>(ctx, a, e) : launch_hop_batch_tile_epi<P, 18, false>(ctx, a, e);
     else
       berr = dag ? launch_hop_batch_tile_epi<P, 12, true>(ctx, a, e) : launch_hop_batch_tile_epi<P, 12, false>(ctx, a, e);
-    if (berr != cudaSuccess) return ctx->fail(cuda_status(berr), std::string("fused hop: ") + cudaGetErrorString(berr));
-    return CLG_SUCCESS;
+    return finish(berr, a.btiles);
   }
   // the block size tuned for the plain hop of the same kind (the hops on the
   // odd checkerboard of each iteration run first and are tuned)
@@ -738,8 +745,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
       const int64_t nslots = (w.Vh + ((tcfg >> 16) >= 24 ? MMA_TS : TILE16) - 1) / ((tcfg >> 16) >= 24 ? MMA_TS : TILE16);
       if (clg_status st = ensure_reduction(ctx, red2_doubles(nslots, w.nrhs, 1, E::NRED))) return st;
       const cudaError_t terr = dag ? launch_hop_tile_epi<true>(ctx, a, e, tcfg) : launch_hop_tile_epi<false>(ctx, a, e, tcfg);
-      if (terr != cudaSuccess) return ctx->fail(cuda_status(terr), std::string("fused hop: ") + cudaGetErrorString(terr));
-      return CLG_SUCCESS;
+      return finish(terr, nslots);
     }
     const int pcfg = tuned_hop_pair_config(ctx, w.U, plain, -1);
     const bool pair = ctx->hop_pair_mode == 1 || (ctx->hop_pair_mode == 2 && pcfg >= 0);
@@ -750,8 +756,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
       if (clg_status st = ensure_reduction(ctx, red2_doubles((w.Vh + pbs - 1) / pbs, w.nrhs, (w.nrhs + 1) / 2, E::NRED)))
         return st;
       const cudaError_t perr = dag ? launch_hop_pair_epi<true>(ctx, a, e, cfg) : launch_hop_pair_epi<false>(ctx, a, e, cfg);
-      if (perr != cudaSuccess) return ctx->fail(cuda_status(perr), std::string("fused hop: ") + cudaGetErrorString(perr));
-      return CLG_SUCCESS;
+      return finish(perr, (w.Vh + pbs - 1) / pbs);
     }
   }
   if constexpr (P != P16) {
@@ -767,8 +772,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
         terr = dag ? launch_hop_tileN_epi<P, 12, true>(ctx, a, e, pc) : launch_hop_tileN_epi<P, 12, false>(ctx, a, e, pc);
       else
         terr = dag ? launch_hop_tileN_epi<P, 18, true>(ctx, a, e, pc) : launch_hop_tileN_epi<P, 18, false>(ctx, a, e, pc);
-      if (terr != cudaSuccess) return ctx->fail(cuda_status(terr), std::string("fused hop: ") + cudaGetErrorString(terr));
-      return CLG_SUCCESS;
+      return finish(terr, nslots);
     }
   }
   if (clg_status st = ensure_reduction(ctx, red2_doubles((w.Vh + bs - 1) / bs, w.nrhs, w.nrhs, E::NRED))) return st;
@@ -783,8 +787,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   } else {
     err = dag ? launch_hop_epi<P, 12, true>(ctx, a, e, bs) : launch_hop_epi<P, 12, false>(ctx, a, e, bs);
   }
-  if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("fused hop: ") + cudaGetErrorString(err));
-  return CLG_SUCCESS;
+  return finish(err, (w.Vh + bs - 1) / bs);
 }
 
 // The same for one right-hand side with the block sums of e left in part
@@ -1002,7 +1005,7 @@ clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, 
   KState* st = w.st;
   clg_status s;
   if ((s = schur_hop_odd(w, d1, p, to, skip, ks))) return s;
-  if ((s = schur_hop_epi1<P>(w, d1, to, p, te, Cg1HopAlpha<P>{{st, 0}}, skip, ks, pap, &npap))) return s;
+  if ((s = schur_hop_epi1<P>(w, d1, to, p, te, CgHopAlpha<P>{st, 0}, skip, ks, pap, &npap))) return s;
   const AlphaFin fin{pap, npap, odd ? &st->rr1 : &st->rr, &st->alpha, &st->status, &st->done, &st->skip, ST_BREAKDOWN};
   if ((s = schur_hop_odd(w, !d1, te, to, skip, ks, &fin))) return s;
   const Cg1HopUpdate<P> up{{dfield(x), dfield(r), dfield(p), st}};
