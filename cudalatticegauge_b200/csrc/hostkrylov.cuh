@@ -38,21 +38,20 @@ __device__ __forceinline__ void ld3(const char* v, int64_t off, int64_t kstride,
   }
 }
 
-// out[i] = s_i v_i^+ w for n vectors, MDG of them per block (right-hand side g
-// of the launch = vectors MDG g ..): w is read once per MDG vectors, and the
-// blocks of all vectors run side by side.  One block over all vectors reduced
-// 32 numbers per block on 32 blocks of 8^3x16 (19 us a launch whatever n).
-// With hcol the results are also added to (first: stored in) a Hessenberg
-// column.
+// out[i] = v_i^+ w for n vectors, MDG of them per block (right-hand side g of
+// the launch = vectors MDG g ..): w is read once per MDG vectors, and the blocks
+// of all vectors run side by side.  One block over all vectors reduced 32
+// numbers per block on 32 blocks of 8^3x16 (19 us a launch whatever n).
+// PART: left as block partials [group][slot][2 MDG] for the linear combination
+// that follows (LinCombF::dots).
+template <bool PART>
 struct MultiDotF {
+  static constexpr bool PARTIALS = PART;
   const char* w;
   VecTab v;
   int64_t blk, kstride;
   int n;
-  const double* scale;  // device, nullable: s_i
   double2* out;
-  double2* hcol;        // nullable
-  int first;
   __device__ bool active(int) const { return true; }
   __device__ void operator()(int g, int p, int64_t h, double* acc) const {
     const int64_t off = p * blk + h * 16;
@@ -78,19 +77,20 @@ struct MultiDotF {
     for (int i = 0; i < MDG; ++i) {
       const int k = MDG * g + i;
       if (k >= n) break;
-      const double sc = scale ? scale[k] : 1.0;
-      const double2 d = make_double2(sc * s[2 * i], sc * s[2 * i + 1]);
-      out[k] = d;
-      if (hcol) hcol[k] = first ? d : make_double2(hcol[k].x + d.x, hcol[k].y + d.y);
+      out[k] = make_double2(s[2 * i], s[2 * i + 1]);
     }
   }
 };
 
 // out_r = beta in_r + sum_i c_(r,i) s_i v_i for the `rhs` outputs r of the
-// launch (ostride bytes apart); the coefficients are kernel arguments (c) or
-// device-resident (dc, times sign).  NRED = 1 also reduces |out|^2: its root
-// goes to hn and its reciprocal (0 for a zero vector) to inv.
-template <int NRED>
+// launch (ostride bytes apart); the coefficients are kernel arguments (HOST),
+// device-resident (DEV: dc), or minus s_i times the inner products whose
+// partials precede the launch (DOTS: every block adds them up, the first one
+// also adds them to the Hessenberg column hcol, or stores them: first).  NRED = 1
+// also reduces |out|^2: its root goes to hn and its reciprocal (0 for a zero
+// vector) to inv.
+enum : int { LC_HOST = 0, LC_DEV = 1, LC_DOTS = 2 };
+template <int NRED, int SRC>
 struct LinCombF {
   char* out;
   const char* in;
@@ -99,15 +99,70 @@ struct LinCombF {
   double2 c[MAXV];
   const double2* dc;
   const double* scale;
-  double sign;
+  const double* dots;
+  int nslots;
+  double2* hcol;
+  int first;
   double2 beta;
   int64_t blk, kstride;
   int n;
   double2* hn;
   double* inv;
+  __device__ static double2* coef() {
+    __shared__ double2 s_c[MAXV];
+    return s_c;
+  }
   __device__ bool active(int) const { return true; }
+  // the coefficients to shared memory (all blocks the same)
+  __device__ bool prologue(int r, bool first_block) const {
+    double2* sc = coef();
+    if constexpr (SRC == LC_DOTS) {
+      // warp w adds up the products w, w + 8, ...: all their partials' loads in flight together
+      constexpr int U = (MAXV + 7) / 8;
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      double2 t[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] = make_double2(0.0, 0.0);
+      for (int b = lane; b < nslots; b += 32) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = warp + 8 * u;
+          if (i < n) {
+            const double2 d = __ldcg(reinterpret_cast<const double2*>(
+                                         dots + ((int64_t)(i / MDG) * nslots + b) * (2 * MDG)) + i % MDG);
+            t[u].x += d.x;
+            t[u].y += d.y;
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = warp + 8 * u;
+        if (i >= n) break;  // uniform over the warp
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          t[u].x += __shfl_xor_sync(0xffffffffu, t[u].x, o);
+          t[u].y += __shfl_xor_sync(0xffffffffu, t[u].y, o);
+        }
+        if (lane == 0) {
+          const double si = scale[i];
+          const double2 d = make_double2(si * t[u].x, si * t[u].y);
+          sc[i] = make_double2(-si * d.x, -si * d.y);
+          if (first_block) hcol[i] = first ? d : make_double2(hcol[i].x + d.x, hcol[i].y + d.y);
+        }
+      }
+    } else if (threadIdx.x < n) {
+      const int i = threadIdx.x;
+      const double2 ci = SRC == LC_DEV ? dc[r * n + i] : c[i];
+      const double si = SRC == LC_DEV ? scale[i] : 1.0;
+      sc[i] = make_double2(si * ci.x, si * ci.y);
+    }
+    __syncthreads();
+    return true;
+  }
   __device__ void operator()(int r, int p, int64_t h, double* acc) const {
     const int64_t off = p * blk + h * 16;
+    const double2* sc = coef();
     cpx<double> o[3];
     if (beta.x != 0.0 || beta.y != 0.0) {
       ld3(in + r * ostride, off, kstride, o);
@@ -122,9 +177,7 @@ struct LinCombF {
     for (int i = 0; i < n; ++i) {
       cpx<double> a[3];
       ld3(v.v[i], off, kstride, a);
-      double2 ci = dc ? dc[r * n + i] : c[i];
-      const double sc = (scale ? scale[i] : 1.0) * sign;
-      const cpx<double> cc = mk<double>(sc * ci.x, sc * ci.y);
+      const cpx<double> cc = mk<double>(sc[i].x, sc[i].y);
 #pragma unroll
       for (int k = 0; k < 3; ++k) o[k] = o[k] + cc * a[k];
     }
@@ -199,29 +252,25 @@ struct HostKrylov {
   // blocks of 3 components of a vector (VecTab)
   int blocks() const { return W.proto.nparity * (nc / 3); }
   int64_t block_bytes() const { return 3 * Vh * 16; }
-  // device out[i] = s_i v_i^+ w (and the Hessenberg column), no host read
-  clg_status dots_dev(const FieldRef& w, const FieldRef* const* vs, int n, double2* out, const double* scale = nullptr,
-                      double2* hcol = nullptr, bool first = true) {
-    if (n > MAXV) return ctx->fail(CLG_ERR_UNSUPPORTED, "too many vectors in one multi-dot");
-    MultiDotF f;
+  template <bool PART>
+  MultiDotF<PART> multidot(const FieldRef& w, const FieldRef* const* vs, int n) const {
+    MultiDotF<PART> f;
     f.w = w.data;
-    for (int i = 0; i < n; ++i) f.v.v[i] = vs[i]->data;
-    for (int i = n; i < MAXV; ++i) f.v.v[i] = nullptr;
+    for (int i = 0; i < MAXV; ++i) f.v.v[i] = i < n ? vs[i]->data : nullptr;
     f.blk = block_bytes();
     f.kstride = Vh * 16;
     f.n = n;
-    f.scale = scale;
-    f.out = out;
-    f.hcol = hcol;
-    f.first = first;
-    return launch_sites<2 * MDG>(ctx, f, 0, blocks(), Vh, (n + MDG - 1) / MDG);
+    f.out = reinterpret_cast<double2*>(W.dev_out);
+    return f;
   }
   // out[i] = v_i^+ w for the n vectors vs (n arbitrary), read to the host
   clg_status dots(const FieldRef& w, const std::vector<const FieldRef*>& vs, std::vector<Z>& out) {
     out.assign(vs.size(), Z(0.0, 0.0));
     for (size_t i0 = 0; i0 < vs.size(); i0 += MAXV) {
       const int n = (int)std::min<size_t>(MAXV, vs.size() - i0);
-      if (clg_status st = dots_dev(w, vs.data() + i0, n, reinterpret_cast<double2*>(W.dev_out))) return st;
+      if (clg_status st = launch_sites<2 * MDG>(ctx, multidot<false>(w, vs.data() + i0, n), 0, blocks(), Vh,
+                                               (n + MDG - 1) / MDG))
+        return st;
       double h[2 * MAXV];
       cudaError_t e = cudaMemcpyAsync(h, W.dev_out, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, ctx->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -235,9 +284,10 @@ struct HostKrylov {
     if (dots(a, {&a}, d)) return -1.0;
     return std::sqrt(std::max(d[0].real(), 0.0));
   }
-  template <int NRED>
-  LinCombF<NRED> combination(const FieldRef& out, const FieldRef& in, Z beta, const FieldRef* const* vs, int n) const {
-    LinCombF<NRED> f;
+  template <int NRED, int SRC>
+  LinCombF<NRED, SRC> combination(const FieldRef& out, const FieldRef& in, Z beta, const FieldRef* const* vs,
+                                  int n) const {
+    LinCombF<NRED, SRC> f;
     f.out = out.data;
     f.in = in.data;
     f.ostride = out.rstride;
@@ -247,7 +297,10 @@ struct HostKrylov {
     }
     f.dc = nullptr;
     f.scale = nullptr;
-    f.sign = 1.0;
+    f.dots = nullptr;
+    f.nslots = 0;
+    f.hcol = nullptr;
+    f.first = 0;
     f.beta = make_double2(beta.real(), beta.imag());
     f.blk = block_bytes();
     f.kstride = Vh * 16;
@@ -259,7 +312,7 @@ struct HostKrylov {
   // out = beta out + sum_i c_i v_i
   clg_status lincomb(const FieldRef& out, Z beta, const std::vector<const FieldRef*>& vs, const std::vector<Z>& c) {
     if (vs.size() > (size_t)MAXV) return ctx->fail(CLG_ERR_UNSUPPORTED, "too many vectors in one linear combination");
-    LinCombF<0> f = combination<0>(out, out, beta, vs.data(), (int)vs.size());
+    auto f = combination<0, LC_HOST>(out, out, beta, vs.data(), (int)vs.size());
     for (size_t i = 0; i < vs.size(); ++i) f.c[i] = make_double2(c[i].real(), c[i].imag());
     return launch_sites<0>(ctx, f, 0, blocks(), Vh, 1);
   }
@@ -283,10 +336,8 @@ struct HostKrylov {
 };
 
 // Device state of an Arnoldi cycle (arnoldi_step): the basis vectors are
-// V'_i = v_i / s_i, not normalised, so that no pass over a vector only scales
-// it; d holds the inner products of the current pass.
+// V'_i = v_i / s_i, not normalised, so that no pass over a vector only scales it.
 struct ArnoldiState {
-  double2 d[MAXV];
   double2 H[(MAXV - 1) * MAXV];  // column j at H + j MAXV, h_(j+1,j) included
   double2 norm;                  // of the vector arnoldi_start normalised
   double s[MAXV];
@@ -294,7 +345,7 @@ struct ArnoldiState {
 
 // V'_0 = scale-free copy of src, s_0 = 1 / |src|, norm = |src|
 inline clg_status arnoldi_start(HostKrylov& K, ArnoldiState* st, const FieldRef& v0, const FieldRef& src) {
-  auto f = K.combination<1>(v0, src, Z(1.0, 0.0), nullptr, 0);
+  auto f = K.combination<1, LC_HOST>(v0, src, Z(1.0, 0.0), nullptr, 0);
   f.hn = &st->norm;
   f.inv = &st->s[0];
   return launch_sites<1>(K.ctx, f, 0, K.blocks(), K.Vh, 1);
@@ -302,26 +353,38 @@ inline clg_status arnoldi_start(HostKrylov& K, ArnoldiState* st, const FieldRef&
 // Column j of the Arnoldi relation: w = A v_j orthogonalised against
 // v_0 .. v_j by classical Gram-Schmidt twice, left in next = V'_(j+1), all of
 // it on the device: 4 launches after the operator, no host read.  The host
-// reads the whole H at the end of a cycle.
-inline clg_status arnoldi_step(HostKrylov& K, ArnoldiState* st, const FieldRef* const* V, int j, const FieldRef& w,
-                               const FieldRef& next) {
+// reads the whole H at the end of a cycle.  part: the inner products' partials
+// (arnoldi_partials doubles); the combination adds them up itself, since a last
+// block that waits for all others costs 4 us a pass and a sum that every block
+// repeats 1 us (one cycle of 30 with 6 shifts on 8^3x16: 3.35 -> 2.64 ms).
+inline int64_t arnoldi_partials(const HostKrylov& K) {
+  int64_t most = 0;
+  for (int g = 1; g <= (MAXV + MDG - 1) / MDG; ++g)
+    most = std::max(most, site_blocks<2 * MDG>(K.ctx, K.blocks(), K.Vh, g) * g * 2 * MDG);
+  return most;
+}
+inline clg_status arnoldi_step(HostKrylov& K, ArnoldiState* st, double* part, const FieldRef* const* V, int j,
+                               const FieldRef& w, const FieldRef& next) {
   if (clg_status e = K.apply(w, *V[j], &st->s[j])) return e;
-  double2* hcol = st->H + (size_t)j * MAXV;
+  const int n = j + 1, groups = (n + MDG - 1) / MDG;
+  auto fill = [&](auto& f, int first) {
+    f.scale = st->s;
+    f.dots = part;
+    f.nslots = (int)site_blocks<2 * MDG>(K.ctx, K.blocks(), K.Vh, groups);
+    f.hcol = st->H + (size_t)j * MAXV;
+    f.first = first;
+  };
   for (int pass = 0; pass < 2; ++pass) {
-    if (clg_status e = K.dots_dev(w, V, j + 1, st->d, st->s, hcol, pass == 0)) return e;
+    if (clg_status e = launch_sites<2 * MDG>(K.ctx, K.multidot<true>(w, V, n), 0, K.blocks(), K.Vh, groups, part)) return e;
     if (pass == 0) {
-      auto f = K.combination<0>(w, w, Z(1.0, 0.0), V, j + 1);
-      f.dc = st->d;
-      f.scale = st->s;
-      f.sign = -1.0;
+      auto f = K.combination<0, LC_DOTS>(w, w, Z(1.0, 0.0), V, n);
+      fill(f, 1);
       if (clg_status e = launch_sites<0>(K.ctx, f, 0, K.blocks(), K.Vh, 1)) return e;
     } else {
-      auto f = K.combination<1>(next, w, Z(1.0, 0.0), V, j + 1);
-      f.dc = st->d;
-      f.scale = st->s;
-      f.sign = -1.0;
-      f.hn = hcol + j + 1;
-      f.inv = &st->s[j + 1];
+      auto f = K.combination<1, LC_DOTS>(next, w, Z(1.0, 0.0), V, n);
+      fill(f, 0);
+      f.hn = f.hcol + n;
+      f.inv = &st->s[n];
       if (clg_status e = launch_sites<1>(K.ctx, f, 0, K.blocks(), K.Vh, 1)) return e;
     }
   }

@@ -48,8 +48,12 @@ struct FomWork : hk::HostVecs {
   FieldRef X;               // the nshift solutions (FP64, right-hand sides = shifts)
   hk::ArnoldiState* st = nullptr;  // device
   double2* coef = nullptr;         // device, [shift][vector]
-  clg_status arnoldi_buffers(int ns) {
+  double* part = nullptr;          // device, the inner products' partials
+  clg_status arnoldi_buffers(int ns, const hk::HostKrylov& K) {
     void* p = nullptr;
+    if (clg_status e = dalloc(ctx, &p, sizeof(double) * hk::arnoldi_partials(K))) return e;
+    allocs.push_back(p);
+    part = static_cast<double*>(p);
     if (clg_status e = dalloc(ctx, &p, sizeof(hk::ArnoldiState))) return e;
     allocs.push_back(p);
     st = static_cast<hk::ArnoldiState*>(p);
@@ -109,14 +113,14 @@ clg_status add_basis(hk::HostKrylov& K, FomWork& W, const FieldRef& X, int ns, c
     return K.ctx->fail(CLG_ERR_CUDA, "multi-shift: coefficient upload");
   std::vector<const FieldRef*> vs;
   for (int i = 0; i < dim; ++i) vs.push_back(&W.V[i]);
-  auto f = K.combination<0>(X, X, Z(1.0, 0.0), vs.data(), dim);
+  auto f = K.combination<0, hk::LC_DEV>(X, X, Z(1.0, 0.0), vs.data(), dim);
   f.dc = W.coef;
   f.scale = W.st->s;
   return launch_sites<0>(K.ctx, f, 0, K.blocks(), K.Vh, ns);
 }
 // all of X = 0
 clg_status zero_solutions(hk::HostKrylov& K, const FieldRef& X, int ns) {
-  return launch_sites<0>(K.ctx, K.combination<0>(X, X, Z(0.0, 0.0), nullptr, 0), 0, K.blocks(), K.Vh, ns);
+  return launch_sites<0>(K.ctx, K.combination<0, hk::LC_HOST>(X, X, Z(0.0, 0.0), nullptr, 0), 0, K.blocks(), K.Vh, ns);
 }
 
 template <int NC>
@@ -168,7 +172,7 @@ clg_status fom_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cache
     if (!st) st = nw->vec(nw->R);
     if (!st) st = nw->full_vec(nw->tmp);
     if (!st) st = nw->out_buffer();
-    if (!st) st = nw->arnoldi_buffers(ns);
+    if (!st) st = nw->arnoldi_buffers(ns, hk::HostKrylov{ctx, *nw, U, kind, op, nc, param, Vh});
     if (!st) {  // the solutions: one allocation, shift k is right-hand side k
       void* p = nullptr;
       st = dalloc(ctx, &p, (size_t)nw->proto.rstride * ns);
@@ -201,7 +205,7 @@ clg_status fom_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cache
     std::vector<const FieldRef*> V;
     for (int j = 0; j < m; ++j) V.push_back(&W->V[j]);
     for (int j = 0; j < m; ++j)
-      if ((st = hk::arnoldi_step(K, W->st, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
+      if ((st = hk::arnoldi_step(K, W->st, W->part, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
     if ((st = read_arnoldi(ctx, *W, h))) return st;
     if (cyc == 0) {
       bnorm = h.norm.x;
@@ -279,7 +283,7 @@ clg_status gmres_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cac
     if (!st) st = nw->vec(nw->R);
     if (!st) st = nw->full_vec(nw->tmp);
     if (!st) st = nw->out_buffer();
-    if (!st) st = nw->arnoldi_buffers(ns);
+    if (!st) st = nw->arnoldi_buffers(ns, hk::HostKrylov{ctx, *nw, U, kind, op, nc, param, Vh});
     if (!st) {
       void* p = nullptr;
       st = dalloc(ctx, &p, (size_t)nw->proto.rstride * ns);
@@ -318,7 +322,7 @@ clg_status gmres_ms_run(clg_context_s* ctx, std::unique_ptr<SolveCacheBase>& cac
     std::vector<const FieldRef*> V;
     for (int j = 0; j < m; ++j) V.push_back(&W->V[j]);
     for (int j = 0; j < m; ++j)
-      if ((st = hk::arnoldi_step(K, W->st, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
+      if ((st = hk::arnoldi_step(K, W->st, W->part, V.data(), j, W->w, j + 1 < m ? W->V[j + 1] : W->R))) return st;
     if ((st = read_arnoldi(ctx, *W, h))) return st;
     const double beta = h.norm.x;
     if (!(beta >= 0)) return ctx->fail(CLG_ERR_BREAKDOWN, "multi-shift GMRES: NaN in the residual");
