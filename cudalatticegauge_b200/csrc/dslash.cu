@@ -37,7 +37,8 @@ std::vector<int> tile_warps(int nrhs);
 // less than SPLIT_MAX threads, and taken untimed where it gives each of the
 // 592 schedulers less than a warp: there a launch is a few dependent round
 // trips to memory, which a loop of independent launches (the autotuner's, bound
-// by the launches themselves) cannot see.  GMRES on 8^4: SPLIT_US
+// by the launches themselves) cannot see.  The FP32 hop inside GMRES on 8^4:
+// 6.4 -> 5.6 us
 constexpr int64_t SPLIT_MAX = (int64_t)1 << 18;
 bool split_worth(const Geom& g, int nrhs) { return g.Vh * nrhs <= SPLIT_MAX; }
 // the untimed choice, recorded like a timed one (the fused epilogues follow it)
@@ -339,13 +340,18 @@ cudaError_t launch_staggered(clg_context_s* ctx, const HopArgs& a, int nrhs, con
 // ------------------------------------------------------------------ both checkerboards in one launch
 // Launch configurations of a full-lattice D: block | variant << 16 with variant
 // 0 = two checkerboard hops, FULL_ONE + (1: register cap) + (2: chunks of
-// y-rows), FULL_SPLIT = four threads per site
-constexpr int FULL_ONE = 32, FULL_SPLIT = 36;
+// y-rows), FULL_SPLIT = four threads per site, FULL_MID (+ 2) = FP64 Wilson with
+// blocks of 64 threads at 168 registers (12 warps per SM; uncapped it takes 254,
+// 8 warps, and at 128 registers it spills): 32^3x16 107 -> 105 us, 48^3x24 in
+// chunks 542 -> 522
+constexpr int FULL_ONE = 32, FULL_SPLIT = 36, FULL_MID = 40;
 
-std::vector<int> full_candidates(const HopArgs& a, int rows, bool split) {
+std::vector<int> full_candidates(const HopArgs& a, int rows, bool split, bool mid) {
   std::vector<int> c = {0};
   for (int v = 0; v < (rows ? 4 : 2); ++v)
     for (int bs : {64, 128, 256}) c.push_back(bs | ((FULL_ONE + v) << 16));
+  if (mid)
+    for (int v = 0; v < (rows ? 4 : 2); v += 2) c.push_back(64 | ((FULL_MID + v) << 16));
   if (split && split_worth(a.g, 2 * a.nrhs)) c.push_back((4 * SPLIT_SITES) | (FULL_SPLIT << 16));
   return c;
 }
@@ -361,6 +367,11 @@ cudaError_t launch_wilson_full(clg_context_s* ctx, const HopArgs& a0, bool dagge
     return dagger ? launch_pdl(ctx, wilson_split_kernel<P, RECON, true, true>, grid, dim3(bs), 0, a)
                   : launch_pdl(ctx, wilson_split_kernel<P, RECON, false, true>, grid, dim3(bs), 0, a);
   a.tile_rows = (v & 2) ? rows : 0;
+  if constexpr (P == P64) {
+    if (v >= FULL_MID)
+      return dagger ? launch_pdl(ctx, wilson_full_kernel<P, RECON, true, 64, 6>, grid, dim3(bs), 0, a)
+                    : launch_pdl(ctx, wilson_full_kernel<P, RECON, false, 64, 6>, grid, dim3(bs), 0, a);
+  }
   if (v & 1)
     return dagger ? launch_pdl(ctx, wilson_full_kernel<P, RECON, true, 256, CAP>, grid, dim3(bs), 0, a)
                   : launch_pdl(ctx, wilson_full_kernel<P, RECON, false, 256, CAP>, grid, dim3(bs), 0, a);
@@ -663,7 +674,7 @@ clg_status hop_full(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec& s) 
                   : launch_staggered_full<P32, 18>(ctx, a, rows, cfg);
   };
   if (wilson) take_split(ctx, hop_key(U, s) + "_full", a.g, 2 * s.nrhs, FULL_SPLIT);
-  const cudaError_t e = go(tune_block(ctx, hop_key(U, s) + "_full", idempotent(a), go, full_candidates(a, rows, wilson),
+  const cudaError_t e = go(tune_block(ctx, hop_key(U, s) + "_full", idempotent(a), go, full_candidates(a, rows, wilson, wilson && s.prec == CLG_PREC_DOUBLE),
                                       128 | ((FULL_ONE + 1) << 16)));
   if (hst) return hst;
   if (e != cudaSuccess) return ctx->fail(cuda_status(e), std::string("full hop launch: ") + cudaGetErrorString(e));
