@@ -262,19 +262,26 @@ __global__ void __launch_bounds__(128) wilson_force_kernel(ForceArgs a) {
 //   F_mu(x) -= Ta(s_+ eta_mu(x) [U_mu(x) A + B U_mu(x)^+]),
 //   A = sum_i a_i phi_i(x+mu) phi_id(x)^+,   B = sum_i a_i phi_i(x) phi_id(x+mu)^+
 // (the reference's two contractions per pole, makeSU3ContractV; Ta is linear, so
-// the poles are summed before the one Ta and the one F update).  Same block
-// shape as the Wilson force: 32 sites x 4 direction warps, parity-interleaved
-// blocks.  The poles are streamed through a ring of cp.async stages (the
-// copies of pole i+1 are in flight while pole i is contracted); U and F are
-// staged once.  Compulsory DRAM traffic per site: 2 x 48 B per pole, U 576 B,
-// F 1152 B.  With 12 poles on 32^3 x 16 the kernel runs at 0.57 of the copy
-// bandwidth: each pole is a short contraction between two block barriers, and
-// the per-pole copy issue and barrier waits, not DRAM, set the pace.
+// the poles are summed before the one Ta and the one F update).  Since
+// Ta(M^+) = -Ta(M), B U^+ counts as -U B^+:
+//   F -= Ta(s_+ eta U W),  W = A - B^+ = sum_i a_i [phi_i(x+mu) phi_id(x)^+ - phi_id(x+mu) phi_i(x)^+],
+// one accumulated matrix instead of two.  Same block shape as the Wilson force:
+// 32 sites x 4 direction warps, parity-interleaved blocks.  The poles, then U,
+// then F are streamed through a ring of cp.async slots: the copies of two items
+// are in flight while one is contracted, and one barrier per pole both publishes
+// its slot and releases the one before.  Compulsory DRAM traffic per site: 2 x 48 B
+// per pole, U 576 B, F 1152 B.  Three slots leave 55 KB a block, 4 blocks (16
+// warps) per SM; with two accumulators, U and F staged beside a ring of two and
+// two barriers per pole 3 blocks fit.  12 poles on 32^3 x 16: 395 -> 321 us (3.8
+// -> 4.7 TB/s), 4 poles 207 -> 176, 24^4 with 12 poles 258 -> 206.  Beside DRAM
+// (227 us) the shared-memory pipe is what is left: each operand is written there
+// and read back, some 200 us by count; the FP64 pipe needs 117 us.
 constexpr int KS_FORCE_MAX = 64;
 constexpr int KS_HERE = 2 * 3 * TILE;     // phi_i(x), phi_id(x)        [field][k][site]
 constexpr int KS_NBR = 4 * 2 * 3 * TILE;  // phi_i(x+mu), phi_id(x+mu)  [mu][field][k][site]
 constexpr int KS_STAGE = KS_HERE + KS_NBR;
-constexpr size_t ks_force_smem(int nstage) { return sizeof(double2) * (nstage * KS_STAGE + 2 * E_LINK); }
+constexpr int KS_SLOT = E_LINK > KS_STAGE ? E_LINK : KS_STAGE;  // a pole, U or F
+constexpr size_t ks_force_smem(int nstage) { return sizeof(double2) * nstage * KS_SLOT; }
 
 struct KsForceArgs {
   Geom g;
@@ -287,29 +294,22 @@ struct KsForceArgs {
   double a[KS_FORCE_MAX];
 };
 
-
-// m[r][q] += w * l[r] conj(r[q])
-__device__ __forceinline__ void outer3_acc(C m[9], double w, const double2* l, const double2* r) {
-  C lv[3], rv[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double2 x = l[k * TILE], y = r[k * TILE];
-    lv[k] = mk<double>(w * x.x, w * x.y);
-    rv[k] = mk<double>(y.x, y.y);
-  }
+// m[r][q] += l[r] conj(r[q])
+__device__ __forceinline__ void outer3_acc(C m[9], const C l[3], const C r[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       C t = m[3 * i + j];
-      t.x = fma(lv[i].x, rv[j].x, fma(lv[i].y, rv[j].y, t.x));
-      t.y = fma(lv[i].y, rv[j].x, fma(-lv[i].x, rv[j].y, t.y));
+      t.x = fma(l[i].x, r[j].x, fma(l[i].y, r[j].y, t.x));
+      t.y = fma(l[i].y, r[j].x, fma(-l[i].x, r[j].y, t.y));
       m[3 * i + j] = t;
     }
 }
 
 template <int NSTAGE>
-__global__ void __launch_bounds__(128) ks_force_kernel(KsForceArgs a) {
+__global__ void __launch_bounds__(128, 4) ks_force_kernel(KsForceArgs a) {
+  static_assert(NSTAGE >= 3, "U and F take two slots while the last pole is read");
   extern __shared__ double2 sm[];
   const int p = (int)(blockIdx.x & 1);
   const int lane = (int)(threadIdx.x & 31), mu = (int)(threadIdx.x >> 5);
@@ -332,89 +332,87 @@ __global__ void __launch_bounds__(128) ks_force_kernel(KsForceArgs a) {
   // of one colour component; per pole only the field base changes
   const int64_t off_here = (int64_t)p * a.blk + h * 16, off_nbr = (int64_t)(1 - p) * a.blk + hn * 16;
   const int64_t kstride = Vh * 16;
-  double2* s_link = sm + NSTAGE * KS_STAGE;
+  const int64_t off_link = (int64_t)mu * 9 * Vh + h;
+  double2* s_u = sm + (a.n % NSTAGE) * KS_SLOT + mu * 9 * TILE + lane;
+  double2* s_f = sm + ((a.n + 1) % NSTAGE) * KS_SLOT + mu * 9 * TILE + lane;
 
-  // copies of pole i into ring stage i % NSTAGE
-  auto issue = [&](int i) {
-    if (!live || i >= a.n) return;
-    double2* st = sm + (i % NSTAGE) * KS_STAGE;
-    const char* fi = a.phi_i[i];
-    const char* fd = a.phi_id[i];
-    // here: the 6 components f (phi_i k = f for f < 3, phi_id k = f - 3) over
-    // the 4 warps, warp mu taking f = mu and f = mu + 4
-    cp_async16(st + mu * TILE + lane,
-               reinterpret_cast<const double2*>((mu == 3 ? fd : fi) + off_here + (mu == 3 ? 0 : mu) * kstride));
-    if (mu < 2)
-      cp_async16(st + (mu + 4) * TILE + lane, reinterpret_cast<const double2*>(fd + off_here + (mu + 1) * kstride));
-    double2* dn = st + KS_HERE + mu * 6 * TILE + lane;
+  auto links = [&](double2* d, const double2* b) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      cp_async16(dn + k * TILE, reinterpret_cast<const double2*>(fi + off_nbr + k * kstride));
-      cp_async16(dn + (3 + k) * TILE, reinterpret_cast<const double2*>(fd + off_nbr + k * kstride));
+    for (int k = 0; k < 9; ++k) cp_async16(d + k * TILE, b + off_link + k * Vh);
+  };
+  // copies of item i into ring slot i % NSTAGE: the poles, then U, then F
+  auto issue = [&](int i) {
+    if (!live) return;
+    if (i < a.n) {
+      double2* st = sm + (i % NSTAGE) * KS_SLOT;
+      const char* fi = a.phi_i[i];
+      const char* fd = a.phi_id[i];
+      // here: the 6 components f (phi_i k = f for f < 3, phi_id k = f - 3) over
+      // the 4 warps, warp mu taking f = mu and f = mu + 4
+      cp_async16(st + mu * TILE + lane,
+                 reinterpret_cast<const double2*>((mu == 3 ? fd : fi) + off_here + (mu == 3 ? 0 : mu) * kstride));
+      if (mu < 2)
+        cp_async16(st + (mu + 4) * TILE + lane, reinterpret_cast<const double2*>(fd + off_here + (mu + 1) * kstride));
+      double2* dn = st + KS_HERE + mu * 6 * TILE + lane;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        cp_async16(dn + k * TILE, reinterpret_cast<const double2*>(fi + off_nbr + k * kstride));
+        cp_async16(dn + (3 + k) * TILE, reinterpret_cast<const double2*>(fd + off_nbr + k * kstride));
+      }
+    } else if (i == a.n) {
+      links(s_u, p ? a.U[1] : a.U[0]);
+    } else if (i == a.n + 1) {
+      links(s_f, p ? a.F[1] : a.F[0]);
     }
   };
-
-  if (live) {
-    const double2* ub = (p ? a.U[1] : a.U[0]) + (int64_t)mu * 9 * Vh + h;
-    const double2* fb = (p ? a.F[1] : a.F[0]) + (int64_t)mu * 9 * Vh + h;
-    double2* su = s_link + mu * 9 * TILE + lane;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      cp_async16(su + k * TILE, ub + k * Vh);
-      cp_async16(su + E_LINK + k * TILE, fb + k * Vh);
-    }
-  }
-  // prologue: poles 0 .. NSTAGE-2 in flight, one commit group each (group 0
-  // also holds the links); every thread commits every group, empty or not
+  // every thread commits every group, empty or not
 #pragma unroll
   for (int j = 0; j < NSTAGE - 1; ++j) {
     issue(j);
     cp_async_commit();
   }
 
-  C A[9], B[9];
+  C W[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) A[k] = B[k] = mk<double>(0, 0);
+  for (int k = 0; k < 9; ++k) W[k] = mk<double>(0, 0);
   for (int i = 0; i < a.n; ++i) {
-    issue(i + NSTAGE - 1);  // into the stage pole i - 1 used (released by the barrier below)
+    cp_async_wait<NSTAGE - 2>();  // this thread's copies of pole i landed
+    __syncthreads();              // everyone's did, and slot i - 1 is free
+    issue(i + NSTAGE - 1);
     cp_async_commit();
-    cp_async_wait<NSTAGE - 1>();  // this thread's copies of pole i (and the links) landed
-    __syncthreads();              // everyone's did
-    if (live) {
-      const double2* st = sm + (i % NSTAGE) * KS_STAGE;
-      const double2* nb = st + KS_HERE + mu * 6 * TILE + lane;
-      const double w = a.a[i];
-      outer3_acc(A, w, nb, st + 3 * TILE + lane);  // phi_i(x+mu) phi_id(x)^+
-      outer3_acc(B, w, st + lane, nb + 3 * TILE);  // phi_i(x) phi_id(x+mu)^+
+    C fn[3], dn[3], v[3];  // a phi_i(x+mu), -a phi_id(x+mu), the other factor
+    const double2* st = sm + (i % NSTAGE) * KS_SLOT;
+    const double2* nb = st + KS_HERE + mu * 6 * TILE + lane;
+    const double w = a.a[i];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double2 x = nb[k * TILE], y = nb[(3 + k) * TILE];
+      fn[k] = mk<double>(w * x.x, w * x.y);
+      dn[k] = mk<double>(-w * y.x, -w * y.y);
     }
-    __syncthreads();  // pole i's stage is free for pole i + NSTAGE
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = mk<double>(st[(3 + k) * TILE + lane].x, st[(3 + k) * TILE + lane].y);
+    outer3_acc(W, fn, v);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = mk<double>(st[k * TILE + lane].x, st[k * TILE + lane].y);
+    outer3_acc(W, dn, v);
   }
-  cp_async_wait<0>();
-  __syncthreads();
+  cp_async_wait<0>();  // U and F: read by the threads that copied them
   if (!live) return;
 
-  // m = U A + B U^+
-  const double2* su = s_link + mu * 9 * TILE + lane;
-  C u[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const double2 d = su[k * TILE];
-    u[k] = mk<double>(d.x, d.y);
-  }
+  // m = U W
   C m[9];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < 3; ++i) {
+    C u[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      C t = u[3 * i] * A[j] + u[3 * i + 1] * A[3 + j] + u[3 * i + 2] * A[6 + j];
-      // (B U^+)_ij = sum_k B_ik conj(U_jk)
-      t = t + B[3 * i] * cj(u[3 * j]) + B[3 * i + 1] * cj(u[3 * j + 1]) + B[3 * i + 2] * cj(u[3 * j + 2]);
-      m[3 * i + j] = t;
-    }
+    for (int k = 0; k < 3; ++k) u[k] = mk<double>(s_u[(3 * i + k) * TILE].x, s_u[(3 * i + k) * TILE].y);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) m[3 * i + j] = u[0] * W[j] + u[1] * W[3 + j] + u[2] * W[6 + j];
+  }
   // F -= s_+ eta Ta(m)
   const double w = -sg * eta;
-  double2* fb = (p ? a.F[1] : a.F[0]) + (int64_t)mu * 9 * Vh + h;
-  const double2* s_f = su + E_LINK;
+  double2* fb = (p ? a.F[1] : a.F[0]) + off_link;
   const double tr = (m[0].y + m[4].y + m[8].y) * (1.0 / 3.0);
 #pragma unroll
   for (int i = 0; i < 3; ++i)
@@ -555,13 +553,12 @@ clg_status clg_ks_force(clg_gauge F, clg_gauge U, int n, const clg_field* phi_i,
   }
   k.blk = phi_i[0]->blk;
   const int64_t nblk = (k.g.Vh + TILE - 1) / TILE;
-  // ring depth 2: 3, 4 and 5 stages (fewer blocks per SM) measured no faster,
-  // nor did two or three poles per stage (409 / 606 us against 403); a
-  // barrier-free form with the poles loaded through registers by four
-  // direction threads per site in one warp ran at 782 us; U and F read from
-  // global memory at the end instead of staged (4 blocks per SM at 128
-  // registers, against 3 with staging) ran at 551 us against 399
-  constexpr int nstage = 2;
+  // ring of 3 slots, 4 blocks per SM; measured on 32^3x16 with 12 poles against
+  // its 321 us: 2 slots with 5 or 6 blocks per SM (spills) 345 / 351, 4 slots with
+  // 3 blocks 325, the neighbours' components through registers instead of shared
+  // memory 405 - 422, a barrier-free form with four direction threads per site in
+  // one warp 782
+  constexpr int nstage = 3;
   void (*kern)(KsForceArgs) = ks_force_kernel<nstage>;
   const size_t smem = ks_force_smem(nstage);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
