@@ -1161,9 +1161,8 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_pair_kernel(HopArgs a) 
 // The pair form of wilson_hop_epi_kernel: E::site runs once per right-hand
 // side of the pair; the block reduces both right-hand sides' values.
 template <bool DAGGER, int MAXT, int MINB, class E>
-__global__ void __launch_bounds__(MAXT, MINB) wilson_hop_pair_epi_kernel(HopArgs a, E e, double* partials,
-                                                                         double* gpart, unsigned* counter,
-                                                                         unsigned group) {
+__global__ void __launch_bounds__(MAXT, MINB) wilson_hop_pair_epi_kernel(HopArgs a, E e, double* partials) {
+  static_assert(partials_only<E>::value, "the sums are left to the next kernel");
   const unsigned npairs = (unsigned)(a.nrhs + 1) / 2u;
   int rhs0, rhs1;
   bool has1;
@@ -1189,23 +1188,16 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_pair_epi_kernel(HopArgs
       e.site(rhs1, h, acc1, red + E::NRED);
     }
   }
-  if constexpr (partials_only<E>::value) {
-    double r0[E::NRED], r1[E::NRED];
+  double r0[E::NRED], r1[E::NRED];
 #pragma unroll
-    for (int k = 0; k < E::NRED; ++k) {
-      r0[k] = red[k];
-      r1[k] = red[E::NRED + k];
-    }
-    const int64_t nslots = gridDim.x / npairs;
-    if (run0) block_partials<E::NRED>(r0, partials, rhs0 * nslots + slot);
-    __syncthreads();
-    if (run1) block_partials<E::NRED>(r1, partials, rhs1 * nslots + slot);
-  } else {
-    const int rr[2] = {rhs0, rhs1};
-    const bool cc[2] = {run0, run1}, hh[2] = {true, has1};
-    grid_reduce_finalize2<E::NRED, 2>(red, e, rr, cc, hh, (unsigned)(rhs0 / 2), npairs, slot, gridDim.x / npairs,
-                                      a.nrhs, group, partials, gpart, counter);
+  for (int k = 0; k < E::NRED; ++k) {
+    r0[k] = red[k];
+    r1[k] = red[E::NRED + k];
   }
+  const int64_t nslots = gridDim.x / npairs;
+  if (run0) block_partials<E::NRED>(r0, partials, rhs0 * nslots + slot);
+  __syncthreads();
+  if (run1) block_partials<E::NRED>(r1, partials, rhs1 * nslots + slot);
 }
 
 // ---------------------------------------------------------------- FP16, a tile of sites for every right-hand side
@@ -1398,14 +1390,13 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_tile16_kernel(HopArgs a
 }
 
 // The epilogue form of tile16_body: per right-hand side the warp reduces its
-// 32 sites and writes the tile's partial (slot = block); in a batch the block
-// writes zero partials for the other lattices' right-hand sides.  The blocks
-// then reduce in two levels (tile_reduce_finalize).
+// 32 sites and writes the tile's partial (slot = block; in a batch this lattice's
+// slots only) for the next kernel.
 template <bool DAGGER, class E>
 __device__ __forceinline__ void tile16_epi_body(const HopArgs& a, const E& e, Tile16& t, const Geom& g,
                                                 const void* Uh, const void* Ut, int64_t h0, int r0, int r1,
-                                                double* partials, double* gpart, unsigned* counter,
-                                                unsigned group) {
+                                                double* partials) {
+  static_assert(partials_only<E>::value, "the sums are left to the next kernel");
   pdl_launch_dependents();
   tile16_neighbours(g, a.out_parity, h0, t);
   pdl_wait();
@@ -1434,35 +1425,20 @@ __device__ __forceinline__ void tile16_epi_body(const HopArgs& a, const E& e, Ti
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + k] = v;
     }
-    if constexpr (!partials_only<E>::value)
-      if (lane == 0) __threadfence();
   }
-  if constexpr (partials_only<E>::value) return;  // left to the next kernel (a batch: this lattice's slots only)
-  if (r0 > 0 || r1 < a.nrhs) {
-    for (int q = threadIdx.x; q < a.nrhs * E::NRED; q += blockDim.x) {
-      const int rhs = q / E::NRED;
-      if (rhs < r0 || rhs >= r1) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + q % E::NRED] = 0.0;
-    }
-    __threadfence();
-  }
-  tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
 }
 
 template <bool DAGGER, int MINB, class E, bool BATCH = false, int MAXT = 256>
-__global__ void __launch_bounds__(MAXT, MINB) wilson_hop_tile16_epi_kernel(HopArgs a, E e, double* partials,
-                                                                          double* gpart, unsigned* counter,
-                                                                          unsigned group) {
+__global__ void __launch_bounds__(MAXT, MINB) wilson_hop_tile16_epi_kernel(HopArgs a, E e, double* partials) {
   __shared__ Tile16 t;
   if constexpr (BATCH) {
     const BatchTile bt = batch_tile(a);
     const HopSeg& sg = a.seg[bt.seg];
     const Geom g = sg.g;
     tile16_epi_body<DAGGER>(a, e, t, g, sg.u[2][a.out_parity], sg.u[2][1 - a.out_parity],
-                            ((int64_t)blockIdx.x - bt.tile0) * TILE16, bt.rhs0, bt.rhs0 + bt.nrhs, partials,
-                            gpart, counter, group);
+                            ((int64_t)blockIdx.x - bt.tile0) * TILE16, bt.rhs0, bt.rhs0 + bt.nrhs, partials);
   } else {
-    tile16_epi_body<DAGGER>(a, e, t, a.g, a.U_here, a.U_there, tile16_index(a) * TILE16, 0, a.nrhs, partials,
-                            gpart, counter, group);
+    tile16_epi_body<DAGGER>(a, e, t, a.g, a.U_here, a.U_there, tile16_index(a) * TILE16, 0, a.nrhs, partials);
   }
 }
 
@@ -1894,11 +1870,10 @@ __global__ void __launch_bounds__(256, MINB) wilson_hop_mma16_kernel(HopArgs a) 
 }
 
 // The epilogue form: per right-hand side the 8 sites of the tile reduce in
-// groups of 8 lanes and write the tile's partial; tile_reduce_finalize after.
+// groups of 8 lanes and write the tile's partial for the next kernel.
 template <bool DAGGER, int MINB, class E>
-__global__ void __launch_bounds__(256, MINB) wilson_hop_mma16_epi_kernel(HopArgs a, E e, double* partials,
-                                                                         double* gpart, unsigned* counter,
-                                                                         unsigned group) {
+__global__ void __launch_bounds__(256, MINB) wilson_hop_mma16_epi_kernel(HopArgs a, E e, double* partials) {
+  static_assert(partials_only<E>::value, "the sums are left to the next kernel");
   extern __shared__ __align__(16) unsigned char mma_smem[];
   Mma16Smem& t = *reinterpret_cast<Mma16Smem*>(mma_smem);
   const int64_t h0 = tile_index<MMA_TS>(a) * MMA_TS;
@@ -1941,13 +1916,9 @@ __global__ void __launch_bounds__(256, MINB) wilson_hop_mma16_epi_kernel(HopArgs
         for (int o = MMA_TS / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, MMA_TS);
         if (live && i == 0) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + k] = v;
       }
-      if constexpr (!partials_only<E>::value)
-        if (live && i == 0) __threadfence();
     }
     __syncthreads();
   }
-  if constexpr (!partials_only<E>::value)
-    tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
 }
 
 // The FP16 staggered direction on half2 words: o = U chi (UDAG: U^+ chi) with

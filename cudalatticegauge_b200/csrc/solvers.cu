@@ -585,16 +585,11 @@ cudaError_t launch_hop_pair_epi(clg_context_s* ctx, const HopArgs& a, const E& e
   const unsigned npairs = (unsigned)(a.nrhs + 1) / 2u;
   const int64_t nslots = (a.g.Vh + bs - 1) / bs;
   dim3 grid((unsigned)(nslots * npairs));
-  const unsigned group = red_group(nslots, npairs);
-  double* gpart = ctx->red_partials + nslots * a.nrhs * E::NRED;
   if ((cfg >> 16) == 1)
-    return launch_pdl(ctx, wilson_hop_pair_epi_kernel<DAG, 256, 2, E>, grid, dim3(bs), 0, a, e, ctx->red_partials,
-                      gpart, ctx->red_counter, group);
-  return launch_pdl(ctx, wilson_hop_pair_epi_kernel<DAG, 256, 1, E>, grid, dim3(bs), 0, a, e, ctx->red_partials,
-                    gpart, ctx->red_counter, group);
+    return launch_pdl(ctx, wilson_hop_pair_epi_kernel<DAG, 256, 2, E>, grid, dim3(bs), 0, a, e, ctx->red_partials);
+  return launch_pdl(ctx, wilson_hop_pair_epi_kernel<DAG, 256, 1, E>, grid, dim3(bs), 0, a, e, ctx->red_partials);
 }
 
-// the tile form (wilson_hop_tile16_epi_kernel): config as in launch_wilson_tile
 // the tensor-core form (wilson_hop_mma16_epi_kernel): config as in launch_wilson_mma
 template <bool DAG, class E>
 cudaError_t launch_hop_mma_epi(clg_context_s* ctx, const HopArgs& a0, const E& e, int cfg) {
@@ -602,18 +597,16 @@ cudaError_t launch_hop_mma_epi(clg_context_s* ctx, const HopArgs& a0, const E& e
   const int v = (cfg >> 16) - 24;
   a.tile_rows = (v & 2) ? tile_rows(a.g, a.nrhs, MMA_TS) : 0;
   const int64_t nslots = (a.g.Vh + MMA_TS - 1) / MMA_TS;
-  const unsigned group = red_group(nslots, 1);
-  double* gpart = ctx->red_partials + nslots * a.nrhs * E::NRED;
   const size_t smem = sizeof(Mma16Smem);
-  auto go = [&](void (*kernel)(HopArgs, E, double*, double*, unsigned*, unsigned)) {
+  auto go = [&](void (*kernel)(HopArgs, E, double*)) {
     if (const cudaError_t err = opt_in_smem((const void*)kernel, smem)) return err;
-    return launch_pdl(ctx, kernel, dim3((unsigned)nslots), dim3(256), smem, a, e, ctx->red_partials, gpart,
-                      ctx->red_counter, group);
+    return launch_pdl(ctx, kernel, dim3((unsigned)nslots), dim3(256), smem, a, e, ctx->red_partials);
   };
   if (v & 1) return go(wilson_hop_mma16_epi_kernel<DAG, 2, E>);
   return go(wilson_hop_mma16_epi_kernel<DAG, 1, E>);
 }
 
+// the tile form (wilson_hop_tile16_epi_kernel): config as in launch_wilson_tile
 template <bool DAG, class E>
 cudaError_t launch_hop_tile_epi(clg_context_s* ctx, const HopArgs& a0, const E& e, int cfg) {
   if ((cfg >> 16) >= 24) return launch_hop_mma_epi<DAG>(ctx, a0, e, cfg);
@@ -621,8 +614,6 @@ cudaError_t launch_hop_tile_epi(clg_context_s* ctx, const HopArgs& a0, const E& 
   HopArgs a = a0;
   a.tile_rows = ((cfg >> 16) & 2) ? tile_rows(a.g, a.nrhs) : 0;
   const int64_t nslots = (a.g.Vh + TILE16 - 1) / TILE16;
-  const unsigned group = red_group(nslots, 1);
-  double* gpart = ctx->red_partials + nslots * a.nrhs * E::NRED;
   int v = cfg >> 16;
   // an epilogue that loads vectors of its own (the CG update: x, r, p) spills
   // under the 72- and 64-register caps: it keeps the 80-register form
@@ -631,15 +622,15 @@ cudaError_t launch_hop_tile_epi(clg_context_s* ctx, const HopArgs& a0, const E& 
     if (bs > 128) return cudaErrorInvalidConfiguration;
     if (v & 1)
       return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, 8, E, false, 128>, dim3((unsigned)nslots), dim3(bs),
-                        0, a, e, ctx->red_partials, gpart, ctx->red_counter, group);
+                        0, a, e, ctx->red_partials);
     return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, 7, E, false, 128>, dim3((unsigned)nslots), dim3(bs), 0,
-                      a, e, ctx->red_partials, gpart, ctx->red_counter, group);
+                      a, e, ctx->red_partials);
   }
   if (v & 1)
     return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, 3, E>, dim3((unsigned)nslots), dim3(bs), 0, a, e,
-                      ctx->red_partials, gpart, ctx->red_counter, group);
+                      ctx->red_partials);
   return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, 2, E>, dim3((unsigned)nslots), dim3(bs), 0, a, e,
-                    ctx->red_partials, gpart, ctx->red_counter, group);
+                    ctx->red_partials);
 }
 
 // the FP64 / FP32 tile form (wilson_hop_tileN_epi_kernel): config as in launch_wilson_tileN
@@ -665,15 +656,13 @@ template <int P, int RECON, bool DAG, class E>
 cudaError_t launch_hop_batch_tile_epi(clg_context_s* ctx, const HopArgs& a, const E& e) {
   constexpr int CAP = P == P64 ? 2 : 3;
   const int64_t nslots = a.btiles;
-  const unsigned group = red_group(nslots, 1);
-  double* gpart = ctx->red_partials + nslots * a.nrhs * E::NRED;
   const dim3 grid((unsigned)nslots), block(128);
   if constexpr (P == P16)
-    return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, CAP, E, true>, grid, block, 0, a, e, ctx->red_partials,
-                      gpart, ctx->red_counter, group);
+    return launch_pdl(ctx, wilson_hop_tile16_epi_kernel<DAG, CAP, E, true>, grid, block, 0, a, e, ctx->red_partials);
   else
     return launch_pdl(ctx, wilson_hop_tileN_epi_kernel<P, RECON, DAG, CAP, E, true>, grid, block, 0, a, e,
-                      ctx->red_partials, gpart, ctx->red_counter, group);
+                      ctx->red_partials, ctx->red_partials + nslots * a.nrhs * E::NRED, ctx->red_counter,
+                      red_group(nslots, 1));
 }
 
 template <int P, int RECON, bool DAG, class E>
