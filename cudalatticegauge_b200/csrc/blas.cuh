@@ -151,15 +151,15 @@ inline FieldRef pieces_view(const FieldRef& f, int pieces) {
   return v;
 }
 template <class Fn>
-clg_status with_pieces(int prec, int nc, Fn&& fn) {
+clg_status with_pieces(int prec, int nc, bool whole, Fn&& fn) {
   using I0 = std::integral_constant<int, 0>;
   using I1 = std::integral_constant<int, 1>;
   using I2 = std::integral_constant<int, 2>;
   using N12 = std::integral_constant<int, 12>;
   using N4 = std::integral_constant<int, 4>;
   using N3 = std::integral_constant<int, 3>;
-  if (prec == 0) return fn(I0{}, N3{});
-  if (prec == 1) return nc == 12 ? fn(I1{}, N4{}) : fn(I1{}, N3{});
+  if (prec == 0) return nc == 12 && whole ? fn(I0{}, N12{}) : fn(I0{}, N3{});
+  if (prec == 1) return nc != 12 ? fn(I1{}, N3{}) : whole ? fn(I1{}, N12{}) : fn(I1{}, N4{});
   return nc == 12 ? fn(I2{}, N12{}) : fn(I2{}, N3{});
 }
 

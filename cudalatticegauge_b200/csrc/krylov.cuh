@@ -615,10 +615,40 @@ struct GmDots {
   __device__ void finalize(int, const double*) const {}
 };
 
+// The same for lattices that fill the chip (gm_wide): one block over all J + 1
+// columns, so w is read once and every column's loads are in flight together; the
+// last block stores the Hessenberg column.  FP32-inner GMRES(12) on 32^3x16:
+// 12.9 ms, with the groups of GmDots and sums in GmOrtho's blocks 15.9.
+template <int P, int NC, int J>
+struct GmDotsJ {
+  VList V;
+  DField w;
+  KState* st;
+  __device__ bool active(int q) const { return !st[q].skip; }
+  __device__ void operator()(int rhs, int par, int64_t h, double* acc) const {
+    using AT = typename AccT<P>::T;
+    cpx<AT> vw[NC];
+    ldv<P, NC, AT>(w, rhs, par, h, vw);
+#pragma unroll
+    for (int i = 0; i <= J; ++i) {
+      cpx<AT> vi[NC];
+      ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
+      acc_dot<NC, AT>(vi, vw, acc + 2 * i);
+    }
+  }
+  __device__ void finalize(int q, const double* s) const {
+    KState& k = st[q];
+    if (k.skip) return;
+    k.iters += 1;
+    for (int i = 0; i <= J; ++i) k.H[i * GM_MAXK + J] = make_double2(k.s[i] * s[2 * i], k.s[i] * s[2 * i + 1]);
+  }
+};
+
 // V'_{j+1} = w - sum_i h_ij v_i ; h_{j+1,j} = |V'_{j+1}| ; Givens rotation of column j
 // (h_ij = s_i <V'_i, w> from GmDots's partials, summed by every block; block 0
-// of the right-hand side stores the column for the last block's rotation)
-template <int P, int NC>
+// of the right-hand side stores the column for the last block's rotation; WIDE:
+// GmDotsJ stored it)
+template <int P, int NC, bool WIDE>
 struct GmOrtho {
   VList V;
   DField w;
@@ -637,6 +667,15 @@ struct GmOrtho {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int groups = j / GM_DG + 1;
     double* c = reinterpret_cast<double*>(coef());
+    if constexpr (WIDE) {
+      if (threadIdx.x <= j) {
+        const double2 hv = k.H[threadIdx.x * GM_MAXK + j];
+        const double si = k.s[threadIdx.x];
+        coef()[threadIdx.x] = make_double2(hv.x * si, hv.y * si);
+      }
+      __syncthreads();
+      return run;
+    }
     for (int v = warp; v < 2 * (j + 1); v += nw) {
       const int i = v >> 1;
       const double* p = dots + (int64_t)(q * groups + i / GM_DG) * nslots * (2 * GM_DG) + 2 * (i % GM_DG) + (v & 1);
@@ -660,8 +699,10 @@ struct GmOrtho {
     const double2* c = coef();
     cpx<AT> vw[NC];
     ldv<P, NC, AT>(w, rhs, par, h, vw);
-#pragma unroll 4
-    for (int i = 0; i <= j; ++i) {
+    constexpr int U = WIDE ? GM_MAXK : 4;
+#pragma unroll U
+    for (int i = 0; i < GM_MAXK; ++i) {
+      if (i > j) break;
       cpx<AT> vi[NC];
       ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);
       const cpx<AT> cc = mk<AT>((AT)c[i].x, (AT)c[i].y);
