@@ -594,6 +594,22 @@ bool fused_cg(const Work& w, int op) {
          (op == CLG_OP_MEE_MEEDAG || op == OP_MEEDAG_MEE);
 }
 
+// Whether the hops of one right-hand side take a tile form: pinned, or read from
+// a tune file that a context pinned to one wrote.  Those have no block for
+// AlphaFin and run the iteration with its own sums (cg_fused_iteration).
+bool tile_form(const Work& w) {
+  if (w.ctx->hop_config >= 0 && (w.ctx->hop_config >> 16) >= 16) return true;
+  HopSpec s{};
+  s.kind = w.kind;
+  s.prec = w.P;
+  s.nrhs = w.nrhs;
+  for (const bool dag : {false, true}) {
+    s.dagger = dag;
+    if ((tuned_hop_config(w.ctx, w.U, s, 0) >> 16) >= 16) return true;
+  }
+  return false;
+}
+
 // the paired FP16 form: config = block | variant << 16 as in launch_wilson_pair
 template <bool DAG, class E>
 cudaError_t launch_hop_pair_epi(clg_context_s* ctx, const HopArgs& a, const E& e, int cfg) {
@@ -1071,8 +1087,7 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       clg_status e = launch_sites<1>(ctx, init, fp, np, Vh, nrhs);
       if (e) return e;
       const bool fused = NV == 12 && fused_cg(w, op);
-      // (a pinned tile form has no block for AlphaFin)
-      const bool one = fused && nrhs == 1 && !w.U->seg && (ctx->hop_config < 0 || (ctx->hop_config >> 16) < 16);
+      const bool one = fused && nrhs == 1 && !w.U->seg && !tile_form(w);
       if (one && (e = w.partials(2 * ((Vh + SPLIT_SITES - 1) / SPLIT_SITES)))) return e;
       int it = 0;  // a chunk is an even number of iterations: replays keep the parity
       auto body = [&]() -> clg_status {

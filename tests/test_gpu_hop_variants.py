@@ -388,6 +388,45 @@ def test_tune_file_round_trip(clg, tmp_path):
             os.environ["CLG_TUNE_FILE"] = old
 
 
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_tune_file_of_a_pinned_context(clg, oracle, tmp_path, prec):
+    """A context pinned to a tile form saves it under the one-source key too; a
+    later unpinned context that reads the file solves with the form it names."""
+    import os
+
+    dims, path = (8, 8, 8, 8), str(tmp_path / "tune.txt")
+    old = {k: os.environ.get(k) for k in ("CLG_TUNE_FILE", "CLG_HOP_CONFIG")}
+    os.environ["CLG_TUNE_FILE"] = path
+    try:
+        for pin in ("17:128", None):
+            os.environ.pop("CLG_HOP_CONFIG", None)
+            if pin:
+                os.environ["CLG_HOP_CONFIG"] = pin
+            c = clg.Context(0)
+            lat = clg.Lattice(c, dims)
+            U = clg.CFieldGaugeSU3(lat)
+            U.InitialField(clg.GAUGE_EXPH, 0xC1A60001, 1, 0.25)
+            b, x = (clg.CFieldFermionWilsonSquareSU3(lat, KAPPA) for _ in range(2))
+            b.InitialField(clg.SOURCE_GAUSS, 960, 2)
+            for op, name in ((clg.EFO_F_D, "WILSON_D"), (clg.EFO_F_Ddagger, "WILSON_DDAG")):
+                S = clg.CSLASolverCG(c, inner_precision=prec, tol_true_rel=1e-10)
+                assert S.Solve(x, b, U, op)[0]["status"] == 0
+                S.close()
+                ref = oracle.Operator(name, dims, U.CopyDataOut(), KAPPA)
+                assert ref.true_residual(b.to_numpy(), x.to_numpy()) <= 1e-10
+            saved = c.tuned()
+            for o in (b, x, U, lat):
+                o.close()
+            c.close()
+            if pin:
+                assert any(v[1] == 17 and "_n1_" in k for k, v in saved.items())
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
+
+
 @pytest.mark.parametrize("cfg", ["16:128", "19:256"])
 @pytest.mark.parametrize("prec", [0, 1])
 def test_staggered_tile(clg, oracle, pinned, cfg, prec):
