@@ -28,6 +28,21 @@
 
 namespace clg {
 
+// The blocks of Cg1P grow with the lattice and so do the partials of |r|^2 that
+// each of them adds up: on 48^3x24, 5184 blocks of up to 20736 partials each
+// moved more through L2 than the vectors do through DRAM.  Above SUM_MOST
+// partials a launch of SUM_TO blocks (3 us) folds them first.  FP32-inner solves
+// before / folded: 48^3x24 117.3 / 114.1 ms, 32^4 45.6 / 45.0; at 1024 partials the
+// launch costs more than it saves (FP16 16^3x32 6.1 ms without it, 6.3 with).
+constexpr int SUM_MOST = 2048, SUM_TO = 32;
+__global__ void __launch_bounds__(256) fold_partials_kernel(const double* in, int n, double* out) {
+  pdl_launch_dependents();
+  const int lo = (int)((int64_t)n * blockIdx.x / SUM_TO), hi = (int)((int64_t)n * (blockIdx.x + 1) / SUM_TO);
+  pdl_wait();
+  const double s = block_total(in + lo, hi - lo);
+  if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
 // One warp per right-hand side, lane l = unknown l: its row of the triangle is
 // loaded at once, then column by column (y_i by lane i, the rest updated).
 // One thread per right-hand side took a global round trip per element (17 us).
@@ -305,7 +320,7 @@ struct Work : public SolveCacheBase {
   // Krylov operator temporaries (precision P)
   Owned kt_odd, kt_even, kt_full;
   // block partials left to the next kernel: CG on one right-hand side ((p, A p),
-  // then |r|^2), GMRES (a column's inner products)
+  // then |r|^2, then its fold), GMRES (a column's inner products)
   double* part = nullptr;
   int64_t npart = 0;
   clg_status partials(int64_t doubles) {
@@ -1021,7 +1036,7 @@ clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, 
   const FieldRef& to = w.kt_odd.ref;
   const FieldRef& te = w.kt_even.ref;
   const int64_t most = (w.Vh + SPLIT_SITES - 1) / SPLIT_SITES;
-  double *pap = w.part, *rrp = w.part + most;
+  double *pap = w.part, *rrp = w.part + most, *fold = w.part + 2 * most;
   int npap = 0, nrr = 0;
   KState* st = w.st;
   clg_status s;
@@ -1031,6 +1046,12 @@ clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, 
   if ((s = schur_hop_odd(w, !d1, te, to, skip, ks, &fin))) return s;
   const Cg1HopUpdate<P> up{{dfield(x), dfield(r), dfield(p), st}};
   if ((s = schur_hop_epi1<P>(w, !d1, to, te, te, up, skip, ks, rrp, &nrr))) return s;
+  if (nrr > SUM_MOST) {
+    const cudaError_t e = launch_pdl(w.ctx, fold_partials_kernel, dim3(SUM_TO), dim3(256), 0, (const double*)rrp, nrr, fold);
+    if (e != cudaSuccess) return w.ctx->fail(cuda_status(e), std::string("CG partials: ") + cudaGetErrorString(e));
+    rrp = fold;
+    nrr = SUM_TO;
+  }
   return launch_sites<0>(w.ctx, Cg1P<P, 12>{dfield(p), dfield(r), st, rrp, nrr, odd, op_weight(op)}, 0, 1, w.Vh, 1);
 }
 
@@ -1088,7 +1109,7 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       if (e) return e;
       const bool fused = NV == 12 && fused_cg(w, op);
       const bool one = fused && nrhs == 1 && !w.U->seg && !tile_form(w);
-      if (one && (e = w.partials(2 * ((Vh + SPLIT_SITES - 1) / SPLIT_SITES)))) return e;
+      if (one && (e = w.partials(2 * ((Vh + SPLIT_SITES - 1) / SPLIT_SITES) + SUM_TO))) return e;
       int it = 0;  // a chunk is an even number of iterations: replays keep the parity
       auto body = [&]() -> clg_status {
         clg_status e2;
