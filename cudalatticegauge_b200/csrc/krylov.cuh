@@ -444,17 +444,20 @@ __global__ void __launch_bounds__(512) epi_final_kernel(E e, const double* parti
 // left by the update hop and added up by every block of Cg1P, whose first block
 // writes the state.
 template <int P>
-struct Cg1HopUpdate : CgHopUpdate<P> {
-  // x, r and p come from DRAM where the vectors and links exceed L2: requested
-  // before the stencil
+struct Cg1HopUpdate : CgHopUpdate<P> {};
+// FP16: x, r and p, in DRAM where the vectors and links exceed L2, are requested
+// before the stencil, 9 words of 16 bytes a thread (the update hop of 32^3x16 34.5
+// -> 30.7 us).  The 18 and 36 words of FP32 and FP64 wait in front of the
+// stencil's own loads instead: FP32 on 48^3x24 228 us without them, 280 with.
+template <>
+struct Cg1HopUpdate<P16> : CgHopUpdate<P16> {
   __device__ void prefetch(int rhs, int64_t h) const {
-    constexpr int W = P == P64 ? 12 : (P == P32 ? 6 : 3);  // 16-byte words per site
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-      const int64_t off = (k * this->x.Vh + h) * 16;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->x.base(rhs, 0) + off));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->r.base(rhs, 0) + off));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(this->p.base(rhs, 0) + off));
+    for (int k = 0; k < 3; ++k) {
+      const int64_t off = (k * x.Vh + h) * 16;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(x.base(rhs, 0) + off));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(r.base(rhs, 0) + off));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.base(rhs, 0) + off));
     }
   }
 };
