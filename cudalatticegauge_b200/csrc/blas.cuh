@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256)
 // The same over a batch of lattices (clg_solve_lattices): right-hand side r
 // holds rhs_vh[r] sites per checkerboard, the rest of the padded range is
 // skipped (it stays zero).  A launch index is per_rhs consecutive ones per
-// right-hand side.
+// right-hand side (GmDots's groups).
 template <int NRED, class F>
 __global__ void __launch_bounds__(256)
     site_reduce_batch_kernel(F f, int64_t nsites, int first_parity, int64_t Vh, double* partials, unsigned* counter,
@@ -60,7 +60,12 @@ __global__ void __launch_bounds__(256)
   double acc[NRED > 0 ? NRED : 1];
 #pragma unroll
   for (int k = 0; k < (NRED > 0 ? NRED : 1); ++k) acc[k] = 0.0;
-  if (f.active(rhs)) {
+  bool work;
+  if constexpr (has_prologue<F>::value)
+    work = f.prologue(rhs, blockIdx.x == 0);
+  else
+    work = f.active(rhs);
+  if (work) {
     const int64_t vr = rhs_vh[rhs / per_rhs];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nsites; i += (int64_t)gridDim.x * blockDim.x) {
       const int pi = (int)(i / Vh);
@@ -68,8 +73,12 @@ __global__ void __launch_bounds__(256)
       if (h < vr) f(rhs, first_parity + pi, h, acc);
     }
   }
-  if constexpr (NRED > 0)
-    grid_reduce_finalize<NRED>(acc, f, rhs, blockIdx.x, gridDim.x, (int)gridDim.y, partials, counter);
+  if constexpr (NRED > 0) {
+    if constexpr (partials_only<F>::value)
+      block_partials<NRED>(acc, partials, blockIdx.x + rhs * gridDim.x);
+    else
+      grid_reduce_finalize<NRED>(acc, f, rhs, blockIdx.x, gridDim.x, (int)gridDim.y, partials, counter);
+  }
 }
 
 // The blocks per right-hand side of launch_sites
@@ -100,18 +109,17 @@ clg_status launch_sites(clg_context_s* ctx, const F& f, int first_parity, int np
     if (st) return st;
   }
   dim3 grid((unsigned)nb, (unsigned)nrhs);
-  cudaError_t e;
-  auto plain = [&]() {
-    return launch_pdl(ctx, site_reduce_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
-                      part ? part : ctx->red_partials, ctx->red_counter);
-  };
-  if constexpr (partials_only<F>::value || has_prologue<F>::value) {
-    e = plain();  // solvers of one lattice only
-  } else if (ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs % ctx->batch_nrhs == 0) {
-    e = launch_pdl(ctx, site_reduce_batch_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh,
-                   ctx->red_partials, ctx->red_counter, (const int64_t*)ctx->batch_vh, nrhs / ctx->batch_nrhs);
-  } else {
-    e = plain();
+  cudaError_t e = cudaSuccess;
+  double* const to = part ? part : ctx->red_partials;
+  bool batch = false;
+  if constexpr (!one_lattice<F>::value)
+    batch = ctx->batch_vh && Vh == ctx->batch_vh_stride && nrhs % ctx->batch_nrhs == 0;
+  if (!batch) {
+    e = launch_pdl(ctx, site_reduce_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh, to,
+                   ctx->red_counter);
+  } else if constexpr (!one_lattice<F>::value) {
+    e = launch_pdl(ctx, site_reduce_batch_kernel<NRED, F>, grid, dim3(bs), 0, f, nsites, first_parity, Vh, to,
+                   ctx->red_counter, (const int64_t*)ctx->batch_vh, nrhs / ctx->batch_nrhs);
   }
   if (e != cudaSuccess) return ctx->fail(cuda_status(e), std::string("site kernel: ") + cudaGetErrorString(e));
   return CLG_SUCCESS;

@@ -46,7 +46,7 @@ __device__ __forceinline__ void ld3(const char* v, int64_t off, int64_t kstride,
 // that follows (LinCombF::dots).
 template <bool PART>
 struct MultiDotF {
-  static constexpr bool PARTIALS = PART;
+  static constexpr bool PARTIALS = PART, ONE_LATTICE = true;
   const char* w;
   VecTab v;
   int64_t blk, kstride;
@@ -92,6 +92,7 @@ struct MultiDotF {
 enum : int { LC_HOST = 0, LC_DEV = 1, LC_DOTS = 2 };
 template <int NRED, int SRC>
 struct LinCombF {
+  static constexpr bool ONE_LATTICE = true;
   char* out;
   const char* in;
   int64_t ostride;

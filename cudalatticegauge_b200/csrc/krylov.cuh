@@ -466,6 +466,7 @@ struct Cg1HopUpdate<P16> : CgHopUpdate<P16> {
 // reads what the first one writes (a finished solve leaves both in rr).
 template <int P, int NC>
 struct Cg1P {
+  static constexpr bool ONE_LATTICE = true;
   DField p, r;
   KState* st;
   const double* rrp;  // nrr partials of |r_new|^2

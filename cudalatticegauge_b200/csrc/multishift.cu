@@ -80,7 +80,7 @@ namespace {
 // (p, q), left as block partials (CgmR's blocks make alpha of them)
 template <int P, int NC>
 struct CgmAlpha {
-  static constexpr bool PARTIALS = true;
+  static constexpr bool PARTIALS = true, ONE_LATTICE = true;
   DField p, q;
   CgmState* st;
   __device__ bool active(int) const { return !st->done; }
@@ -198,7 +198,7 @@ __device__ __forceinline__ double* cgm_scalar() {
 // |r|^2.  LAST: finalised here (the flush follows), else left to CgmP.
 template <int P, int NC, bool LAST>
 struct CgmR {
-  static constexpr bool PARTIALS = !LAST;
+  static constexpr bool PARTIALS = !LAST, ONE_LATTICE = true;
   DField ring, q;
   CgmState* st;
   int t, M;
@@ -252,6 +252,7 @@ struct CgmR {
 // beta = |r_{j+1}|^2 / |r_j|^2; p = r_{j+1} + beta p (ring slot t + 1), inside a block
 template <int P, int NC>
 struct CgmP {
+  static constexpr bool ONE_LATTICE = true;
   DField ring, p;
   CgmState* st;
   int t;

@@ -90,6 +90,12 @@ template <class F, class = void>
 struct has_prologue : std::false_type {};
 template <class F>
 struct has_prologue<F, std::void_t<decltype(&F::prologue)>> : std::true_type {};
+// One with ONE_LATTICE = true belongs to solvers that clg_solve_lattices does not
+// run, and has no batch form (launch_sites).
+template <class F, class = void>
+struct one_lattice : std::false_type {};
+template <class F>
+struct one_lattice<F, std::void_t<decltype(F::ONE_LATTICE)>> : std::bool_constant<F::ONE_LATTICE> {};
 
 // The last block's part: totals per right-hand side -> f.finalize.  Called by
 // every thread of that block (at most 256 threads, 8 warps).
