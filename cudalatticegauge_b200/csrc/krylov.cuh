@@ -668,33 +668,32 @@ struct GmOrtho {
   __device__ bool prologue(int q, bool first) const {
     KState& k = st[q];
     const bool run = !k.skip;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int groups = j / GM_DG + 1;
-    double* c = reinterpret_cast<double*>(coef());
     if constexpr (WIDE) {
       if (threadIdx.x <= j) {
         const double2 hv = k.H[threadIdx.x * GM_MAXK + j];
         const double si = k.s[threadIdx.x];
         coef()[threadIdx.x] = make_double2(hv.x * si, hv.y * si);
       }
-      __syncthreads();
-      return run;
-    }
-    for (int v = warp; v < 2 * (j + 1); v += nw) {
-      const int i = v >> 1;
-      const double* p = dots + (int64_t)(q * groups + i / GM_DG) * nslots * (2 * GM_DG) + 2 * (i % GM_DG) + (v & 1);
-      const double si = k.s[i];
-      double s = 0.0;
-      for (int b = lane; b < nslots; b += 32) s += __ldcg(p + (int64_t)b * (2 * GM_DG));
+    } else {
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+      const int groups = j / GM_DG + 1;
+      double* c = reinterpret_cast<double*>(coef());
+      for (int v = warp; v < 2 * (j + 1); v += nw) {
+        const int i = v >> 1;
+        const double* p = dots + (int64_t)(q * groups + i / GM_DG) * nslots * (2 * GM_DG) + 2 * (i % GM_DG) + (v & 1);
+        const double si = k.s[i];
+        double s = 0.0;
+        for (int b = lane; b < nslots; b += 32) s += __ldcg(p + (int64_t)b * (2 * GM_DG));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      const double h = si * s;
-      if (lane == 0) {
-        c[v] = h * si;
-        if (first && run) reinterpret_cast<double*>(&k.H[i * GM_MAXK + j])[v & 1] = h;
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const double h = si * s;
+        if (lane == 0) {
+          c[v] = h * si;
+          if (first && run) reinterpret_cast<double*>(&k.H[i * GM_MAXK + j])[v & 1] = h;
+        }
       }
+      if (first && run && threadIdx.x == 0) k.iters += 1;
     }
-    if (first && run && threadIdx.x == 0) k.iters += 1;
     __syncthreads();
     return run;
   }
@@ -716,50 +715,49 @@ struct GmOrtho {
     stv<P, NC, AT>(V.v[j + 1], rhs, par, h, vw);
     acc[0] += site_norm2<NC, AT>(vw);
   }
-  __device__ void finalize(int q, const double* s) const {
+  // Lane i holds row i of column j and rotation i.  The previous rotations
+  // (RotateH, CSolverGMRES.cpp:262-327, incrementally) run down the column as one
+  // chain that every lane follows through shuffles: one round trip to memory,
+  // and registers for one row.  One thread with the column and its rotations in
+  // registers (49 complex numbers) held the whole site kernel at 248 registers, one
+  // block per SM.
+  __device__ void finalize_warp(int q, const double* s, int lane) const {
+    static_assert(GM_MAXK <= 32, "one lane per row");
     KState& k = st[q];
-    if (k.skip) return;
+    if (k.skip) return;  // uniform
     const double hn = sqrt(s[0]);
+    const double2 zero = make_double2(0.0, 0.0);
     double2* H = k.H;
-    k.s[j + 1] = hn > 0.0 ? 1.0 / hn : 0.0;
-    // apply the previous rotations to column j (RotateH, CSolverGMRES.cpp:262-327,
-    // incrementally); the column and the rotations are loaded before the first
-    // is used (one thread walking them took a global round trip per rotation)
-    double2 hc[GM_MAXK + 1], ci[GM_MAXK], si[GM_MAXK];
-#pragma unroll
-    for (int i = 0; i < GM_MAXK; ++i) {
-      hc[i] = i <= j ? H[i * GM_MAXK + j] : make_double2(i == j + 1 ? hn : 0.0, 0.0);
-      ci[i] = i < j ? k.cs[i] : make_double2(0.0, 0.0);
-      si[i] = i < j ? k.sn[i] : make_double2(0.0, 0.0);
-    }
-    hc[GM_MAXK] = make_double2(j + 1 == GM_MAXK ? hn : 0.0, 0.0);
+    double2 row = lane <= j ? H[lane * GM_MAXK + j] : zero;
+    const double2 ci = lane < j ? k.cs[lane] : zero, si = lane < j ? k.sn[lane] : zero;
     const double2 gj = k.g[j];
     const double tol2 = k.tol2, rr0 = k.rr0;
-    double2 hjj = hc[0], hj1 = hc[1];
-#pragma unroll
-    for (int i = 0; i < GM_MAXK; ++i) {
-      if (i < j) {
-        const double2 a = cmul(cconj(ci[i]), hc[i]), b = cmul(cconj(si[i]), hc[i + 1]);
-        const double2 c = cmul(ci[i], hc[i + 1]), d = cmul(si[i], hc[i]);
-        H[i * GM_MAXK + j] = make_double2(a.x + b.x, a.y + b.y);
-        hc[i + 1] = make_double2(c.x - d.x, c.y - d.y);
-      }
-      if (i == j) {
-        hjj = hc[i];
-        hj1 = hc[i + 1];
-      }
+    auto from = [](double2 v, int i) {
+      return make_double2(__shfl_sync(0xffffffffu, v.x, i), __shfl_sync(0xffffffffu, v.y, i));
+    };
+    double2 hjj = from(row, 0);  // the chain: row i after the rotations above it
+#pragma unroll 4
+    for (int i = 0; i < j; ++i) {
+      const double2 next = from(row, i + 1), cs = from(ci, i), sn = from(si, i);
+      const double2 a = cmul(cconj(cs), hjj), b = cmul(cconj(sn), next);
+      const double2 c = cmul(cs, next), d = cmul(sn, hjj);
+      if (lane == i) row = make_double2(a.x + b.x, a.y + b.y);
+      hjj = make_double2(c.x - d.x, c.y - d.y);
     }
-    const double den = sqrt(hjj.x * hjj.x + hjj.y * hjj.y + hj1.x * hj1.x + hj1.y * hj1.y);
+    if (lane < j) H[lane * GM_MAXK + j] = row;
+    if (lane != 0) return;
+    k.s[j + 1] = hn > 0.0 ? 1.0 / hn : 0.0;
+    const double den = sqrt(hjj.x * hjj.x + hjj.y * hjj.y + hn * hn);
     if (!(den > 0.0) || bad(den)) {
       k.status = ST_BREAKDOWN;
       k.skip = 1;
       return;
     }
-    const double2 cs = make_double2(hjj.x / den, hjj.y / den), sn = make_double2(hj1.x / den, hj1.y / den);
+    const double2 cs = make_double2(hjj.x / den, hjj.y / den), sn = make_double2(hn / den, 0.0);
     k.cs[j] = cs;
     k.sn[j] = sn;
     H[j * GM_MAXK + j] = make_double2(den, 0.0);
-    H[(j + 1) * GM_MAXK + j] = make_double2(0.0, 0.0);
+    H[(j + 1) * GM_MAXK + j] = zero;
     const double2 m = cmul(sn, gj);
     k.g[j + 1] = make_double2(-m.x, -m.y);
     k.g[j] = cmul(cconj(cs), gj);
@@ -788,7 +786,8 @@ struct GmUpdate {
     cpx<AT> vx[NC];
     ldv<P, NC, AT>(x, rhs, par, h, vx);
     const int kj = k.j;
-#pragma unroll 4
+    constexpr int U = NC == 12 ? 1 : 4;  // whole sites: 80 registers, 3 blocks per SM
+#pragma unroll U
     for (int i = 0; i < kj; ++i) {
       cpx<AT> vi[NC];
       ldv<P, NC, AT>(V.v[i], rhs, par, h, vi);

@@ -8,10 +8,10 @@
 // tree, so the result does not depend on which block finished last, and hands
 // the totals to f.finalize(rhs, tot) on the device.  The ticket is reset for
 // the next launch on the same stream.  A functor with a member
-// finalize_warp(rhs, tot, lane) has it run by the 32 lanes of warp 0 instead
-// (scalar updates over many independent entries, e.g. the shifts of a
-// multi-shift solve, then take one round of global-memory latency, not one
-// per entry).
+// finalize_warp(rhs, tot, lane) has it run by the 32 lanes of a warp instead
+// (scalar updates over many entries, e.g. the shifts of a multi-shift solve or
+// a Hessenberg column, then take one round of global-memory latency, not one
+// per entry, and a few registers per lane).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -108,43 +108,47 @@ __device__ __forceinline__ void grid_final_reduce(const F& f, unsigned nslots, i
   const int nw = (blockDim.x + 31) >> 5;
   // U independent partial loads in flight per thread and step (fixed order)
   constexpr int U = NRED >= 8 ? 1 : 8 / NRED;
-  if constexpr (!has_warp_finalize<F>::value) {
-    // several right-hand sides: warp w sums and finalises rhs w, w + nw, ...
-    // (each finalize touches only its own rhs's state), so the finalize
-    // latencies of up to nw right-hand sides overlap and no block barrier
-    // separates them
-    if (nrhs > 1) {
-      for (int r = warp; r < nrhs; r += nw) {
-        double s[NRED];
+  // several right-hand sides: warp w sums and finalises rhs w, w + nw, ...
+  // (each finalize touches only its own rhs's state), so the finalize
+  // latencies of up to nw right-hand sides overlap and no block barrier
+  // separates them
+  if (nrhs > 1) {
+    for (int r = warp; r < nrhs; r += nw) {
+      double s[NRED];
 #pragma unroll
-        for (int k = 0; k < NRED; ++k) s[k] = 0.0;
-        const double* pr = partials + (int64_t)r * nslots * NRED;
-        const unsigned ns = rhs_sites ? (unsigned)min((int64_t)nslots, (rhs_sites[r] + blockDim.x - 1) / blockDim.x)
-                                      : nslots;
-        for (unsigned b0 = lane; b0 < ns; b0 += U * 32) {
-          double v[U][NRED];
+      for (int k = 0; k < NRED; ++k) s[k] = 0.0;
+      const double* pr = partials + (int64_t)r * nslots * NRED;
+      const unsigned ns = rhs_sites ? (unsigned)min((int64_t)nslots, (rhs_sites[r] + blockDim.x - 1) / blockDim.x)
+                                    : nslots;
+      for (unsigned b0 = lane; b0 < ns; b0 += U * 32) {
+        double v[U][NRED];
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const unsigned b = b0 + u * 32;
+        for (int u = 0; u < U; ++u) {
+          const unsigned b = b0 + u * 32;
 #pragma unroll
-            for (int k = 0; k < NRED; ++k) v[u][k] = b < ns ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int k = 0; k < NRED; ++k) s[k] += v[u][k];
+          for (int k = 0; k < NRED; ++k) v[u][k] = b < ns ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
         }
 #pragma unroll
-        for (int k = 0; k < NRED; ++k) {
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], o);
-        }
+          for (int k = 0; k < NRED; ++k) s[k] += v[u][k];
+      }
+#pragma unroll
+      for (int k = 0; k < NRED; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], o);
+      }
+      if constexpr (has_warp_finalize<F>::value) {
+#pragma unroll
+        for (int k = 0; k < NRED; ++k) s[k] = __shfl_sync(0xffffffffu, s[k], 0);
+        f.finalize_warp(r, s, lane);
+      } else {
         if (lane == 0) f.finalize(r, s);
       }
-      __syncthreads();
-      if (threadIdx.x == 0) *counter = 0u;
-      return;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) *counter = 0u;
+    return;
   }
   for (int r = 0; r < nrhs; ++r) {
     double s[NRED];

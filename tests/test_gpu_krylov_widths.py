@@ -1,7 +1,8 @@
 """GMRES and multi-shift FOM / GMRES at Krylov dimensions around the group size
 of the multi-dot launches (4 inner products per block) and at the limits, on a
-lattice whose checkerboard is no multiple of a block, and GMRES in a batch of
-uneven lattices: solutions to the oracle's true residual 1e-10."""
+lattice whose checkerboard is no multiple of a block, GMRES on both sides of the
+size from which one block takes all columns, and in a batch of uneven lattices:
+solutions to the oracle's true residual 1e-10."""
 import numpy as np
 import pytest
 
@@ -29,6 +30,28 @@ def test_gmres_widths(ctx, clg, oracle, max_dim, prec):
     for r in range(3):
         assert infos[r]["status"] == 0
         assert op.true_residual(b.to_numpy(r), x.to_numpy(r)) <= TOL
+
+
+# 16384 sites over all right-hand sides is the last size of the grouped form:
+# 8^4 with 8 and 9 of them, and 20160 on a checkerboard of 5040 sites (19.7 blocks)
+@pytest.mark.parametrize("dims,nrhs", [((8, 8, 8, 8), 8), ((8, 8, 8, 8), 9), ((6, 10, 14, 12), 4)])
+@pytest.mark.parametrize("max_dim", [1, 4, 5, 16])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_gmres_forms(ctx, clg, oracle, dims, nrhs, max_dim, prec):
+    lat = clg.Lattice(ctx, dims)
+    U = clg.CFieldGaugeSU3(lat)
+    U.InitialField(clg.GAUGE_HAAR, 0xC1A60001, 1)
+    b, x = (clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=nrhs) for _ in range(2))
+    for r in range(nrhs):
+        b.InitialField(clg.SOURCE_GAUSS, 50 + r, 2, rhs=r)
+    S = clg.CSLASolverGMRES(ctx, inner_precision=prec, MaxDim=max_dim)
+    infos = S.Solve(x, b, U, clg.EFO_F_D)
+    op = oracle.Operator("WILSON_D", dims, U.CopyDataOut(), KAPPA)
+    for r in range(nrhs):
+        assert infos[r]["status"] == 0
+        assert op.true_residual(b.to_numpy(r), x.to_numpy(r)) <= TOL
+    for o in (S, b, x, U, lat):
+        o.close()
 
 
 @pytest.mark.parametrize("prec", [0, 1, 2])
