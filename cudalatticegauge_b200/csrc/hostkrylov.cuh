@@ -20,7 +20,12 @@ namespace hk {
 using dense::Z;
 
 constexpr int MAXV = 34;  // vectors of one multi-dot or linear combination (m + 1 <= 33, + 1)
-constexpr int MDG = 4;    // inner products per block of a multi-dot
+// Inner products per block of a multi-dot: w is read once per group.  MDH for the
+// products read back to the host, whose launch ends with a last block: GCRO-DR on
+// 16^3x32 takes 210 ms with 4 and 186 with 8, on 32^3x16 725 and 613.  In the
+// device's Arnoldi cycle, where nothing waits for the products' last block, 8 are
+// slower: FOM(30) on 16^3x32 24.4 ms with 4, 26.8 with 8.
+constexpr int MDG = 4, MDH = 8;
 
 // The vectors of one launch by their data pointers; all have the shape of the
 // launch (HostVecs::proto), seen as NC / 3 times as many blocks of 3 components
@@ -38,13 +43,12 @@ __device__ __forceinline__ void ld3(const char* v, int64_t off, int64_t kstride,
   }
 }
 
-// out[i] = v_i^+ w for n vectors, MDG of them per block (right-hand side g of
-// the launch = vectors MDG g ..): w is read once per MDG vectors, and the blocks
-// of all vectors run side by side.  One block over all vectors reduced 32
-// numbers per block on 32 blocks of 8^3x16 (19 us a launch whatever n).
-// PART: left as block partials [group][slot][2 MDG] for the linear combination
-// that follows (LinCombF::dots).
-template <bool PART>
+// out[i] = v_i^+ w for n vectors, G of them per block (right-hand side g of the
+// launch = vectors G g ..), so that the blocks of all vectors run side by side.
+// One block over all vectors reduced 32 numbers per block on 32 blocks of 8^3x16
+// (19 us a launch whatever n).  PART: left as block partials [group][slot][2 G]
+// for the linear combination that follows (LinCombF::dots).
+template <bool PART, int G>
 struct MultiDotF {
   static constexpr bool PARTIALS = PART, ONE_LATTICE = true;
   const char* w;
@@ -58,10 +62,10 @@ struct MultiDotF {
     cpx<double> wv[3];
     ld3(w, off, kstride, wv);
 #pragma unroll
-    for (int i = 0; i < MDG; ++i) {
-      if (MDG * g + i >= n) break;
+    for (int i = 0; i < G; ++i) {
+      if (G * g + i >= n) break;
       cpx<double> a[3];
-      ld3(v.v[MDG * g + i], off, kstride, a);
+      ld3(v.v[G * g + i], off, kstride, a);
       double re = 0.0, im = 0.0;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -74,8 +78,8 @@ struct MultiDotF {
   }
   __device__ void finalize(int g, const double* s) const {
 #pragma unroll
-    for (int i = 0; i < MDG; ++i) {
-      const int k = MDG * g + i;
+    for (int i = 0; i < G; ++i) {
+      const int k = G * g + i;
       if (k >= n) break;
       out[k] = make_double2(s[2 * i], s[2 * i + 1]);
     }
@@ -253,9 +257,9 @@ struct HostKrylov {
   // blocks of 3 components of a vector (VecTab)
   int blocks() const { return W.proto.nparity * (nc / 3); }
   int64_t block_bytes() const { return 3 * Vh * 16; }
-  template <bool PART>
-  MultiDotF<PART> multidot(const FieldRef& w, const FieldRef* const* vs, int n) const {
-    MultiDotF<PART> f;
+  template <bool PART, int G>
+  MultiDotF<PART, G> multidot(const FieldRef& w, const FieldRef* const* vs, int n) const {
+    MultiDotF<PART, G> f;
     f.w = w.data;
     for (int i = 0; i < MAXV; ++i) f.v.v[i] = i < n ? vs[i]->data : nullptr;
     f.blk = block_bytes();
@@ -269,9 +273,11 @@ struct HostKrylov {
     out.assign(vs.size(), Z(0.0, 0.0));
     for (size_t i0 = 0; i0 < vs.size(); i0 += MAXV) {
       const int n = (int)std::min<size_t>(MAXV, vs.size() - i0);
-      if (clg_status st = launch_sites<2 * MDG>(ctx, multidot<false>(w, vs.data() + i0, n), 0, blocks(), Vh,
-                                               (n + MDG - 1) / MDG))
-        return st;
+      const FieldRef* const* v = vs.data() + i0;
+      const clg_status st =
+          n <= MDG ? launch_sites<2 * MDG>(ctx, multidot<false, MDG>(w, v, n), 0, blocks(), Vh, 1)
+                   : launch_sites<2 * MDH>(ctx, multidot<false, MDH>(w, v, n), 0, blocks(), Vh, (n + MDH - 1) / MDH);
+      if (st) return st;
       double h[2 * MAXV];
       cudaError_t e = cudaMemcpyAsync(h, W.dev_out, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, ctx->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -376,7 +382,7 @@ inline clg_status arnoldi_step(HostKrylov& K, ArnoldiState* st, double* part, co
     f.first = first;
   };
   for (int pass = 0; pass < 2; ++pass) {
-    if (clg_status e = launch_sites<2 * MDG>(K.ctx, K.multidot<true>(w, V, n), 0, K.blocks(), K.Vh, groups, part)) return e;
+    if (clg_status e = launch_sites<2 * MDG>(K.ctx, K.multidot<true, MDG>(w, V, n), 0, K.blocks(), K.Vh, groups, part)) return e;
     if (pass == 0) {
       auto f = K.combination<0, LC_DOTS>(w, w, Z(1.0, 0.0), V, n);
       fill(f, 1);
