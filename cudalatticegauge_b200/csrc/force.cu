@@ -294,16 +294,16 @@ struct KsForceArgs {
   double a[KS_FORCE_MAX];
 };
 
-// m[r][q] += l[r] conj(r[q])
-__device__ __forceinline__ void outer3_acc(C m[9], const C l[3], const C r[3]) {
+// m[r][q] += l[r] conj(r[q]) + k[r] conj(s[q]); the four products of an entry are
+// summed before they meet the pole sum, so that it is rounded once per pole
+__device__ __forceinline__ void outer3_pair(C m[9], const C l[3], const C r[3], const C k[3], const C s[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      C t = m[3 * i + j];
-      t.x = fma(l[i].x, r[j].x, fma(l[i].y, r[j].y, t.x));
-      t.y = fma(l[i].y, r[j].x, fma(-l[i].x, r[j].y, t.y));
-      m[3 * i + j] = t;
+      C& t = m[3 * i + j];
+      t.x += fma(l[i].x, r[j].x, fma(l[i].y, r[j].y, fma(k[i].x, s[j].x, k[i].y * s[j].y)));
+      t.y += fma(l[i].y, r[j].x, fma(-l[i].x, r[j].y, fma(k[i].y, s[j].x, -k[i].x * s[j].y)));
     }
 }
 
@@ -380,22 +380,19 @@ __global__ void __launch_bounds__(128, 4) ks_force_kernel(KsForceArgs a) {
     __syncthreads();              // everyone's did, and slot i - 1 is free
     issue(i + NSTAGE - 1);
     cp_async_commit();
-    C fn[3], dn[3], v[3];  // a phi_i(x+mu), -a phi_id(x+mu), the other factor
-    const double2* st = sm + (i % NSTAGE) * KS_SLOT;
-    const double2* nb = st + KS_HERE + mu * 6 * TILE + lane;
+    C fn[3], dn[3], fh[3], dh[3];  // a phi_i(x+mu), -a phi_id(x+mu), phi_i(x), phi_id(x)
+    const double2* st = sm + (i % NSTAGE) * KS_SLOT + lane;
+    const double2* nb = sm + (i % NSTAGE) * KS_SLOT + KS_HERE + mu * 6 * TILE + lane;
     const double w = a.a[i];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double2 x = nb[k * TILE], y = nb[(3 + k) * TILE];
+      const double2 x = nb[k * TILE], y = nb[(3 + k) * TILE], u = st[k * TILE], v = st[(3 + k) * TILE];
       fn[k] = mk<double>(w * x.x, w * x.y);
       dn[k] = mk<double>(-w * y.x, -w * y.y);
+      fh[k] = mk<double>(u.x, u.y);
+      dh[k] = mk<double>(v.x, v.y);
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) v[k] = mk<double>(st[(3 + k) * TILE + lane].x, st[(3 + k) * TILE + lane].y);
-    outer3_acc(W, fn, v);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) v[k] = mk<double>(st[k * TILE + lane].x, st[k * TILE + lane].y);
-    outer3_acc(W, dn, v);
+    outer3_pair(W, fn, dh, dn, fh);
   }
   cp_async_wait<0>();  // U and F: read by the threads that copied them
   if (!live) return;
