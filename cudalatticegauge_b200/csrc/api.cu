@@ -64,6 +64,21 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
+// Frees idle blocks of s (locked), the one idle longest first, until `room` more
+// bytes fit under the bound and the table has a free entry; all of them for room =
+// most.  cudaFree waits for the kernels that used a block.
+static void scratch_evict(ScratchPool& s, size_t room) {
+  while (s.n && (s.total + room > ScratchPool::most || s.n == ScratchPool::table)) {
+    int old = -1;
+    for (int k = 0; k < s.n; ++k)
+      if (!s.blocks[k].used && (old < 0 || s.blocks[k].last < s.blocks[old].last)) old = k;
+    if (old < 0) return;
+    s.total -= s.blocks[old].bytes;
+    dfree(s.blocks[old].p);
+    s.blocks[old] = s.blocks[--s.n];
+  }
+}
+
 clg_status Scratch::get(clg_context_s* ctx, size_t bytes) {
   ctx_ = ctx;
   bytes = std::max<size_t>((bytes + 511) & ~(size_t)511, 512);
@@ -71,25 +86,31 @@ clg_status Scratch::get(clg_context_s* ctx, size_t bytes) {
   // and the wait of such a call were
   if (stream_capturing(ctx->stream))
     return ctx->fail(CLG_ERR_CUDA, "scratch memory inside a stream capture");
-  const bool pool = bytes <= ScratchPool::most / 2;
+  const bool pool = bytes <= ScratchPool::most;
   ScratchPool& s = ctx->pool;
   if (pool) {
     std::lock_guard<std::mutex> lk(s.m);
     ScratchPool::Block* best = nullptr;
-    for (auto& b : s.blocks)
+    for (int k = 0; k < s.n; ++k) {
+      ScratchPool::Block& b = s.blocks[k];
       if (!b.used && b.bytes >= bytes && b.bytes <= 2 * bytes && (!best || b.bytes < best->bytes)) best = &b;
+    }
     if (best) {
       best->used = true;
+      best->last = ++s.clock;
       p_ = best->p;
       pooled_ = true;
       return CLG_SUCCESS;
     }
+    size_t held = bytes;  // what evicting cannot give back
+    for (int k = 0; k < s.n; ++k) held += s.blocks[k].used ? s.blocks[k].bytes : 0;
+    if (held <= ScratchPool::most) scratch_evict(s, bytes);
   }
   if (clg_status st = dalloc(ctx, &p_, bytes)) return st;
   if (!pool) return CLG_SUCCESS;
   std::lock_guard<std::mutex> lk(s.m);
-  if (s.total + bytes > ScratchPool::most) return CLG_SUCCESS;
-  s.blocks.push_back({p_, bytes, true});
+  if (s.total + bytes > ScratchPool::most || s.n == ScratchPool::table) return CLG_SUCCESS;
+  s.blocks[s.n++] = {p_, bytes, true, ++s.clock};
   s.total += bytes;
   pooled_ = true;
   return CLG_SUCCESS;
@@ -103,23 +124,13 @@ Scratch::~Scratch() {
     return;
   }
   std::lock_guard<std::mutex> lk(ctx_->pool.m);
-  for (auto& b : ctx_->pool.blocks)
-    if (b.p == p_) b.used = false;
+  for (int k = 0; k < ctx_->pool.n; ++k)
+    if (ctx_->pool.blocks[k].p == p_) ctx_->pool.blocks[k].used = false;
 }
 
 void scratch_trim(clg_context_s* ctx) {
-  ScratchPool& s = ctx->pool;
-  std::lock_guard<std::mutex> lk(s.m);
-  std::vector<ScratchPool::Block> keep;
-  for (auto& b : s.blocks) {
-    if (b.used) {
-      keep.push_back(b);
-      continue;
-    }
-    s.total -= b.bytes;
-    dfree(b.p);  // waits for the kernels that used it
-  }
-  s.blocks.swap(keep);
+  std::lock_guard<std::mutex> lk(ctx->pool.m);
+  scratch_evict(ctx->pool, ScratchPool::most);
 }
 
 // bytes of one right-hand side of a host (FP64 lexicographic) field array

@@ -64,18 +64,24 @@ namespace clg {
 // 1 ms and a device-wide wait, more than the operator itself on every lattice
 // up to 32^3x16.  A block belongs to one call from get to put; its next user
 // comes later on the same stream, so nothing waits.  At most `most` bytes are
-// kept, and an allocation of any context of the device that fails gives the
-// idle ones back and is tried once more (dalloc).  Locked: several threads may use one context.
+// kept; a request that would exceed them first frees the blocks idle the longest,
+// so a program that goes on to other sizes keeps theirs instead.  An allocation
+// of any context of the device that fails gives the idle ones back and is tried
+// once more (dalloc).  Locked: several threads may use one context.
 struct ScratchPool {
   struct Block {
     void* p;
     size_t bytes;
     bool used;
+    uint64_t last;  // `clock` when it was last taken
   };
   static constexpr size_t most = (size_t)1 << 30;
+  static constexpr int table = 64;  // a fixed table: the pool allocates nothing on the host
   std::mutex m;
-  std::vector<Block> blocks;
+  Block blocks[table];
+  int n = 0;
   size_t total = 0;
+  uint64_t clock = 0;
 };
 }  // namespace clg
 

@@ -1,6 +1,7 @@
 """The context's scratch pool: operators in place and products reuse its blocks,
-results do not depend on what a block held before, the pool stays bounded and
-gives its memory back when an allocation needs it and when the context ends."""
+results do not depend on what a block held before, the pool stays bounded, lets
+the longest idle blocks go for new sizes, and gives its memory back when an
+allocation fails and when the context ends."""
 import numpy as np
 import pytest
 
@@ -76,3 +77,36 @@ def test_pool_is_bounded_and_given_back(clg):
     assert free0 - torch.cuda.mem_get_info(0)[0] <= 64 << 20
     assert lib.clg_context_synchronize(base.h) == clg.SUCCESS
     base.close()
+
+
+def test_idle_blocks_make_room(clg):
+    """Three blocks of 288 MiB fill the pool; a product that then needs 384 MiB
+    takes the place of one of them and is kept, so that its next call allocates
+    nothing.  An allocation that cannot succeed returns every idle block."""
+    import torch
+
+    def held():
+        c.synchronize()
+        return free0 - torch.cuda.mem_get_info(0)[0]
+
+    c = clg.Context(0)
+    lat = clg.Lattice(c, (32, 32, 32, 16))
+    U = clg.CFieldGaugeSU3(lat)
+    U.InitialField(clg.GAUGE_EXPH, 5, 1, 0.25)
+    f = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, subset=clg.EVEN, nrhs=6)
+    g = clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=4)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info(0)[0]
+    f.ApplyOperator(clg.OP_MEE_MEEDAG, U)
+    three = held()
+    assert abs(three - (864 << 20)) <= 16 << 20
+    for _ in range(3):
+        g.DDdagger(U)
+        assert abs(held() - three - (96 << 20)) <= 16 << 20
+    with pytest.raises(clg.CLGError):
+        clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=4000)  # 400 GB
+    assert held() <= 16 << 20
+    g.DDdagger(U)  # and the context goes on
+    for o in (f, g, U, lat):
+        o.close()
+    c.close()
