@@ -721,6 +721,9 @@ clg_status clg_gauge_export(clg_gauge g, double* data, int on_device) {
 
 clg_status clg_gauge_random(clg_gauge g, int init, uint64_t seed, uint32_t field_id, double eps) {
   if (!g || init < 0 || init > CLG_GAUGE_ZERO) return CLG_ERR_BAD_ARG;
+  // the links' deviation is noted below, not when a graph would write them
+  if (stream_capturing(g->lat->ctx->stream))
+    return g->lat->ctx->fail(CLG_ERR_CUDA, "links are not generated inside a stream capture");
   clg_status st = gauge_generate(g, init, seed, field_id, eps);
   if (st) return st;
   // unit links deviate by 0, zero links (a force accumulator) by |0 - 1| = 1

@@ -110,3 +110,31 @@ def test_idle_blocks_make_room(clg):
     for o in (f, g, U, lat):
         o.close()
     c.close()
+
+
+@pytest.mark.parametrize("init", ["GAUGE_ZERO", "GAUGE_IDENTITY", "GAUGE_HAAR"])
+def test_links_are_not_generated_in_a_capture(clg, init):
+    """What the links deviate by is noted on the host at once, so a generation that
+    a graph would run later is refused and changes nothing."""
+    import torch
+
+    s = torch.cuda.Stream()
+    c = clg.Context(0, s.cuda_stream)
+    lat = clg.Lattice(c, (4, 4, 4, 4))
+    U = clg.CFieldGaugeSU3(lat)
+    U.InitialField(clg.GAUGE_EXPH, 5, 1, 0.25)
+    before, dev = U.CopyDataOut(), U.unitarity()
+    t = torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s, capture_error_mode="relaxed"):
+        t += 1
+        status = c.lib.clg_gauge_random(U.h, getattr(clg, init), 1, 1, 0.0)
+    assert status != clg.SUCCESS
+    graph.replay()
+    torch.cuda.synchronize()
+    assert U.unitarity() == dev
+    np.testing.assert_array_equal(U.CopyDataOut(), before)
+    for o in (U, lat):
+        o.close()
+    c.close()
