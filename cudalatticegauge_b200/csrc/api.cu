@@ -223,15 +223,16 @@ clg_status ensure_reduction(clg_context_s* ctx, int64_t doubles) {
   if (doubles <= ctx->red_capacity) return CLG_SUCCESS;
   if (stream_capturing(ctx->stream))
     return ctx->fail(CLG_ERR_BAD_ARG, "reduction scratch must be sized before stream capture");
-  int64_t n = doubles < 65536 ? 65536 : doubles;
-  if (ctx->red_partials) {
-    cudaStreamSynchronize(ctx->stream);
-    dfree(ctx->red_partials);
-    ctx->red_partials = nullptr;
-    ctx->red_capacity = 0;
-  }
-  clg_status st = dalloc(ctx, (void**)&ctx->red_partials, (size_t)n * sizeof(double));
-  if (st) return st;
+  // A solver's captured graphs keep the buffer's address: one that was outgrown
+  // stays until the context ends.  Each is at least twice the one before, so all
+  // of them are less than the newest.
+  const int64_t n = std::max<int64_t>({doubles, 2 * ctx->red_capacity, 65536});
+  void* p = nullptr;
+  if (ctx->red_old == std::size(ctx->red_outgrown))
+    return ctx->fail(CLG_ERR_OOM, "reduction scratch");
+  if (clg_status st = dalloc(ctx, &p, (size_t)n * sizeof(double))) return st;
+  if (ctx->red_partials) ctx->red_outgrown[ctx->red_old++] = ctx->red_partials;
+  ctx->red_partials = static_cast<double*>(p);
   ctx->red_capacity = n;
   return CLG_SUCCESS;
 }
@@ -533,6 +534,7 @@ clg_status clg_context_destroy(clg_context ctx) {
     cudaGetLastError();
   }
   scratch_trim(ctx);
+  for (size_t k = 0; k < ctx->red_old; ++k) dfree(ctx->red_outgrown[k]);
   dfree(ctx->red_partials);
   dfree(ctx->red_counter);
   dfree(ctx->staging);

@@ -98,6 +98,8 @@ struct clg_context_s {
   // red_counter[1 .. kRedGroups] the group tickets (grid_reduce_finalize2)
   double* red_partials = nullptr;
   int64_t red_capacity = 0;  // doubles
+  void* red_outgrown[48];    // smaller ones that captured graphs may hold (ensure_reduction)
+  size_t red_old = 0;
   unsigned int* red_counter = nullptr;
   // device staging buffer of host field imports/exports (grow-only; one FP64
   // lexicographic field).  Kept across calls so that a host round trip costs

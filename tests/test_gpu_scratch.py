@@ -138,3 +138,40 @@ def test_links_are_not_generated_in_a_capture(clg, init):
     for o in (U, lat):
         o.close()
     c.close()
+
+
+def test_graphs_outlive_a_larger_reduction(clg, oracle):
+    """A solver's captured iterations hold the address of the context's reduction
+    buffer: a larger solve on the same context may replace the buffer, and the
+    first solver's next call replays on the one it captured."""
+    c = clg.Context(0)
+    dims = (8, 8, 8, 16)
+
+    def setup(dims, nrhs):
+        lat = clg.Lattice(c, dims)
+        U = clg.CFieldGaugeSU3(lat)
+        U.InitialField(clg.GAUGE_EXPH, 5, 1, 0.25)
+        b, x = (clg.CFieldFermionWilsonSquareSU3(lat, KAPPA, nrhs=nrhs) for _ in range(2))
+        for r in range(nrhs):
+            b.InitialField(clg.SOURCE_GAUSS, 9 + r, 2, rhs=r)
+        return lat, U, b, x
+
+    lat, U, b, x = setup(dims, 4)
+    for prec in (clg.HALF, clg.DOUBLE):
+        S = clg.CSLASolverCG(c, inner_precision=prec, tol_true_rel=1e-10)
+        for _ in range(2):
+            S.Solve(x, b, U, clg.EFO_F_D)
+        first = [x.to_numpy(r) for r in range(4)]
+        big = setup((32, 32, 32, 16), 12 if prec == clg.HALF else 24)  # partials for 8192 tiles each
+        T = clg.CSLASolverCG(c, inner_precision=clg.HALF, tol_true_rel=1e-10, max_iterations=32)
+        T.Solve(big[3], big[2], big[1], clg.EFO_F_D, raise_on_fail=False)
+        for o in (T, *reversed(big)):
+            o.close()
+        x.Zero()
+        S.Solve(x, b, U, clg.EFO_F_D)
+        for r in range(4):
+            np.testing.assert_array_equal(x.to_numpy(r), first[r])
+        S.close()
+    for o in (x, b, U, lat):
+        o.close()
+    c.close()
