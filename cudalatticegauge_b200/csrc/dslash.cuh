@@ -39,6 +39,8 @@ struct AlphaFin {
   int* status;
   int* done;
   int* skip;
+  int* iters;     // a breakdown ends the iteration here: its `weight` applications
+  int weight;     // are counted (else Cg1P counts them)
   int breakdown;  // the status value
 };
 
@@ -368,6 +370,7 @@ __device__ __forceinline__ void alpha_block(const AlphaFin& f) {
   const double pAp = block_total(f.partials, f.n);
   if (threadIdx.x != 0 || skip) return;
   if (!(pAp > 0.0) || isinf(pAp)) {
+    *f.iters += f.weight;
     *f.status = f.breakdown;
     *f.done = *f.skip = 1;
   } else {
@@ -808,7 +811,16 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_kernel(HopArgs a
     alpha_block(a.fin);
     return;
   }
-  if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;  // uniform over the block
+  bool skip = a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride];
+  if (!FULL && a.fin.n) {
+    // alpha_block may set it meanwhile (the result is unused then): the block
+    // follows thread 0's reading, so that it stays together at the barrier
+    __shared__ bool s_skip;
+    if (threadIdx.x == 0) s_skip = skip;
+    __syncthreads();
+    skip = s_skip;
+  }
+  if (skip) return;
   if (h < a.g.Vh) wilson_split_stage<P, RECON, DAGGER>(a, rhs, h, i, t);
   __syncthreads();
   if (threadIdx.x >= 32 || h >= a.g.Vh) return;

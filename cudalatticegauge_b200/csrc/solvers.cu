@@ -1042,7 +1042,8 @@ clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, 
   clg_status s;
   if ((s = schur_hop_odd(w, d1, p, to, skip, ks))) return s;
   if ((s = schur_hop_epi1<P>(w, d1, to, p, te, CgHopAlpha<P>{st, 0}, skip, ks, pap, &npap))) return s;
-  const AlphaFin fin{pap, npap, odd ? &st->rr1 : &st->rr, &st->alpha, &st->status, &st->done, &st->skip, ST_BREAKDOWN};
+  const AlphaFin fin{pap, npap, odd ? &st->rr1 : &st->rr, &st->alpha, &st->status, &st->done, &st->skip,
+                     &st->iters, op_weight(op), ST_BREAKDOWN};
   if ((s = schur_hop_odd(w, !d1, te, to, skip, ks, &fin))) return s;
   const Cg1HopUpdate<P> up{{dfield(x), dfield(r), dfield(p), st}};
   if ((s = schur_hop_epi1<P>(w, !d1, to, te, te, up, skip, ks, rrp, &nrr))) return s;

@@ -1,7 +1,9 @@
 """CG on one Wilson source: the sums that the next kernel adds up itself, on both
-sides of the partial count from which they are folded first."""
+sides of the partial count from which they are folded first, and a breakdown in
+(p, A p)."""
 import os
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +46,27 @@ def test_partials_are_folded(clg, oracle, prec):
         c.close()
     (few, n0), (many, n1) = count
     assert abs(n0 - n1) <= 8 and many - few >= n1 // 2
+
+
+@pytest.mark.parametrize("cfg", [None, "0:128"])
+def test_breakdown_counts_its_iteration(clg, cfg):
+    """Links of 1e13 are finite in single precision and (p, A p) is not: the solve
+    ends with a breakdown, at the same count of applications as the iteration with
+    separate sums, and leaves a finite solution."""
+    dims, got = (8, 8, 8, 8), []
+    for fused in ("1", "0"):
+        c = _context(clg, cfg, CLG_FUSED_CG=fused)
+        lat = clg.Lattice(c, dims)
+        U = clg.CFieldGaugeSU3(lat)
+        U.InitialField(clg.GAUGE_HAAR, 0xC1A60001, 1)
+        U.InitialWithByte(1e13 * U.CopyDataOut())
+        b, x = (clg.CFieldFermionWilsonSquareSU3(lat, KAPPA) for _ in range(2))
+        b.InitialField(clg.SOURCE_GAUSS, 400, 2)
+        S = clg.CSLASolverCG(c, inner_precision=clg.SINGLE, tol_true_rel=1e-10)
+        info = S.Solve(x, b, U, clg.EFO_F_D, raise_on_fail=False)[0]
+        got.append((info["status"], info["iterations"], info["outer"], bool(np.isfinite(x.to_numpy()).all())))
+        for o in (S, b, x, U, lat):
+            o.close()
+        c.close()
+    assert got[0] == got[1]
+    assert got[0][0] != 0 and got[0][1] > 0 and got[0][3]
