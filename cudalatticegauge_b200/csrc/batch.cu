@@ -168,7 +168,6 @@ extern "C" clg_status clg_solve_lattices(clg_solver S, int n, clg_field* x, clg_
         cudaStreamSynchronize(ctx->stream) != cudaSuccess)
       return ctx->fail(CLG_ERR_CUDA, "solve_lattices: table upload");
     nw->vgauge.seg = nw->seg_dev;
-    nw->vgauge.seg_vh = nw->vh_dev;
     nw->vgauge.btile = nw->tile_dev;
     nw->vgauge.nbtile = (int)tiles.size();
     nw->vgauge.btiles = ntiles;

@@ -132,22 +132,16 @@ cudaError_t launch_wilson_pair(clg_context_s* ctx, const HopArgs& a, bool dagger
 // a batch of lattices: one right-hand side per lattice segment, untuned
 template <int P, int RECON>
 cudaError_t launch_wilson_batch(clg_context_s* ctx, const HopArgs& a, bool dagger) {
-  if (a.btile) {
-    // the tile form, one block per tile of 32 sites of one lattice (4 warps;
-    // FP16 / FP32 capped at 80 registers, FP64 at 128)
-    constexpr int CAP = P == P64 ? 2 : 3;
-    const dim3 grid((unsigned)a.btiles), block(128);
-    if constexpr (P == P16)
-      return dagger ? launch_pdl(ctx, wilson_hop_tile16_kernel<true, CAP, true>, grid, block, 0, a)
-                    : launch_pdl(ctx, wilson_hop_tile16_kernel<false, CAP, true>, grid, block, 0, a);
-    else
-      return dagger ? launch_pdl(ctx, wilson_hop_tileN_kernel<P, RECON, true, CAP, true>, grid, block, 0, a)
-                    : launch_pdl(ctx, wilson_hop_tileN_kernel<P, RECON, false, CAP, true>, grid, block, 0, a);
-  }
-  const int bs = P == P64 ? 64 : 128;
-  dim3 grid((unsigned)(((a.g.Vh + bs - 1) / bs) * a.nrhs));
-  return dagger ? launch_pdl(ctx, wilson_hop_batch_kernel<P, RECON, true>, grid, dim3(bs), 0, a)
-                : launch_pdl(ctx, wilson_hop_batch_kernel<P, RECON, false>, grid, dim3(bs), 0, a);
+  // the tile form, one block per tile of 32 sites of one lattice (4 warps;
+  // FP16 / FP32 capped at 80 registers, FP64 at 128)
+  constexpr int CAP = P == P64 ? 2 : 3;
+  const dim3 grid((unsigned)a.btiles), block(128);
+  if constexpr (P == P16)
+    return dagger ? launch_pdl(ctx, wilson_hop_tile16_kernel<true, CAP, true>, grid, block, 0, a)
+                  : launch_pdl(ctx, wilson_hop_tile16_kernel<false, CAP, true>, grid, block, 0, a);
+  else
+    return dagger ? launch_pdl(ctx, wilson_hop_tileN_kernel<P, RECON, true, CAP, true>, grid, block, 0, a)
+                  : launch_pdl(ctx, wilson_hop_tileN_kernel<P, RECON, false, CAP, true>, grid, block, 0, a);
 }
 
 }  // namespace
@@ -549,7 +543,6 @@ clg_status make_hop_args(clg_context_s* ctx, const clg_gauge_s* U, const HopSpec
   a.skip_stride = s.skip_stride;
   a.nrhs = s.nrhs > 0 ? s.nrhs : 1;
   a.seg = U->seg;
-  a.seg_vh = U->seg_vh;
   a.tile_rows = 0;
   a.btile = U->btile;
   a.nbtile = U->nbtile;

@@ -69,11 +69,9 @@ struct HopArgs {
   int skip_stride;
   int nrhs;                 // right-hand sides (interleaved in blockIdx.x)
   // a batch of lattices (nullable): right-hand side r lives on lattice seg[r]
-  // (geometry and links, checkerboard size seg_vh[r]); g.Vh is then the
-  // fields' chunk stride, the largest checkerboard of the batch, and sites
-  // h >= seg_vh[r] are padding
+  // (geometry and links); g.Vh is then the fields' chunk stride, the largest
+  // checkerboard of the batch, and sites h >= seg[r].g.Vh are padding
   const HopSeg* seg;
-  const int64_t* seg_vh;
   // the tile hops' block order (wilson_hop_tile16_kernel): 0 = tiles in site
   // order, else the rows y are walked in chunks of tile_rows (tile16_index)
   int tile_rows;
@@ -543,17 +541,6 @@ __device__ __forceinline__ void wilson_hop_site(const HopArgs& a, int rhs, int64
 // The precision index of the batch link table (HopSeg::u)
 template <int P> constexpr int seg_prec() { return P == P64 ? 0 : (P == P32 ? 1 : 2); }
 
-// Right-hand side rhs of a batch of lattices: its own geometry and links.
-// False for a padding site (h beyond that lattice's checkerboard).
-template <int P, int RECON, bool DAGGER, typename AT>
-__device__ __forceinline__ bool wilson_hop_site_batch(const HopArgs& a, int rhs, int64_t h, cpx<AT> acc[12]) {
-  const HopSeg& sg = a.seg[rhs];
-  if (h >= sg.g.Vh) return false;
-  wilson_hop_site_on<P, RECON, DAGGER, true>(a, sg.g, sg.u[seg_prec<P>()][a.out_parity], sg.u[seg_prec<P>()][1 - a.out_parity],
-                                       rhs, h, acc);
-  return true;
-}
-
 // Register caps through the launch bounds (the autotuner picks per operator):
 // (256, 3) caps at 80 registers (24 resident warps per SM instead of 16): the
 // hop is latency-bound on its gathers, and the low-precision variants fit in
@@ -829,32 +816,17 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_kernel(HopArgs a
   wilson_hop_store<P>(a, rhs, h, acc);
 }
 
-// The hop over a batch of lattices (HopArgs::seg): right-hand side r on its own
-// lattice, the grid spanning the largest checkerboard.
-// (the register caps of the tuned one-lattice kernels: 80 for FP32 / FP16,
-// 128 for FP64)
-template <int P, int RECON, bool DAGGER>
-__global__ void __launch_bounds__(256, P == P64 ? 2 : 3) wilson_hop_batch_kernel(HopArgs a) {
-  using AT = typename AccT<P>::T;
-  const int rhs = (int)(blockIdx.x % (unsigned)a.nrhs);
-  const int64_t h = (int64_t)(blockIdx.x / (unsigned)a.nrhs) * blockDim.x + threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();
-  if (h >= a.g.Vh) return;
-  if (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) return;
-  cpx<AT> acc[12];
-  if (wilson_hop_site_batch<P, RECON, DAGGER>(a, rhs, h, acc)) wilson_hop_store<P>(a, rhs, h, acc);
-}
-
 // The hop with a fused epilogue E (used by the Krylov solvers):
 //   E::STORE      the result is stored to a.out (else it only feeds E::site)
-//   E::NRED       doubles reduced over the grid per rhs, E::finalize(rhs, tot)
-//                 runs on the device in the last block (grid_reduce_finalize2)
+//   E::NRED       doubles reduced over the grid per rhs: E::PARTIALS leaves one
+//                 partial per block ([rhs][slot]) to the next kernel (Cg1P,
+//                 AlphaFin, epi_final_kernel), else E::finalize(rhs, tot) runs in
+//                 the last block (grid_reduce_finalize2)
 //   E::site(rhs, h, acc, red)   per-site work on the result in registers
 // Every thread reaches the block reduction: out-of-range sites contribute
-// zero; a block of a skipped (finished) right-hand side only takes its ticket,
-// and E::finalize ignores such right-hand sides.
-template <int P, int RECON, bool DAGGER, int MAXT, int MINB, class E, bool BATCH = false>
+// zero.  A block of a skipped (finished) right-hand side writes no partial and at
+// most takes its ticket; whoever sums ignores such right-hand sides.
+template <int P, int RECON, bool DAGGER, int MAXT, int MINB, class E>
 __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E e, double* partials,
                                                                     double* gpart, unsigned* counter,
                                                                     unsigned group) {
@@ -864,9 +836,7 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
   const int64_t h = (int64_t)slot * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();
-  // in a batch of lattices a block wholly in this rhs's padding reduces nothing
-  const bool skipped = (a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride]) ||
-                       (BATCH && (int64_t)slot * blockDim.x >= a.seg_vh[rhs]);
+  const bool skipped = a.skip_dev && a.skip_dev[(int64_t)rhs * a.skip_stride];
   double red[E::NRED];
 #pragma unroll
   for (int k = 0; k < E::NRED; ++k) red[k] = 0.0;
@@ -874,24 +844,15 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_hop_epi_kernel(HopArgs a, E
     if (!skipped && h < a.g.Vh) e.prefetch(rhs, h);
   if (!skipped && h < a.g.Vh) {
     cpx<AT> acc[12];
-    bool valid = true;
-    if constexpr (BATCH)
-      valid = wilson_hop_site_batch<P, RECON, DAGGER>(a, rhs, h, acc);
-    else
-      wilson_hop_site<P, RECON, DAGGER>(a, rhs, h, acc);
-    if (valid) {
-      if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
-      e.site(rhs, h, acc, red);
-    }
+    wilson_hop_site<P, RECON, DAGGER>(a, rhs, h, acc);
+    if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
+    e.site(rhs, h, acc, red);
   }
   if constexpr (partials_only<E>::value) {
     if (!skipped) block_partials<E::NRED>(red, partials, (int64_t)rhs * (gridDim.x / (unsigned)a.nrhs) + slot);
   } else {
-    const int rr[1] = {rhs};
-    const bool cc[1] = {!skipped}, hh[1] = {true};
-    grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
-                                      gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter,
-                                      BATCH ? a.seg_vh : nullptr);
+    grid_reduce_finalize2<E::NRED>(red, e, rhs, !skipped, slot, gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials,
+                                   gpart, counter);
   }
 }
 
@@ -919,10 +880,7 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_full_epi_kernel(HopArgs a, 
     if constexpr (E::STORE) wilson_hop_store<P>(a, rhs, h, acc);
     e.site(rhs, h, acc, red);
   }
-  const int rr[1] = {0};
-  const bool cc[1] = {true}, hh[1] = {true};
-  grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, 0u, 1u, blockIdx.x, gridDim.x, 1, group, partials, gpart,
-                                    counter);
+  grid_reduce_finalize2<E::NRED>(red, e, 0, true, blockIdx.x, gridDim.x, 1, group, partials, gpart, counter);
 }
 
 // The epilogue form with four threads per site (wilson_split_kernel): warp 0
@@ -960,10 +918,8 @@ __global__ void __launch_bounds__(4 * SPLIT_SITES) wilson_split_epi_kernel(HopAr
   if constexpr (partials_only<E>::value) {
     if (!skipped) block_partials<E::NRED>(red, partials, (int64_t)rhs * (gridDim.x / (unsigned)a.nrhs) + slot);
   } else {
-    const int rr[1] = {rhs};
-    const bool cc[1] = {!skipped}, hh[1] = {true};
-    grid_reduce_finalize2<E::NRED, 1>(red, e, rr, cc, hh, (unsigned)rhs, (unsigned)a.nrhs, slot,
-                                      gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials, gpart, counter);
+    grid_reduce_finalize2<E::NRED>(red, e, rhs, !skipped, slot, gridDim.x / (unsigned)a.nrhs, a.nrhs, group, partials,
+                                   gpart, counter);
   }
 }
 
@@ -1589,15 +1545,9 @@ __device__ __forceinline__ void tileN_epi_body(const HopArgs& a, const E& e, Til
     if constexpr (!partials_only<E>::value)
       if (lane == 0) __threadfence();
   }
-  if constexpr (partials_only<E>::value) return;  // left to the next kernel (a batch: this lattice's slots only)
-  if (r0 > 0 || r1 < a.nrhs) {
-    for (int q = threadIdx.x; q < a.nrhs * E::NRED; q += blockDim.x) {
-      const int rhs = q / E::NRED;
-      if (rhs < r0 || rhs >= r1) partials[((int64_t)rhs * nslots + blockIdx.x) * E::NRED + q % E::NRED] = 0.0;
-    }
-    __threadfence();
-  }
-  tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
+  // else left to the next kernel (a batch: this lattice's slots only)
+  if constexpr (!partials_only<E>::value)
+    tile_reduce_finalize<E::NRED>(e, nslots, a.nrhs, group, partials, gpart, counter);
 }
 
 template <int P, int RECON, bool DAGGER, int MINB, class E, bool BATCH = false>
@@ -1607,6 +1557,7 @@ __global__ void __launch_bounds__(256, MINB) wilson_hop_tileN_epi_kernel(HopArgs
   using AT = typename AccT<P>::T;
   __shared__ TileN<AT> t;
   if constexpr (BATCH) {
+    static_assert(partials_only<E>::value, "the other lattices' slots stay unwritten");
     const BatchTile bt = batch_tile(a);
     const HopSeg& sg = a.seg[bt.seg];
     const Geom g = sg.g;

@@ -196,7 +196,6 @@ struct clg_gauge_s {
   // a batch of lattices (clg_solve_lattices): per right-hand side geometry and
   // link arrays on the device; lat is then the batch's padded virtual lattice
   const clg::HopSeg* seg = nullptr;
-  const int64_t* seg_vh = nullptr;  // per right-hand side checkerboard sizes (device)
   // the batch's tiles of 32 sites per lattice (device; the tile-form hops)
   const clg::BatchTile* btile = nullptr;
   int nbtile = 0;

@@ -616,7 +616,6 @@ struct GmDots {
       acc_dot<NC, AT>(vi, vw, acc + 2 * i);
     }
   }
-  __device__ void finalize(int, const double*) const {}
 };
 
 // The same for lattices that fill the chip (gm_wide): one block over all J + 1

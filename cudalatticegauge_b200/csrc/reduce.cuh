@@ -101,7 +101,7 @@ struct one_lattice<F, std::void_t<decltype(F::ONE_LATTICE)>> : std::bool_constan
 // every thread of that block (at most 256 threads, 8 warps).
 template <int NRED, class F>
 __device__ __forceinline__ void grid_final_reduce(const F& f, unsigned nslots, int nrhs, const double* partials,
-                                                  unsigned* counter, const int64_t* rhs_sites = nullptr) {
+                                                  unsigned* counter) {
   __shared__ double sm[NRED][8];
   __shared__ double tot[NRED];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -118,15 +118,13 @@ __device__ __forceinline__ void grid_final_reduce(const F& f, unsigned nslots, i
 #pragma unroll
       for (int k = 0; k < NRED; ++k) s[k] = 0.0;
       const double* pr = partials + (int64_t)r * nslots * NRED;
-      const unsigned ns = rhs_sites ? (unsigned)min((int64_t)nslots, (rhs_sites[r] + blockDim.x - 1) / blockDim.x)
-                                    : nslots;
-      for (unsigned b0 = lane; b0 < ns; b0 += U * 32) {
+      for (unsigned b0 = lane; b0 < nslots; b0 += U * 32) {
         double v[U][NRED];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const unsigned b = b0 + u * 32;
 #pragma unroll
-          for (int k = 0; k < NRED; ++k) v[u][k] = b < ns ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
+          for (int k = 0; k < NRED; ++k) v[u][k] = b < nslots ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -155,16 +153,13 @@ __device__ __forceinline__ void grid_final_reduce(const F& f, unsigned nslots, i
 #pragma unroll
     for (int k = 0; k < NRED; ++k) s[k] = 0.0;
     const double* pr = partials + (int64_t)r * nslots * NRED;
-    // a batch of lattices: only the slots that hold sites of this rhs's lattice wrote a partial
-    const unsigned ns = rhs_sites ? (unsigned)min((int64_t)nslots, (rhs_sites[r] + blockDim.x - 1) / blockDim.x)
-                                  : nslots;
-    for (unsigned b0 = threadIdx.x; b0 < ns; b0 += U * blockDim.x) {
+    for (unsigned b0 = threadIdx.x; b0 < nslots; b0 += U * blockDim.x) {
       double v[U][NRED];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const unsigned b = b0 + u * blockDim.x;
 #pragma unroll
-        for (int k = 0; k < NRED; ++k) v[u][k] = b < ns ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
+        for (int k = 0; k < NRED; ++k) v[u][k] = b < nslots ? __ldcg(pr + (int64_t)b * NRED + k) : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -202,7 +197,7 @@ __device__ __forceinline__ void grid_final_reduce(const F& f, unsigned nslots, i
 template <int NRED, class F>
 __device__ __forceinline__ void grid_reduce_finalize(double (&acc)[NRED], const F& f, int rhs, unsigned slot,
                                                      unsigned nslots, int nrhs, double* partials, unsigned* counter,
-                                                     bool contribute = true, const int64_t* rhs_sites = nullptr) {
+                                                     bool contribute = true) {
   __shared__ double sm[NRED][8];
   __shared__ bool last;
   if (contribute) {
@@ -232,93 +227,31 @@ __device__ __forceinline__ void grid_reduce_finalize(double (&acc)[NRED], const 
   __syncthreads();
   if (!last) return;
   __threadfence();
-  grid_final_reduce<NRED>(f, nslots, nrhs, partials, counter, rhs_sites);
+  grid_final_reduce<NRED>(f, nslots, nrhs, partials, counter);
 }
 
-// Two-level form for grids with many blocks per right-hand side (the hop
-// epilogues: one block per 64-256 sites, thousands per right-hand side).  A
-// block computes R right-hand sides (rhs[0..R), R = 1 or 2, the unit `unit`
-// of nunits); acc holds NRED values per member, c[i] says whether member i
-// contributes and has[i] whether it exists (the second member of the last
-// pair of an odd count does not).  The slots of each unit are grouped by
-// `group`; the block that completes a group (ticket counter[1 + unit *
-// ngroups + g]) sums the group's partials in slot order and writes each
-// member's group total to gpart[(rhs * ngroups + g) * NRED + k]; the block
-// that completes the last group of all (ticket counter[0]) runs
-// grid_final_reduce over the group totals.  No block reads more than `group`
-// partials per right-hand side, every sum has a fixed order (deterministic),
-// and the tickets are reset for the next launch.  In a batch of lattices
-// (rhs_sites, R = 1) a group sums only the slots holding this rhs's sites.
-template <int NRED, int R, class F>
-__device__ __forceinline__ void grid_reduce_finalize2(double (&acc)[R * NRED], const F& f, const int (&rhs)[R],
-                                                      const bool (&c)[R], const bool (&has)[R], unsigned unit,
-                                                      unsigned nunits, unsigned slot, unsigned nslots, int nrhs,
-                                                      unsigned group, double* partials, double* gpart,
-                                                      unsigned* counter, const int64_t* rhs_sites = nullptr) {
-  __shared__ double sm[R * NRED][8];
+// Two-level form for grids with many blocks per right-hand side (the residual
+// hops' epilogues: one block per 32-256 sites, thousands per right-hand side).
+// `contribute` (uniform over the block) says whether the block writes a partial
+// of right-hand side rhs.  The slots of each right-hand side are grouped by
+// `group`; the block that completes a group (ticket counter[1 + rhs * ngroups +
+// g]) sums the group's partials in slot order and writes the group total to
+// gpart[(rhs * ngroups + g) * NRED + k]; the block that completes the last group
+// of all (ticket counter[0]) runs grid_final_reduce over the group totals.  No
+// block reads more than `group` partials, every sum has a fixed order
+// (deterministic), and the tickets are reset for the next launch.
+template <int NRED, class F>
+__device__ __forceinline__ void grid_reduce_finalize2(double (&acc)[NRED], const F& f, int rhs, bool contribute,
+                                                      unsigned slot, unsigned nslots, int nrhs, unsigned group,
+                                                      double* partials, double* gpart, unsigned* counter) {
+  __shared__ double sm[NRED][8];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nw = (blockDim.x + 31) >> 5;
-  bool any = false;
-#pragma unroll
-  for (int i = 0; i < R; ++i) any = any || c[i];
-  if (any) {
-#pragma unroll
-    for (int k = 0; k < R * NRED; ++k) {
-      double v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) sm[k][warp] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < R * NRED) {
-      const int i = threadIdx.x / NRED, k = threadIdx.x % NRED;
-      bool ci = c[0];
-#pragma unroll
-      for (int j = 1; j < R; ++j)
-        if (i == j) ci = c[j];
-      if (ci) {
-        double v = 0.0;
-        for (int w = 0; w < nw; ++w) v += sm[threadIdx.x][w];
-        int ri = rhs[0];
-#pragma unroll
-        for (int j = 1; j < R; ++j)
-          if (i == j) ri = rhs[j];
-        partials[((int64_t)ri * nslots + slot) * NRED + k] = v;
-        __threadfence();
-      }
-    }
-    __syncthreads();
-  }
-  const unsigned ngroups = (nslots + group - 1) / group;
-  const unsigned g = slot / group;
-  const unsigned g0 = g * group;
-  const unsigned gs = min(group, nslots - g0);
-  unsigned* gc = counter + 1 + (int64_t)unit * ngroups + g;
-  if (threadIdx.x == 0) last = atomicAdd(gc, 1u) == gs - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // this block completed group g of its unit: each member's total, in slot order
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    if (!has[i]) continue;  // uniform over the block
-    unsigned ns = gs;
-    if (rhs_sites) {
-      const int64_t used = (rhs_sites[rhs[i]] + blockDim.x - 1) / blockDim.x;
-      ns = used <= (int64_t)g0 ? 0u : (unsigned)min((int64_t)gs, used - (int64_t)g0);
-    }
-    double s[NRED];
-#pragma unroll
-    for (int k = 0; k < NRED; ++k) s[k] = 0.0;
-    const double* pg = partials + ((int64_t)rhs[i] * nslots + g0) * NRED;
-    for (unsigned b = threadIdx.x; b < ns; b += blockDim.x)
-#pragma unroll
-      for (int k = 0; k < NRED; ++k) s[k] += __ldcg(pg + (int64_t)b * NRED + k);
-    __syncthreads();  // sm is reused
+  if (contribute) {
 #pragma unroll
     for (int k = 0; k < NRED; ++k) {
-      double v = s[k];
+      double v = acc[k];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) sm[k][warp] = v;
@@ -327,13 +260,45 @@ __device__ __forceinline__ void grid_reduce_finalize2(double (&acc)[R * NRED], c
     if (threadIdx.x < NRED) {
       double v = 0.0;
       for (int w = 0; w < nw; ++w) v += sm[threadIdx.x][w];
-      gpart[((int64_t)rhs[i] * ngroups + g) * NRED + threadIdx.x] = v;
+      partials[((int64_t)rhs * nslots + slot) * NRED + threadIdx.x] = v;
       __threadfence();
     }
+    __syncthreads();
+  }
+  const unsigned ngroups = (nslots + group - 1) / group;
+  const unsigned g = slot / group;
+  const unsigned g0 = g * group;
+  const unsigned gs = min(group, nslots - g0);
+  unsigned* gc = counter + 1 + (int64_t)rhs * ngroups + g;
+  if (threadIdx.x == 0) last = atomicAdd(gc, 1u) == gs - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // this block completed group g of its right-hand side: the total, in slot order
+  double s[NRED];
+#pragma unroll
+  for (int k = 0; k < NRED; ++k) s[k] = 0.0;
+  const double* pg = partials + ((int64_t)rhs * nslots + g0) * NRED;
+  for (unsigned b = threadIdx.x; b < gs; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NRED; ++k) s[k] += __ldcg(pg + (int64_t)b * NRED + k);
+#pragma unroll
+  for (int k = 0; k < NRED; ++k) {
+    double v = s[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) sm[k][warp] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < NRED) {
+    double v = 0.0;
+    for (int w = 0; w < nw; ++w) v += sm[threadIdx.x][w];
+    gpart[((int64_t)rhs * ngroups + g) * NRED + threadIdx.x] = v;
+    __threadfence();
   }
   if (threadIdx.x == 0) *gc = 0u;
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == ngroups * nunits - 1;
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == ngroups * (unsigned)nrhs - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();

@@ -719,9 +719,6 @@ cudaError_t launch_hop_epi(clg_context_s* ctx, const HopArgs& a, const E& e, int
   const unsigned group = red_group(nslots, a.nrhs);
   double* gpart = ctx->red_partials + nslots * a.nrhs * E::NRED;
   constexpr int MINB = P == P64 ? 1 : 3;
-  if (a.seg)  // a batch of lattices
-    return launch_pdl(ctx, wilson_hop_epi_kernel<P, RECON, DAG, 256, MINB, E, true>, grid, dim3(bs), 0, a, e,
-                      ctx->red_partials, gpart, ctx->red_counter, group);
   if (bs == SPLIT_SITES)  // four threads per site (bs: sites per block)
     return launch_pdl(ctx, wilson_split_epi_kernel<P, RECON, DAG, E>, grid, dim3(4 * SPLIT_SITES), 0, a, e,
                       ctx->red_partials, gpart, ctx->red_counter, group);
@@ -756,11 +753,11 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   auto finish = [&](cudaError_t err, int64_t nslots) -> clg_status {
     if (err == cudaSuccess)
       err = launch_pdl(ctx, epi_final_kernel<E>, dim3((unsigned)w.nrhs), dim3(512), 0, e,
-                       (const double*)ctx->red_partials, nslots, skip, ks, a.btile, a.btile ? a.nbtile : 0, a.btiles);
+                       (const double*)ctx->red_partials, nslots, skip, ks, a.btile, a.seg ? a.nbtile : 0, a.btiles);
     if (err != cudaSuccess) return ctx->fail(cuda_status(err), std::string("fused hop: ") + cudaGetErrorString(err));
     return CLG_SUCCESS;
   };
-  if (a.seg && a.btile) {  // a batch of lattices: the tile form
+  if (a.seg) {  // a batch of lattices: the tile form
     if (clg_status st = ensure_reduction(ctx, red2_doubles(a.btiles, w.nrhs, 1, E::NRED))) return st;
     cudaError_t berr;
     if constexpr (P == P64)
@@ -776,7 +773,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   const int cfg1 = tuned_hop_config(ctx, w.U, plain, P == P64 ? 64 : 128);
   const int bs = (cfg1 >> 16) == HOP_SPLIT ? SPLIT_SITES : cfg1 & 0xffff;
   if constexpr (P == P16) {
-    const int tcfg = w.nrhs >= 2 && !a.seg ? tuned_hop_tile_config(ctx, w.U, plain, -1) : -1;
+    const int tcfg = w.nrhs >= 2 ? tuned_hop_tile_config(ctx, w.U, plain, -1) : -1;
     if (tcfg >= 0) {
       const int64_t nslots = (w.Vh + ((tcfg >> 16) >= 24 ? MMA_TS : TILE16) - 1) / ((tcfg >> 16) >= 24 ? MMA_TS : TILE16);
       if (clg_status st = ensure_reduction(ctx, red2_doubles(nslots, w.nrhs, 1, E::NRED))) return st;
@@ -785,7 +782,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
     }
     const int pcfg = tuned_hop_pair_config(ctx, w.U, plain, -1);
     const bool pair = ctx->hop_pair_mode == 1 || (ctx->hop_pair_mode == 2 && pcfg >= 0);
-    if (w.nrhs >= 2 && pair && !a.seg) {
+    if (w.nrhs >= 2 && pair) {
       const int cfg = pcfg >= 0 ? pcfg : 128;
       const int pbs = cfg & 0xffff;
       // partials are indexed [rhs][slot]: nslots x nrhs of them
@@ -797,7 +794,7 @@ clg_status schur_hop_epi(Work& w, bool dag, const FieldRef& t_odd, const FieldRe
   }
   if constexpr (P != P16) {
     // the tile form, when the autotuner chose it for the plain hop
-    const int pc = w.nrhs >= 2 && !a.seg ? tuned_hop_config(ctx, w.U, plain, -1) : -1;
+    const int pc = w.nrhs >= 2 ? tuned_hop_config(ctx, w.U, plain, -1) : -1;
     if (pc >= 0 && (pc >> 16) >= 16) {
       const int64_t nslots = (w.Vh + TILE16 - 1) / TILE16;
       if (clg_status st = ensure_reduction(ctx, red2_doubles(nslots, w.nrhs, 1, E::NRED))) return st;
