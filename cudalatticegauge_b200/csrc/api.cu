@@ -1,6 +1,8 @@
 // api.cu -- the C ABI (include/clg_b200.h): contexts, lattices, gauge and
 // fermion fields, operator application (CField::ApplyOperator,
 // Data/Field/CField.h:203) and field BLAS.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
@@ -663,23 +665,52 @@ static clg_status refresh_unitarity(clg_gauge_s* g) {
   return st;
 }
 
-// Whether the kernels can take the caller's on_device array of doubles as it
-// is: memory of this device, 8-byte aligned.  Anything else a device-to-device
-// copy accepts (another device's memory, an odd address) is staged.
-static bool direct_doubles(const clg_context_s* ctx, const void* p) {
+// How an on_device array of `bytes` reaches the kernels: as it is (memory of this
+// device, 8-byte aligned, all of it inside one allocation), or through a copy,
+// which takes whatever else a device-to-device copy accepts (another device's
+// memory, an odd address, several mappings in a row) and refuses the rest.  A
+// kernel would run past the end of an array that is too short; for memory of
+// cudaMalloc, which ends with its allocation, that is refused here.
+enum class ArrayRoute { DIRECT, COPY, SHORT };
+static ArrayRoute array_route(const clg_context_s* ctx, const void* p, size_t bytes) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return ArrayRoute::COPY;
   }
-  return a.type == cudaMemoryTypeDevice && a.device == ctx->device && (reinterpret_cast<uintptr_t>(p) & 7) == 0;
+  if (a.type != cudaMemoryTypeDevice || a.device != ctx->device) return ArrayRoute::COPY;
+  static const auto entry = [](const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return f;
+  };
+  static const auto range = reinterpret_cast<CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr)>(entry("cuMemGetAddressRange"));
+  static const auto attribute =
+      reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(entry("cuPointerGetAttribute"));
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!range || range(&base, &size, at) != CUDA_SUCCESS) return ArrayRoute::COPY;
+  if (bytes > size - (size_t)(at - base)) {
+    int malloced = 0;
+    if (attribute && attribute(&malloced, CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE, at) == CUDA_SUCCESS && malloced)
+      return ArrayRoute::SHORT;
+    return ArrayRoute::COPY;
+  }
+  return (at & 7) == 0 ? ArrayRoute::DIRECT : ArrayRoute::COPY;
 }
 
 clg_status clg_gauge_import(clg_gauge g, const double* data, int layout, int on_device) {
   if (!g || !data || (layout != CLG_LAYOUT_CLGBIN && layout != CLG_LAYOUT_BRIDGEPP)) return CLG_ERR_BAD_ARG;
   clg_context_s* ctx = g->lat->ctx;
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
-  const bool direct = on_device && direct_doubles(ctx, data);
+  const ArrayRoute route = on_device ? array_route(ctx, data, bytes) : ArrayRoute::COPY;
+  if (route == ArrayRoute::SHORT) return ctx->fail(CLG_ERR_CUDA, "the device array is shorter than the links");
+  const bool direct = route == ArrayRoute::DIRECT;
   // the links' deviation from SU(3), then (staged) the links
   Scratch sw, sb;
   clg_status st = sw.get(ctx, sizeof(unsigned long long));
@@ -707,7 +738,9 @@ clg_status clg_gauge_export(clg_gauge g, double* data, int on_device) {
   if (!g || !data) return CLG_ERR_BAD_ARG;
   clg_context_s* ctx = g->lat->ctx;
   const size_t bytes = (size_t)g->lat->g.V * 4 * 18 * sizeof(double);
-  const bool direct = on_device && direct_doubles(ctx, data);
+  const ArrayRoute route = on_device ? array_route(ctx, data, bytes) : ArrayRoute::COPY;
+  if (route == ArrayRoute::SHORT) return ctx->fail(CLG_ERR_CUDA, "the device array is shorter than the links");
+  const bool direct = route == ArrayRoute::DIRECT;
   Scratch sb;
   clg_status st = CLG_SUCCESS;
   if (!direct && (st = sb.get(ctx, bytes))) return st;

@@ -87,3 +87,28 @@ def test_field_reorder(ctx, clg, dims, kind, subset, shift):
             d = np.abs((got - want[r]).reshape(V, -1).view(np.float64)).max(1)
             top = np.abs(want[r].reshape(V, -1).view(np.float64)).max(1)
             assert (d <= tol * top).all()
+
+
+def test_short_device_array_is_refused(ctx, clg):
+    """A link array whose allocation ends early is refused on the host (a kernel
+    would read or write past it); one that ends with the links is taken."""
+    from cuda.bindings import driver, runtime
+
+    lat = clg.Lattice(ctx, (4, 4, 4, 4))
+    u = clg.CFieldGaugeSU3(lat)
+    u.InitialField(clg.GAUGE_HAAR, 5, 1)
+    want, need = u.CopyDataOut(), lat.volume * 4 * 18 * 8
+    for size, ok in ((need, True), (need // 2, False)):
+        err, p = runtime.cudaMalloc(size)
+        assert err == runtime.cudaError_t.cudaSuccess
+        attr = driver.CUpointer_attribute.CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE
+        err, legacy = driver.cuPointerGetAttribute(attr, p)
+        err2, _, held = driver.cuMemGetAddressRange(p)
+        known = int(err) == 0 and int(err2) == 0 and legacy and (held < need) != ok
+        if known:  # else the host cannot tell that the array is too short
+            for call in (lambda: ctx.lib.clg_gauge_export(u.h, C.c_void_p(int(p)), 1),
+                         lambda: ctx.lib.clg_gauge_import(u.h, C.c_void_p(int(p)), clg.LAYOUT_CLGBIN, 1)):
+                assert (call() == clg.SUCCESS) == ok
+            np.testing.assert_array_equal(u.CopyDataOut(), want)
+        runtime.cudaFree(p)
+        assert known
