@@ -601,7 +601,7 @@ __device__ __forceinline__ void full_block(const HopArgs& a, int& rhs, int& p, u
 }
 // The checkerboard index of the i-th site in launch order: i itself, or with
 // tile_rows > 0 (a divisor of L_y) chunk after chunk of tile_rows y-rows with x
-// slowest in a chunk, so that three x-slabs of a chunk fit in L2 (full_rows)
+// slowest in a chunk, so that two x-slabs of a chunk fit in 40 MB of L2 (full_rows)
 __device__ __forceinline__ int64_t full_site(const HopArgs& a, int64_t i) {
   if (a.tile_rows <= 0) return i;
   const unsigned np = (unsigned)a.g.L[2] * (unsigned)a.g.L[3] / 2u;
@@ -641,8 +641,12 @@ __global__ void __launch_bounds__(MAXT, MINB) wilson_full_kernel(HopArgs a) {
 // 16^3x32 it loses (37.5 against 31.1 us, FP64).
 constexpr int SPLIT_SITES = 32;
 constexpr int HOP_SPLIT = 4;  // this form's launch variant (dslash.cu)
-// up to this many sites a launch gives each of the 592 schedulers less than a
-// warp: the form is taken untimed
+// Up to this many sites the one-thread form gives each of the 592 schedulers less
+// than a warp: this form is taken untimed.  us per operator application of a CG
+// solve, the best one-thread form / this one, in FP64, FP32 and FP16: 2048 sites
+// 18.1 / 16.1, 17.6 / 13.7, 16.0 / 15.7; 10368: 22.6 / 17.5, 17.5 / 17.1, 15.6 / 17.1;
+// 18432: 25.4 / 21.9, 19.2 / 16.4, 16.5 / 16.9; above the line, where it is timed,
+// 32768: 25.2 / 31.6, 21.2 / 17.1, 20.6 / 17.5.
 constexpr int64_t SPLIT_ALWAYS = 592 * 32;
 template <int P>
 struct SplitSmem {

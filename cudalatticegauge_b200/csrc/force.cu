@@ -272,10 +272,14 @@ __global__ void __launch_bounds__(128) wilson_force_kernel(ForceArgs a) {
 // its slot and releases the one before.  Compulsory DRAM traffic per site: 2 x 48 B
 // per pole, U 576 B, F 1152 B.  Three slots leave 55 KB a block, 4 blocks (16
 // warps) per SM; with two accumulators, U and F staged beside a ring of two and
-// two barriers per pole 3 blocks fit.  12 poles on 32^3 x 16: 395 -> 321 us (3.8
-// -> 4.7 TB/s), 4 poles 207 -> 176, 24^4 with 12 poles 258 -> 206.  Beside DRAM
-// (227 us) the shared-memory pipe is what is left: each operand is written there
-// and read back, some 200 us by count; the FP64 pipe needs 117 us.
+// two barriers per pole 3 blocks fit.  The products of a pole are summed before
+// they meet W (outer3_pair): 2.8e-16 from the force in 64-bit arithmetic of another
+// order, where two accumulators gave 3.1e-16 and one running sum of all products
+// 3.6e-16.  12 poles on 32^3 x 16, in a row: two accumulators 418 us, now 343 (one
+// running sum 335); 4 poles 228 / 192 (191), 24 poles 777 / 675 (637).  Beside DRAM
+// (227 us at 6.65 TB/s) the shared-memory pipe is what is left: each operand is
+// written there and read back, some 200 us by count; the FP64 pipe is busy half
+// the time.
 constexpr int KS_FORCE_MAX = 64;
 constexpr int KS_HERE = 2 * 3 * TILE;     // phi_i(x), phi_id(x)        [field][k][site]
 constexpr int KS_NBR = 4 * 2 * 3 * TILE;  // phi_i(x+mu), phi_id(x+mu)  [mu][field][k][site]
@@ -550,8 +554,8 @@ clg_status clg_ks_force(clg_gauge F, clg_gauge U, int n, const clg_field* phi_i,
   }
   k.blk = phi_i[0]->blk;
   const int64_t nblk = (k.g.Vh + TILE - 1) / TILE;
-  // ring of 3 slots, 4 blocks per SM; measured on 32^3x16 with 12 poles against
-  // its 321 us: 2 slots with 5 or 6 blocks per SM (spills) 345 / 351, 4 slots with
+  // ring of 3 slots, 4 blocks per SM; measured on 32^3x16 with 12 poles, with one
+  // running sum, against its 321 us: 2 slots with 5 or 6 blocks per SM (spills) 345 / 351, 4 slots with
   // 3 blocks 325, the neighbours' components through registers instead of shared
   // memory 405 - 422, a barrier-free form with four direction threads per site in
   // one warp 782

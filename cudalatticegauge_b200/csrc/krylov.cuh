@@ -621,7 +621,7 @@ struct GmDots {
 // The same for lattices that fill the chip (gm_wide): one block over all J + 1
 // columns, so w is read once and every column's loads are in flight together; the
 // last block stores the Hessenberg column.  FP32-inner GMRES(12) on 32^3x16:
-// 12.9 ms, with the groups of GmDots and sums in GmOrtho's blocks 15.9.
+// 12.9 ms, with the groups of GmDots and sums in GmOrtho's blocks 13.7.
 template <int P, int NC, int J>
 struct GmDotsJ {
   VList V;

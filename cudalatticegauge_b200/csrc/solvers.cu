@@ -581,10 +581,13 @@ clg_status iterate(Work& w, int graph_slot, int chunk, int max_chunks, Body&& bo
   return CLG_SUCCESS;
 }
 
-// GMRES vector kernels with one thread per site and one block over all columns:
-// where the sites of all right-hand sides give more than half a warp per scheduler.
-// 8^4 (2048 sites) 945 us in this form against 690 in the grouped one, 16^4 (32768)
-// FP32 3.2 ms against 3.5
+// GMRES vector kernels with one thread per site and one block over all columns
+// (whole), where the sites of all right-hand sides give more than half a warp per
+// scheduler.  GMRES(12), one source, ms grouped / whole in FP64, FP32 and FP16:
+// 2048 sites 0.65 / 0.87, 0.66 / 0.80, 1.07 / 1.20; 16384: 2.48 / 2.93, 2.21 / 2.29,
+// 2.40 / 2.61; 18432: 2.96 / 3.43, 2.63 / 2.65, 2.60 / 2.84; 32768: 4.29 / 4.44, 3.11 /
+// 2.78, 2.85 / 2.96; 110592: 11.9 / 11.5, 7.05 / 5.69, 4.94 / 4.75.  The line lies where
+// FP32, the default inner precision, turns.
 bool gm_wide(int np, int64_t Vh, int nrhs) { return (int64_t)np * Vh * nrhs > 16384; }
 template <int PV, int NV, int J>
 clg_status launch_gm_dots(clg_context_s* ctx, const VList& vl, const DField& w, KState* st, int j, int fp, int np,
@@ -1023,9 +1026,10 @@ clg_status cg_fused_iteration(Work& w, int op, const FieldRef& x, const FieldRef
 }
 
 // The same for one right-hand side, with p = r + beta p: the reductions'
-// results are made by the kernels that need them (Cg1HopAlpha .. Cg1P).  On the
-// 32^3x16 FP16-inner solve (ncu, warm): alpha hop 27.1 -> 22.8 us, update hop
-// 34.5 -> 30.7, p 9.8 -> 12.4; the solve 13.07 -> 12.39 ms.
+// results are made by the kernels that need them (CgHopAlpha .. Cg1P).  On the
+// 32^3x16 FP16-inner solve (ncu, warm): alpha hop 27.1 -> 21.1 us, update hop
+// 34.5 -> 29.3, p 9.8 -> 10.1 and 3.0 for the fold of its 4096 partials; the solve
+// 13.1 -> 12.3 ms.
 template <int P>
 clg_status cg1_iteration(Work& w, int op, const FieldRef& x, const FieldRef& r, const FieldRef& p, const int* skip,
                          int ks, int odd) {

@@ -53,7 +53,10 @@ def test_full_forms(clg, tmp_path, kind, prec, dims):
             if kind == "staggered" and cfg == FULL[-1]:
                 continue
             dags = (0, 1) if kind == "wilson" else (0,)
-            c = _context(clg, tmp_path, {_key(kind, prec, d, dims, nrhs) + "_full": cfg for d in dags})
+            keys = [_key(kind, prec, d, dims, nrhs) for d in dags]
+            # the checkerboard hops that form 0 launches: one thread per site
+            plain = {k + auto: _cfg(128, 0) for k in keys for auto in ("", "_auto")}
+            c = _context(clg, tmp_path, {**plain, **{k + "_full": cfg for k in keys}})
             lat = clg.Lattice(c, dims, (1, -1, 1, -1))
             U = clg.CFieldGaugeSU3(lat)
             U.InitialField(clg.GAUGE_EXPH, 0xC1A60001, 1, 0.25)
@@ -103,7 +106,7 @@ def test_split_hop(clg, tmp_path, dims, prec):
 @pytest.mark.parametrize("prec", [0, 1, 2])
 def test_split_cg_epilogues(clg, oracle, tmp_path, prec):
     """the fused CG iteration on the four-threads-per-site epilogues, with a
-    partial last block (2520 sites per checkerboard), to the oracle's residual"""
+    partial last block (5040 sites per checkerboard), to the oracle's residual"""
     dims, n = (6, 10, 14, 12), 1 if prec == 2 else 2
     c = _context(clg, tmp_path, {_key("wilson", prec, d, dims, n): _cfg(128, 4) for d in (0, 1)})
     lat = clg.Lattice(c, dims)
