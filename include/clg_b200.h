@@ -111,7 +111,14 @@ typedef struct clg_solver_s* clg_solver;
  * Replaces appInitialCLG / CCLGLibManager::InitialWithParameter device setup
  * (Core/CLGLibManager.cpp:882-917).  stream == NULL creates a private stream.
  * Objects made on a context (lattices, gauge and fermion fields, solvers,
- * whose workspaces hold fields) are destroyed before the context. */
+ * whose workspaces hold fields) are destroyed before the context.
+ *
+ * A context keeps the temporaries of its calls (operator products, in-place
+ * operators, staged imports and exports, reductions), at most 1 GiB of them, for
+ * the next call; a call that needs room frees the ones idle longest.  All idle
+ * ones go back when a device allocation of any context on the device fails and
+ * when the context is destroyed.  Calls that need such memory are refused
+ * (CLG_ERR_CUDA) while the context's stream is being captured. */
 clg_status clg_context_create(int device, void* cuda_stream, clg_context* out);
 clg_status clg_context_destroy(clg_context ctx);
 clg_status clg_context_set_stream(clg_context ctx, void* cuda_stream);
@@ -142,7 +149,8 @@ clg_status clg_lattice_destroy(clg_lattice lat);
  *   CFieldGaugeSU3.cu:568-592); `data` holds 4*V*18 doubles, on the host unless
  *   on_device != 0.
  * export: CopyDataOutDouble (CFieldGaugeSU3.cu:1693-1760), CLGBin order.
- * random: seeded Haar SU(3), exp(i eps H), identity or zero links generated on the device. */
+ * random: seeded Haar SU(3), exp(i eps H), identity or zero links generated on the
+ *   device; refused while the context's stream is being captured. */
 clg_status clg_gauge_create(clg_lattice lat, clg_gauge* out);
 clg_status clg_gauge_destroy(clg_gauge g);
 clg_status clg_gauge_import(clg_gauge g, const double* data, int layout, int on_device);
@@ -206,7 +214,10 @@ clg_status clg_field_load(clg_field f, int rhs, const char* path, int format);
 
 /* ------------------------------------------------------------------ operators
  * CField::ApplyOperator (Data/Field/CField.h:203): in place, the field is both
- * input and output; coefficient EOCT_None / Minus / Real / Complex. */
+ * input and output; coefficient EOCT_None / Minus / Real / Complex.  Both calls
+ * return once the kernels are queued on the context's stream, products (D D^+,
+ * D D, Schur forms) and in-place operators included; an error of the kernels
+ * themselves is reported by a later call that waits. */
 clg_status clg_apply(int op, clg_field inout, clg_gauge g, int coeff_type, double cre, double cim);
 /* out-of-place variant: out = coeff * op(in) */
 clg_status clg_apply_to(int op, clg_field out, clg_field in, clg_gauge g, int coeff_type, double cre, double cim);
