@@ -46,6 +46,7 @@ constexpr int CGM_RING_MAX = 8;
 // Ring length M of the deferred shift updates: the flush holds M residuals of
 // a site in registers (M * NC complex doubles).
 constexpr int cgm_ring(int nc) { return nc == 3 ? 8 : 2; }
+static_assert(cgm_ring(3) % 2 == 0 && cgm_ring(12) % 2 == 0, "a block ends with |r|^2 in CgmState::rr");
 
 // Device state of a multi-shift CG.  The shifted vectors x_k, p_k are not
 // touched every iteration: within a block of M iterations starting at s they

@@ -1132,7 +1132,8 @@ clg_status krylov(Work& w, int op, const FieldRef& x, const FieldRef& b, int slo
       // 8 iterations per chunk: an inner solve overshoots its convergence by
       // fewer (skipped) iterations; measured on the 32^3x16 FP16-inner solve
       // against chunks of 4, 12 and 16 (65.5, 66.0, 67.2 -> 69.8 solves/s)
-      const int chunk = 8;
+      constexpr int chunk = 8;
+      static_assert(chunk % 2 == 0, "cg1_iteration: a chunk starts with |r|^2 in KState::rr");
       return iterate(w, slot_base + 1, chunk, w.prm->max_iterations / chunk + 2, body, true);
     });
   }
